@@ -84,7 +84,7 @@ def stage_kernels(cfg, form, guess="warm"):
     if cfg.mhd:
         nax = 3 if cfg.sdims == 3 else 1
         if form == "fp32_split":
-            per = cfg.sdims + nax + cfg.sdims + 1 + (1 if guess == "mlp_rescue" else 0)
+            per = cfg.sdims + 3 + (1 if guess == "mlp_rescue" else 0)
             names = "k_face_split_mhd + k_corner_split + k_bface_split + k_c2p_mhd_split"
         else:
             per = cfg.sdims + nax + cfg.sdims + 1

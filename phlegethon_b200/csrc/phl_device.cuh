@@ -22,6 +22,26 @@ constexpr double EM15 = 1.0e-15;
 enum { R_LHLLC = 0, R_HLLC = 1, R_HLLD = 2, R_LHLLD = 3 };
 enum { BC_PERIODIC = 0, BC_REFLECTIVE = 1 };
 
+// Unsigned division by a divisor fixed on the host: q = n m >> (31 + L) with L = ceil(log2 d) and
+// m = floor(2^(31+L) / d) + 1, exact for n < 2^31 (m d exceeds 2^(31+L) by e <= d <= 2^L, and
+// n e < 2^(31+L)).  A division by a run-time divisor is a ~20-instruction sequence, and every
+// index decomposition has two: they were half of the instructions of the corner and face-B kernels.
+struct FastDiv {
+  unsigned d, m, s;
+  static FastDiv by(unsigned div) {
+    FastDiv f;
+    unsigned L = 0;
+    while ((1ull << L) < div) ++L;
+    f.d = div;
+    f.s = 31 + L;
+    f.m = (unsigned)((1ull << f.s) / div + 1);
+    return f;
+  }
+  __host__ __device__ __forceinline__ unsigned quot(unsigned n) const {
+    return (unsigned)(((unsigned long long)n * m) >> s);
+  }
+};
+
 // ------------------------------------------------------------------ grid description
 struct Geo {
   int sdims, nx[3];
@@ -29,6 +49,8 @@ struct Geo {
   int bc[3][2];
   double inv_dx[3];
   double gm, mu, cfl, mach_cutoff, mach_ct;
+  // divisors of the index decompositions: nx[0], nx[0] + 1 and nx[1], nx[1] + 1
+  FastDiv div0[2], div1[2];
   int bg_profile;     // 1: background fields stored as profiles along x2
   int all_mach;       // FLUX_IS_ALL_MACH: LHLLC / LHLLD take the upwind state outside the wave fan
   int use_acc;        // USE_CONSTANT_ACCELERATION with the vector acc
@@ -77,9 +99,20 @@ __device__ __forceinline__ void unflatten3(long long t, int n0, int n1, int &i, 
   k = (int)r;
 }
 
-__device__ __forceinline__ long long lin(const Geo &g, int i, int j, int k) {
-  return (long long)i + (long long)g.nx[0] * ((long long)j + (long long)g.nx[1] * k);
+// the same with host-prepared divisors; index spaces of 2^31 and more do not fit device memory
+__device__ __forceinline__ void unflatten3(long long t, const FastDiv &d0, const FastDiv &d1, int &i, int &j, int &k) {
+  const unsigned u = (unsigned)t, q = d0.quot(u), r = d1.quot(q);
+  i = (int)(u - q * d0.d);
+  j = (int)(q - r * d1.d);
+  k = (int)r;
 }
+
+// index spaces stay below 2^32 (checked at phl_init), so linear indices are formed in 32 bits and
+// widened once
+__device__ __forceinline__ long long lin3(int n0, int n1, int i, int j, int k) {
+  return (long long)((unsigned)i + (unsigned)n0 * ((unsigned)j + (unsigned)n1 * (unsigned)k));
+}
+__device__ __forceinline__ long long lin(const Geo &g, int i, int j, int k) { return lin3(g.nx[0], g.nx[1], i, j, k); }
 
 // ------------------------------------------------------------------ reconstructions
 enum { REC_LIM2ND = 0, REC_PPH = 1, REC_LIM5TH = 2 };

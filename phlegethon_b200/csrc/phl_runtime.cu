@@ -579,6 +579,10 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
   g.sdims = cfg->sdims;
   g.nx[0] = cfg->nx1; g.nx[1] = cfg->nx2; g.nx[2] = cfg->nx3;
   g.N = (long long)cfg->nx1 * cfg->nx2 * cfg->nx3;
+  for (int q = 0; q < 2; ++q) {
+    g.div0[q] = FastDiv::by((unsigned)cfg->nx1 + q);
+    g.div1[q] = FastDiv::by((unsigned)cfg->nx2 + q);
+  }
   for (int d = 0; d < 3; ++d)
     for (int s = 0; s < 2; ++s) g.bc[d][s] = cfg->bc[d][s];
   // dx as initialize_simulation (source.F90:1717-1735)

@@ -16,7 +16,7 @@
 //
 // Hydro stage: one fused kernel (k_stage_split_tiled, TMA-staged planes; k_stage_split per
 // cell).  MHD stage: k_face_split_mhd_walk (PLM) or k_face_split_mhd (PPH, LIM5TH) per
-// direction, k_corner_split per axis, k_bface_split per direction, k_c2p_mhd_split; with the
+// direction, k_corner_split, k_bface_split, k_c2p_mhd_split; with the
 // learned temperature guess k_c2p_mhd_split_features, k_mlp_guess, k_c2p_mhd_split_guessed.
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
@@ -392,6 +392,34 @@ __device__ __forceinline__ void riemann_mhd_split(const float *qL, const float *
   }
 }
 
+// --------------------------------------------------------------------- face flux storage
+// The NV flux components of a face in P.fflux[d] lie in planes of vectors over the faces: one
+// plane of float4 per four components, then a float2 and a float plane for the rest (7 components:
+// 16 + 8 + 4 B).  A face is stored and read with 3 accesses instead of 7 and without padding.
+template <int NV>
+struct FluxPlanes {
+  static constexpr int N4 = NV / 4, N2 = (NV % 4) / 2, N1 = NV % 2;
+  static __device__ __forceinline__ void store(float *p, long long nf, long long f, const float *F) {
+#pragma unroll
+    for (int q = 0; q < N4; ++q)
+      reinterpret_cast<float4 *>(p + 4ll * q * nf)[f] = make_float4(F[4 * q], F[4 * q + 1], F[4 * q + 2], F[4 * q + 3]);
+    if (N2) reinterpret_cast<float2 *>(p + 4ll * N4 * nf)[f] = make_float2(F[4 * N4], F[4 * N4 + 1]);
+    if (N1) p[(4ll * N4 + 2 * N2) * nf + f] = F[NV - 1];
+  }
+  static __device__ __forceinline__ void load(const float *p, long long nf, long long f, float *F) {
+#pragma unroll
+    for (int q = 0; q < N4; ++q) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(p + 4ll * q * nf) + f);
+      F[4 * q] = v.x; F[4 * q + 1] = v.y; F[4 * q + 2] = v.z; F[4 * q + 3] = v.w;
+    }
+    if (N2) {
+      const float2 v = __ldg(reinterpret_cast<const float2 *>(p + 4ll * N4 * nf) + f);
+      F[4 * N4] = v.x; F[4 * N4 + 1] = v.y;
+    }
+    if (N1) F[NV - 1] = __ldg(p + (4ll * N4 + 2 * N2) * nf + f);
+  }
+};
+
 // --------------------------------------------------------------------- FP32 loads
 template <class C>
 __device__ __forceinline__ void load_wf(const Prm &P, int i, int j, int k, float w[C::NV], float g2[2]) {
@@ -730,18 +758,20 @@ __device__ __forceinline__ void split_cell_update(const Prm &P, long long c, int
 template <class C>
 __device__ __forceinline__ void split_stat_flush(const Prm &P, const SplitStat &st) {
   if (P.last_stage) block_max_atomic(st.smax, P.smax_bits);
-  if (C::HELM) {
-    block_sum_atomic(st.calls, P.stat + STAT_NEWTON_CALLS);
-    block_sum_atomic(st.iters, P.stat + STAT_NEWTON_ITERS);
-    block_sum_atomic(st.nonconv, P.stat + STAT_NEWTON_NONCONV);
-    block_sum_atomic(st.clamp, P.stat + STAT_NEWTON_CLAMP);
-    if (P.mlp_w) {
-      block_sum_atomic(st.mlp_acc, P.stat + STAT_MLP_ACC);
-      block_sum_atomic(st.mlp_rej, P.stat + STAT_MLP_REJ);
-      block_sum_atomic(st.gevals, P.stat + STAT_GUESS_EVALS);
-    }
+  if (C::HELM && P.mlp_w) {
+    const unsigned v[8] = {st.bad, st.calls, st.iters, st.nonconv, st.clamp, st.mlp_acc, st.mlp_rej, st.gevals};
+    const int slot[8] = {STAT_NONFINITE, STAT_NEWTON_CALLS, STAT_NEWTON_ITERS, STAT_NEWTON_NONCONV, STAT_NEWTON_CLAMP,
+                         STAT_MLP_ACC, STAT_MLP_REJ, STAT_GUESS_EVALS};
+    block_counters(v, slot, P.stat);
+  } else if (C::HELM) {
+    const unsigned v[5] = {st.bad, st.calls, st.iters, st.nonconv, st.clamp};
+    const int slot[5] = {STAT_NONFINITE, STAT_NEWTON_CALLS, STAT_NEWTON_ITERS, STAT_NEWTON_NONCONV, STAT_NEWTON_CLAMP};
+    block_counters(v, slot, P.stat);
+  } else {
+    const unsigned v[1] = {st.bad};
+    const int slot[1] = {STAT_NONFINITE};
+    block_counters(v, slot, P.stat);
   }
-  block_sum_atomic(st.bad, P.stat + STAT_NONFINITE);
 }
 
 // One thread per cell; every face is solved by both of its cells.  Any grid size.
@@ -754,7 +784,7 @@ __global__ void __launch_bounds__(128) k_stage_split(Prm P) {
   SplitStat st;
   if (c < g.N) {
     int i, j, k;
-    unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+    unflatten3(c, g.div0[0], g.div1[0], i, j, k);
     float res[NV];
     float rho_dev = 0.0f;
 #pragma unroll
@@ -793,6 +823,10 @@ __global__ void __launch_bounds__(128) k_stage_split(Prm P) {
 __device__ __forceinline__ void cp_async4(float *smem_dst, const float *gmem_src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(double *smem_dst, const double *gmem_src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
@@ -1218,9 +1252,8 @@ __device__ __forceinline__ void face_split_mhd_at(const Prm &P, long long f) {
   constexpr int NV = C::NV;
   const Geo &g = P.g;
   const long long nf = nfaces(g, d);
-  const int n0 = g.nx[0] + (d == 0), n1 = g.nx[1] + (d == 1);
   int fi, fj, fk;
-  unflatten3(f, n0, n1, fi, fj, fk);
+  unflatten3(f, g.div0[d == 0], g.div1[d == 1], fi, fj, fk);
   // cells m-3 .. m+2 (the reconstruction reads m-SW .. m+SW-1); a stencil inside the domain
   // is read by linear index, one at a boundary maps each ghost index
   float w[6][NV], gm4[6][2], b4[6][3];
@@ -1251,8 +1284,7 @@ __device__ __forceinline__ void face_split_mhd_at(const Prm &P, long long f) {
   const float *const bv[6] = {b4[0], b4[1], b4[2], b4[3], b4[4], b4[5]};
   float F[NV], Fb[3], rs;
   face_flux_split_mhd<C>(P, d, fi, fj, fk, wv, gv, bv, F, Fb, rs);
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) P.fflux[d][(long long)iv * nf + f] = F[iv];
+  FluxPlanes<NV>::store(P.fflux[d], nf, f, F);
   store_face_emf_split<C>(P, d, f, d == 0 ? fi : (d == 1 ? fj : fk), Fb, F[0], rs, (float)(P.scal[2] * P.inv_v_ref));
 }
 
@@ -1268,8 +1300,6 @@ __global__ void __launch_bounds__(128, C::MINB_FACE32) k_face_split_mhd(Prm P) {
 // so their loads stay within a few cache lines) and along y, z (threads of a warp are
 // neighbours in x and walk side by side)
 constexpr int WALK_K0 = 4, WALK_K = 8;
-// resident blocks of 128 threads per SM of the EoS half of the two-launch cons->prim
-constexpr int C2P_EOS_MINB = 7;
 // grid of the rescue-queue kernels: 4 blocks of 128 threads per SM of a B200 (148 SMs)
 constexpr int RESCUE_BLOCKS = 4 * 148;
 // resident blocks of 128 threads per SM the walking kernels are compiled for (72 registers; the
@@ -1389,8 +1419,7 @@ __global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : 
     }
     float F[NV], Fb[3], rs;
     face_solve_split_mhd<C>(P, D, fidx, fbg, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F, Fb, rs);
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) P.fflux[D][(long long)iv * nf + fidx] = F[iv];
+    FluxPlanes<NV>::store(P.fflux[D], nf, fidx, F);
     store_face_emf_split<C>(P, D, fidx, q, Fb, F[0], rs, smax_s);
 #pragma unroll
     for (int v = 0; v < NR; ++v) {
@@ -1581,8 +1610,7 @@ __global__ void __launch_bounds__(FaceTileSmem<C, D>::NT, FaceTile<D>::MINB)
     float F[NV], Fb[3], rs;
     face_solve_split_mhd<C>(P, D, fidx, fbg, qL, qR, bL, bR, gL, gR, tface, false, F, Fb, rs);
     const long long nf = nfaces(g, D);
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) P.fflux[D][(long long)iv * nf + fidx] = F[iv];
+    FluxPlanes<NV>::store(P.fflux[D], nf, fidx, F);
     store_face_emf_split<C>(P, D, fidx, c0 + td, Fb, F[0], rs, (float)(P.scal[2] * P.inv_v_ref));
   }
   // the faces at the upper domain boundary along D, one per thread, strided over the grid
@@ -1697,83 +1725,105 @@ __device__ __forceinline__ float corner_emf_split(const Prm &P, const int c[3]) 
   return 0.25f * (emf_S + emf_W + emf_N + emf_E + demf_S - demf_N + demf_W - demf_E);
 }
 
-// Corner EMFs along axis A, one thread per corner (one instantiation per axis: the face and cell
-// strides fold into constants).  The first nin_blocks blocks take the interior corners (1 <=
-// c[pa] < nx[pa], 1 <= c[qa] < nx[qa]), which read their faces and cells by linear index with no
-// branch; the blocks after them take the corners on the domain faces of pa and qa, which map
-// their ghost indices.  Threads over all corners in array order had a quarter of their warps
-// diverge into the mapping path, where the rows of corners (nx + 1 long) straddle the warps.
-template <class C, int A>
-__global__ void __launch_bounds__(256) k_corner_split(Prm P, unsigned nin_blocks) {
-  constexpr int a = A, pa = A == 2 ? 0 : (A == 0 ? 1 : 2), qa = A == 2 ? 1 : (A == 0 ? 2 : 0);
+// Corner EMFs of every axis, one thread per grid node (i, j, k): the corner of axis a whose lower
+// end is the node.  A node's three corners share their index arithmetic, the signs of the node's
+// faces and the cache lines of its cells; one launch a stage.  The first nin_blocks blocks take
+// the interior nodes (1 <= index < nx in every dimension), which read faces and cells by linear
+// index with no branch; the blocks after them take the nodes on the domain's faces, whose corners
+// map their ghost indices (threads over all nodes in array order had a quarter of their warps
+// diverge into the mapping path, where the rows of nodes, nx + 1 long, straddle the warps).
+// Bound by its loads: 36 B of face EMFs and signs, 12 B of cell EMFs in, 12 B out per cell.
+template <class C>
+__global__ void __launch_bounds__(256) k_corner_split(Prm P, unsigned nin_blocks, FastDiv e0, FastDiv e1) {
   if (!*P.active) return;
   const Geo &g = P.g;
   int c[3];
   if (blockIdx.x < nin_blocks) {
-    // interior extents per dimension (x1 fastest, as the arrays): nx - 1 from index 1 along pa
-    // and qa, nx from index 0 along a
-    const int e0 = a == 0 ? g.nx[0] : g.nx[0] - 1, e1 = a == 1 ? g.nx[1] : g.nx[1] - 1;
-    const int e2 = C::DIM == 3 ? (a == 2 ? g.nx[2] : g.nx[2] - 1) : 1;
+    // e0 and e1 are nx - 1 of x1 and x2
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)e0 * e1 * e2) return;
+    if (t >= (long long)e0.d * e1.d * (C::DIM == 3 ? g.nx[2] - 1 : 1)) return;
     unflatten3(t, e0, e1, c[0], c[1], c[2]);
-    c[0] += a != 0;
-    c[1] += a != 1;
-    if (C::DIM == 3) c[2] += a != 2;
-    P.fcor[a][cor_lin(g, a, c[0], c[1], c[2])] = corner_emf_split<C, A, true>(P, c);
+    c[0] += 1;
+    c[1] += 1;
+    if (C::DIM == 3) {
+      c[2] += 1;
+      P.fcor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf_split<C, 0, true>(P, c);
+      P.fcor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf_split<C, 1, true>(P, c);
+    }
+    P.fcor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf_split<C, 2, true>(P, c);
     return;
   }
-  // the rim: per index along a, the border of the (nx[pa] + 1) x (nx[qa] + 1) rectangle of
-  // corners, 2 (nx[pa] + nx[qa]) of them
-  const int np_ = g.nx[pa], nq = g.nx[qa], na = C::DIM == 3 ? g.nx[a] : 1, rim = 2 * (np_ + nq);
-  const long long t = (long long)(blockIdx.x - nin_blocks) * blockDim.x + threadIdx.x;
-  if (t >= (long long)rim * na) return;
-  const int m = (int)(t % rim);
-  c[a] = (int)(t / rim);
-  if (m < np_ + 1) { c[pa] = m; c[qa] = 0; }                             // qa = 0 row
-  else if (m < 2 * (np_ + 1)) { c[pa] = m - (np_ + 1); c[qa] = nq; }       // qa = nx[qa] row
-  else if (m < 2 * (np_ + 1) + (nq - 1)) { c[pa] = 0; c[qa] = m - 2 * (np_ + 1) + 1; }  // pa = 0 column
-  else { c[pa] = np_; c[qa] = m - 2 * (np_ + 1) - (nq - 1) + 1; }         // pa = nx[pa] column
-  P.fcor[a][cor_lin(g, a, c[0], c[1], c[2])] = corner_emf_split<C, A, false>(P, c);
+  // the nodes on the domain's faces: the k = 0 and k = nx[2] planes (3D), then per inner plane the
+  // border of the (nx[0] + 1) x (nx[1] + 1) rectangle, 2 (nx[0] + nx[1]) of them
+  const int n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2], rim = 2 * (n0 + n1);
+  const long long ncap = C::DIM == 3 ? 2ll * (n0 + 1) * (n1 + 1) : 0;
+  long long t = (long long)(blockIdx.x - nin_blocks) * blockDim.x + threadIdx.x;
+  if (t < ncap) {
+    unflatten3(t, g.div0[1], g.div1[1], c[0], c[1], c[2]);
+    c[2] = c[2] ? n2 : 0;
+  } else {
+    t -= ncap;
+    if (t >= (long long)rim * (C::DIM == 3 ? n2 - 1 : 1)) return;
+    const int m = (int)(t % rim);
+    c[2] = C::DIM == 3 ? (int)(t / rim) + 1 : 0;
+    if (m < n0 + 1) { c[0] = m; c[1] = 0; }                                      // x2 = 0 row
+    else if (m < 2 * (n0 + 1)) { c[0] = m - (n0 + 1); c[1] = n1; }               // x2 = nx[1] row
+    else if (m < 2 * (n0 + 1) + (n1 - 1)) { c[0] = 0; c[1] = m - 2 * (n0 + 1) + 1; }  // x1 = 0 column
+    else { c[0] = n0; c[1] = m - 2 * (n0 + 1) - (n1 - 1) + 1; }                  // x1 = nx[0] column
+  }
+  if (C::DIM == 3) {
+    if (c[0] < n0) P.fcor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf_split<C, 0, false>(P, c);
+    if (c[1] < n1) P.fcor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf_split<C, 1, false>(P, c);
+    if (c[2] >= n2) return;
+  }
+  P.fcor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf_split<C, 2, false>(P, c);
 }
 
-// face-B update (source.F90:12208-12437) in FP64 from the FP32 corner EMFs; one thread per face
-template <class C, int D>
+// face-B update (source.F90:12208-12437) in FP64 from the FP32 corner EMFs; one thread per grid
+// node (i, j, k), which updates the low face of cell (i, j, k) in every direction (the three
+// share corner EMFs: 9 loads for the three faces, most of them cache hits).  Bound by memory:
+// 12 B of corner EMFs in, and B and B0 in and B out in FP64 (72 B) per cell.
+template <class C>
 __global__ void __launch_bounds__(256) k_bface_split(Prm P) {
-  constexpr int d = D;
   if (!*P.active) return;
   const Geo &g = P.g;
-  long long nf = nfaces(g, d);
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf) return;
-  int n0 = g.nx[0] + (d == 0), n1 = g.nx[1] + (d == 1);
+  const int n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)(n0 + 1) * (n1 + 1) * (C::DIM == 3 ? n2 + 1 : 1)) return;
   int i, j, k;
-  unflatten3(t, n0, n1, i, j, k);
+  unflatten3(t, g.div0[1], g.div1[1], i, j, k);
+  const bool in0 = i < n0, in1 = j < n1, in2 = C::DIM == 2 || k < n2;
   const double dt = P.scal[1];
   const double a1 = P.a1, a2 = P.a2, a3 = P.c3 * dt * (P.v_ref * P.b_ref);
-  const float *E1 = P.fcor[0], *E2 = P.fcor[1], *E3 = P.fcor[2];
   // differences of the FP32 corner EMFs are formed in FP64 (exact), so the discrete divergence
   // of the update cancels to FP64 rounding as in the FP64 form
-  auto e = [](const float *E, long long q) { return (double)E[q]; };
-  double tmp;
-  if (d == 0) {
-    if (C::DIM == 2) tmp = (e(E3, cor_lin(g, 2, i, j + 1, k)) - e(E3, cor_lin(g, 2, i, j, k))) * g.inv_dx[1];
-    else tmp = -(e(E2, cor_lin(g, 1, i, j, k + 1)) - e(E2, cor_lin(g, 1, i, j, k))) * g.inv_dx[2] +
-               (e(E3, cor_lin(g, 2, i, j + 1, k)) - e(E3, cor_lin(g, 2, i, j, k))) * g.inv_dx[1];
-  } else if (d == 1) {
-    if (C::DIM == 2) tmp = (e(E3, cor_lin(g, 2, i, j, k)) - e(E3, cor_lin(g, 2, i + 1, j, k))) * g.inv_dx[0];
-    else tmp = (e(E1, cor_lin(g, 0, i, j, k + 1)) - e(E1, cor_lin(g, 0, i, j, k))) * g.inv_dx[2] +
-               (e(E3, cor_lin(g, 2, i, j, k)) - e(E3, cor_lin(g, 2, i + 1, j, k))) * g.inv_dx[0];
-  } else {
-    tmp = (e(E2, cor_lin(g, 1, i + 1, j, k)) - e(E2, cor_lin(g, 1, i, j, k))) * g.inv_dx[0] -
-          (e(E1, cor_lin(g, 0, i, j + 1, k)) - e(E1, cor_lin(g, 0, i, j, k))) * g.inv_dx[1];
+  auto e = [&](int a, long long q) { return (double)__ldg(P.fcor[a] + q); };
+  // where each corner array continues along the other two directions
+  const long long q2 = cor_lin(g, 2, i, j, k), q2y = n0 + 1;
+  auto update = [&](int d, double tmp) {
+    const long long f = face_lin(g, d, i, j, k);
+    const double b = P.bf[d][f];
+    double b0;
+    if (P.first_stage) { b0 = b; P.b0f[d][f] = b; } else { b0 = P.b0f[d][f]; }
+    P.bf[d][f] = a1 * b0 + a2 * b + a3 * tmp;
+  };
+  if (C::DIM == 2) {
+    const double E3 = e(2, q2);
+    if (in1) update(0, (e(2, q2 + q2y) - E3) * g.inv_dx[1]);
+    if (in0) update(1, (E3 - e(2, q2 + 1)) * g.inv_dx[0]);
+    return;
   }
-  double b = P.bf[d][t];
-  double b0;
-  if (P.first_stage) { b0 = b; P.b0f[d][t] = b; } else { b0 = P.b0f[d][t]; }
-  P.bf[d][t] = a1 * b0 + a2 * b + a3 * tmp;
+  const long long q0 = cor_lin(g, 0, i, j, k), q0y = n0, q0z = (long long)n0 * (n1 + 1);
+  const long long q1 = cor_lin(g, 1, i, j, k), q1z = (long long)(n0 + 1) * n1;
+  // E1 exists for i < nx1, E2 for j < nx2, E3 for k < nx3
+  const double E1 = in0 ? e(0, q0) : 0.0, E2 = in1 ? e(1, q1) : 0.0, E3 = in2 ? e(2, q2) : 0.0;
+  if (in1 && in2) update(0, -(e(1, q1 + q1z) - E2) * g.inv_dx[2] + (e(2, q2 + q2y) - E3) * g.inv_dx[1]);
+  if (in0 && in2) update(1, (e(0, q0 + q0z) - E1) * g.inv_dx[2] + (E3 - e(2, q2 + 1)) * g.inv_dx[0]);
+  if (in0 && in1) update(2, (e(1, q1 + 1) - E2) * g.inv_dx[0] - (e(0, q0 + q0y) - E1) * g.inv_dx[1]);
 }
 
+// cells per block of the cons->prim kernels
+constexpr int C2P_BLOCK = 128;
 // New state of one cell that the EoS part of cons->prim needs (the rest is stored before it)
 struct C2pState {
   double rho = 1.0, inv_rho = 1.0, eint = 0.0, ye = 0.0, inv_abar = 1.0;
@@ -1793,9 +1843,21 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
   long long &bc = cs.bc;
   {
     int i, j, k;
-    unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+    unflatten3(c, g.div0[0], g.div1[0], i, j, k);
     bc = bg_cc(g, i, j, k);
     double bcc[3] = {0, 0, 0}, u[NV];
+    // the running and initial conserved state travel to shared memory (each thread its own cell's,
+    // so no barrier) while the fluxes are read: with all 56 loads through the 64 to 72 registers a
+    // thread has here they went out in small batches, each waiting for the memory
+    __shared__ double su[2 * NV][C2P_BLOCK];
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int iv = 0; iv < NV; ++iv) cp_async8(&su[iv][tid], P.U + (long long)iv * g.N + c);
+    if (!P.first_stage) {
+#pragma unroll
+      for (int iv = 0; iv < NV; ++iv) cp_async8(&su[NV + iv][tid], P.U0 + (long long)iv * g.N + c);
+    }
+    cp_async_commit();
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
       int ui = i + (d == 0), uj = j + (d == 1), uk = k + (d == 2);
@@ -1807,11 +1869,13 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
       const long long nf = nfaces(g, d);
-      const long long flo = face_lin(g, d, i, j, k), fhi = face_lin(g, d, i + (d == 0), j + (d == 1), k + (d == 2));
+      float lo[NV], hi[NV];
+      FluxPlanes<NV>::load(P.fflux[d], nf, face_lin(g, d, i, j, k), lo);
+      FluxPlanes<NV>::load(P.fflux[d], nf, face_lin(g, d, i + (d == 0), j + (d == 1), k + (d == 2)), hi);
       const float inv_dl = (float)g.inv_dx[d];
 #pragma unroll
       for (int iv = 0; iv < NV; ++iv) {
-        float dd = (P.fflux[d][(long long)iv * nf + fhi] - P.fflux[d][(long long)iv * nf + flo]) * inv_dl;
+        float dd = (hi[iv] - lo[iv]) * inv_dl;
         res[iv] = d == 0 ? dd : res[iv] + dd;
       }
     }
@@ -1832,8 +1896,9 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
     {
       const double dt = P.scal[1], a1 = P.a1, a2 = P.a2, a3 = P.c3 * dt;
       double un[NV];
+      cp_async_wait_all();
 #pragma unroll
-      for (int iv = 0; iv < NV; ++iv) un[iv] = P.U[(long long)iv * g.N + c];
+      for (int iv = 0; iv < NV; ++iv) un[iv] = su[iv][tid];
       if (g.use_acc) constant_acceleration<DIM, IP>(g, un, rd);
 #pragma unroll
       for (int iv = 0; iv < NV; ++iv) {
@@ -1842,7 +1907,7 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
           u0 = un[iv];
           P.U0[(long long)iv * g.N + c] = un[iv];
         } else {
-          u0 = P.U0[(long long)iv * g.N + c];
+          u0 = su[NV + iv][tid];
         }
         u[iv] = a1 * u0 + a2 * un[iv] + a3 * rd[iv];
         P.U[(long long)iv * g.N + c] = u[iv];
@@ -1980,7 +2045,7 @@ __device__ __forceinline__ bool c2p_mhd_split_eos(const Prm &P, long long c, con
     if (P.last_stage) {
       // |v| and b_cc^2 of the new state, read back (U and the face B are this cell's own)
       int i, j, k;
-      unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+      unflatten3(c, g.div0[0], g.div1[0], i, j, k);
       double vabs[3] = {0.0, 0.0, 0.0}, ca2 = 0.0;
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
@@ -2000,11 +2065,8 @@ __device__ __forceinline__ bool c2p_mhd_split_eos(const Prm &P, long long c, con
   return true;
 }
 
-// cells per block of the cons->prim kernels
-constexpr int C2P_BLOCK = 128;
-
-template <class C, int MODE, int MINB = C::MINB_C2P32>
-__global__ void __launch_bounds__(C2P_BLOCK, MINB) k_c2p_mhd_split(Prm P) {
+template <class C, int MODE>
+__global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_mhd_split(Prm P) {
   if (!*P.active) return;
   SplitStat st;
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2018,28 +2080,13 @@ __global__ void __launch_bounds__(C2P_BLOCK, MINB) k_c2p_mhd_split(Prm P) {
   split_stat_flush<C>(P, st);
 }
 
-// cons->prim in two launches (PHL_C2P=two): the combine with the stores that depend on the
-// conserved state alone (and eint), then the EoS part from U and eint read back; the second
-// kernel holds only the Newton's registers and runs at a higher occupancy
-template <class C>
-__global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_mhd_split_combine(Prm P) {
-  if (!*P.active) return;
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= P.g.N) return;
-  C2pState cs;
-  c2p_mhd_split_combine<C>(P, c, cs);
-  P.eint[c] = cs.eint;
-}
-template <class C>
-__global__ void __launch_bounds__(128, C2P_EOS_MINB) k_c2p_mhd_split_eos(Prm P);
-
 // the state of the combine for cell c, read back from U and eint
 template <class C>
 __device__ __forceinline__ void c2p_state_from_u(const Prm &P, long long c, C2pState &cs) {
   constexpr int IAS = C::IAS;
   const Geo &g = P.g;
   int i, j, k;
-  unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+  unflatten3(c, g.div0[0], g.div1[0], i, j, k);
   cs.bc = bg_cc(g, i, j, k);
   cs.rho = P.U[c];
   cs.inv_rho = 1.0 / cs.rho;
@@ -2116,19 +2163,6 @@ static __global__ void __launch_bounds__(128) k_mlp_guess(const __grid_constant_
   if (t < n) out[t] = have ? y : __int_as_float(0x7fc00000);
 }
 
-template <class C>
-__global__ void __launch_bounds__(128, C2P_EOS_MINB) k_c2p_mhd_split_eos(Prm P) {
-  if (!*P.active) return;
-  SplitStat st;
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < P.g.N) {
-    C2pState cs;
-    c2p_state_from_u<C>(P, c, cs);
-    c2p_mhd_split_eos<C, C2P_WARM>(P, c, cs, 0.0f, st);
-  }
-  split_stat_flush<C>(P, st);
-}
-
 // ---- learned rescue of poor warm starts (eos_guess = PHL_GUESS_MLP_RESCUE): one kernel on a
 // fixed grid over the queue that k_c2p_mhd_split<C, C2P_RESCUE> fills.  Tiles of 128 queue
 // slots, strided over the blocks: each thread reads its cell's state back (U, eint) and forms
@@ -2178,7 +2212,7 @@ __global__ void k_split_from_prim(Prm P) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.N) return;
   int i, j, k;
-  unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+  unflatten3(c, g.div0[0], g.div1[0], i, j, k);
   const long long bc = bg_cc(g, i, j, k);
   double w[NV];
 #pragma unroll
@@ -2234,7 +2268,7 @@ __global__ void k_split_to_prim(Prm P) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.N) return;
   int i, j, k;
-  unflatten3(c, g.nx[0], g.nx[1], i, j, k);
+  unflatten3(c, g.div0[0], g.div1[0], i, j, k);
   const long long bc = bg_cc(g, i, j, k);
   double u[NV];
 #pragma unroll
@@ -2381,19 +2415,6 @@ struct SplitRunnerT : Runner {
       if constexpr (C::DIM == 3) tile_wave[2] = wave_of(k_face_split_mhd_tile<C, 2>, FaceTileSmem<C, 2>::NT);
     }
   }
-  // resident blocks per SM the Helmholtz MHD cons->prim is compiled for: 8 (64 registers, ~100
-  // B of spills), which ran a step at 256^3 in 13.56 ms against 13.89 at 7 (72 registers), 14.37
-  // at 6 (80), 13.73 at 9 and 14.14 at 10: its time is latency, and more resident warps hide it
-  // until the spills dominate; PHL_C2P_MINB=6 selects the 80-register build (comparison)
-  const int c2p_minb = [] {
-    const char *e = getenv("PHL_C2P_MINB");
-    return e && atoi(e) == 6 ? 6 : 8;
-  }();
-  // PHL_C2P=two runs the warm-start cons->prim of the MHD stage as two launches
-  const bool c2p_two = [] {
-    const char *e = getenv("PHL_C2P");
-    return e && strcmp(e, "two") == 0;
-  }();
   // face kernel per direction: by default the shared-memory tiles along x1 (where the walking
   // kernel's threads stride K0 cells apart) and the walking kernels along x2 and x3 (threads of
   // a warp are neighbours in x1 there, and the walk, with no block barrier and the edges in
@@ -2472,22 +2493,14 @@ struct SplitRunnerT : Runner {
         k_face_split_mhd<C, 1><<<nblk(nfc(1), 128), 128, 0, s>>>(P);
         if constexpr (C::DIM == 3) k_face_split_mhd<C, 2><<<nblk(nfc(2), 128), 128, 0, s>>>(P);
       }
-      if constexpr (C::DIM == 3) {
-        corners<0>(P, s);
-        corners<1>(P, s);
-      }
-      corners<2>(P, s);
-      k_bface_split<C, 0><<<nblk(nfc(0), 256), 256, 0, s>>>(P);
-      k_bface_split<C, 1><<<nblk(nfc(1), 256), 256, 0, s>>>(P);
-      if constexpr (C::DIM == 3) k_bface_split<C, 2><<<nblk(nfc(2), 256), 256, 0, s>>>(P);
+      corners(P, s);
+      const long long nodes = (long long)(g.nx[0] + 1) * (g.nx[1] + 1) * (C::DIM == 3 ? g.nx[2] + 1 : 1);
+      k_bface_split<C><<<nblk(nodes, 256), 256, 0, s>>>(P);
       if constexpr (C::HELM) {
         if (P.mlp_w && P.mlp_small && P.rescue_q) {
           // warm start everywhere; cells with a poor warm start through the learned guess
           cudaMemsetAsync(P.rescue_q, 0, sizeof(unsigned), s);
-          if (C::HELM && c2p_minb == 8)
-            k_c2p_mhd_split<C, C2P_RESCUE, 8><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
-          else
-            k_c2p_mhd_split<C, C2P_RESCUE><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
+          k_c2p_mhd_split<C, C2P_RESCUE><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
           k_c2p_rescue<C><<<RESCUE_BLOCKS, 128, sizeof(MlpUmmaSmem), s>>>(P, *P.mlp_small);
           return;
         }
@@ -2499,28 +2512,20 @@ struct SplitRunnerT : Runner {
           return;
         }
       }
-      if (c2p_two) {
-        k_c2p_mhd_split_combine<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
-        k_c2p_mhd_split_eos<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
-      } else if (C::HELM && c2p_minb == 8) {
-        k_c2p_mhd_split<C, C2P_WARM, 8><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
-      } else {
-        k_c2p_mhd_split<C, C2P_WARM><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
-      }
+      k_c2p_mhd_split<C, C2P_WARM><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
     } else {
       hydro_stage(P, s);
     }
   }
-  // corner EMFs along axis A: the interior corners' blocks, then the rim's, in one launch
-  template <int A>
+  // corner EMFs: the interior nodes' blocks, then those of the nodes on the domain's faces
   void corners(const Prm &P, cudaStream_t s) {
-    constexpr int pa = A == 2 ? 0 : (A == 0 ? 1 : 2), qa = A == 2 ? 1 : (A == 0 ? 2 : 0);
     const Geo &g = P.g;
-    const long long na = C::DIM == 3 ? g.nx[A] : 1;
-    const long long nin = (long long)(g.nx[pa] - 1) * (g.nx[qa] - 1) * na;
-    const long long nrim = 2ll * (g.nx[pa] + g.nx[qa]) * na;
+    const long long n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2];
+    const long long nin = (n0 - 1) * (n1 - 1) * (C::DIM == 3 ? n2 - 1 : 1);
+    const long long nrim = 2 * (n0 + n1) * (C::DIM == 3 ? n2 - 1 : 1) + (C::DIM == 3 ? 2 * (n0 + 1) * (n1 + 1) : 0);
     const unsigned bin = nblk(nin, 256);
-    k_corner_split<C, A><<<bin + nblk(nrim, 256), 256, 0, s>>>(P, bin);
+    k_corner_split<C><<<bin + nblk(nrim, 256), 256, 0, s>>>(P, bin, FastDiv::by((unsigned)n0 - 1),
+                                                            FastDiv::by((unsigned)n1 - 1));
   }
   void hydro_stage(const Prm &P, cudaStream_t s) {
     if constexpr (C::DIM == 3 && C::SW == 2) {
