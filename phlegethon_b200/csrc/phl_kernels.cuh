@@ -75,8 +75,9 @@ struct Prm {
   // of rho_ref, p_ref and v_ref = sqrt(p_ref / rho_ref) so that no product leaves FP32 range
   double rho_ref, p_ref, v_ref;
   double inv_rho_ref, inv_p_ref, inv_v_ref;
-  // face background of the split path in those units, FP32 (x / ref rounded once at upload)
-  const float *sf_rho_f[3], *sf_p_f[3], *sf_ge_f[3], *sf_phi_f[3];
+  // face background of the split path in those units, FP32 (x / ref rounded once at upload): density,
+  // pressure, gamma_e and potential of a face side by side
+  const float4 *sf_bg[3];
   // MHD in the split path: B in units of b_ref = sqrt(p_ref) (magnetic pressure B^2/2 in p_ref),
   // EMFs in v_ref b_ref; cell-centred B, face EMFs, mass-flux signs and corner EMFs in FP32
   double b_ref, inv_b_ref;

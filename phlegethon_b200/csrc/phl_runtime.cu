@@ -126,10 +126,11 @@ Runner *make_runner(int dim, int nv, bool mhd, bool helm, bool strat, int riem, 
   return nullptr;
 }
 
-// dst = (float)(src / ref): the split path's FP32 copy of a background array
+// dst[4 i] = (float)(src[i] / ref): the split path's FP32 copy of a background array, one of the four
+// components of a face
 __global__ void k_scale_f32(const double *src, float *dst, long long n, double ref) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)(src[i] / ref);
+  if (i < n) dst[4 * i] = (float)(src[i] / ref);
 }
 
 // ----------------------------------------------------------------------------- transposes
@@ -210,7 +211,7 @@ struct phl_ctx {
   int bg_profile = 0;
   double *eq_rho_cc = nullptr, *eq_p_cc = nullptr, *eq_ge_cc = nullptr, *phi_cc = nullptr, *grav = nullptr;
   double *eq_rho_f[3] = {}, *eq_p_f[3] = {}, *eq_ge_f[3] = {}, *phi_f[3] = {};
-  float *sf_rho_f[3] = {}, *sf_p_f[3] = {}, *sf_ge_f[3] = {}, *sf_phi_f[3] = {};  // split path
+  float *sf_bg[3] = {};  // split path
   float *bccf = nullptr, *femf[3] = {}, *fsgn[3] = {}, *fcor[3] = {};                // split MHD
   float *fflux[3] = {};
   float *fecell = nullptr;                                                             // split MHD
@@ -349,7 +350,7 @@ struct phl_ctx {
     P.eq_rho_cc = eq_rho_cc; P.eq_p_cc = eq_p_cc; P.eq_ge_cc = eq_ge_cc; P.phi_cc = phi_cc; P.grav = grav;
     for (int d = 0; d < 3; ++d) {
       P.eq_rho_f[d] = eq_rho_f[d]; P.eq_p_f[d] = eq_p_f[d]; P.eq_ge_f[d] = eq_ge_f[d]; P.phi_f[d] = phi_f[d];
-      P.sf_rho_f[d] = sf_rho_f[d]; P.sf_p_f[d] = sf_p_f[d]; P.sf_ge_f[d] = sf_ge_f[d]; P.sf_phi_f[d] = sf_phi_f[d];
+      P.sf_bg[d] = reinterpret_cast<const float4 *>(sf_bg[d]);
       P.bf[d] = bf[d]; P.b0f[d] = b0f[d]; P.emf[d] = emf[d]; P.sgnf[d] = sgnf[d]; P.cor[d] = cor[d];
     }
     P.bcc_in = bcc;
@@ -389,13 +390,11 @@ struct phl_ctx {
     for (int d = 0; d < dim; ++d) {
       long long nf = geo.bg_profile ? (long long)(geo.nx[1] + (d == 1)) : nfaces(d);
       int rc;
-      if (!sf_rho_f[d] && ((rc = alloc(&sf_rho_f[d], nf)) || (rc = alloc(&sf_p_f[d], nf)) ||
-                           (rc = alloc(&sf_phi_f[d], nf)) || (rc = alloc(&sf_ge_f[d], nf))))
-        return rc;
-      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_rho_f[d], sf_rho_f[d], nf, rho_ref);
-      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_p_f[d], sf_p_f[d], nf, p_ref);
-      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(phi_f[d], sf_phi_f[d], nf, v_ref * v_ref);
-      if (helm) k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_ge_f[d], sf_ge_f[d], nf, 1.0);
+      if (!sf_bg[d] && (rc = alloc(&sf_bg[d], 4 * nf))) return rc;
+      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_rho_f[d], sf_bg[d], nf, rho_ref);
+      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_p_f[d], sf_bg[d] + 1, nf, p_ref);
+      if (helm) k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_ge_f[d], sf_bg[d] + 2, nf, 1.0);
+      k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(phi_f[d], sf_bg[d] + 3, nf, v_ref * v_ref);
     }
     CK(cudaGetLastError());
     return PHL_OK;
