@@ -77,14 +77,14 @@ def default_size(name):
 
 
 def stage_kernels(cfg, form, guess="warm"):
-    """Name of what the per-stage timing covers, and the kernel launches of one step (the stage
-    kernels plus k_pre_step and k_post_step; the learned rescue adds its queue kernel to every
-    stage)."""
+    """The parts of a stage that the traffic model below counts, and their number in one step with
+    every direction and axis a part of its own (plus k_pre_step and k_post_step).  What one launch
+    covers is step_launches' business."""
     s = cfg.rk_stages
     if cfg.mhd:
         nax = 3 if cfg.sdims == 3 else 1
         if form == "fp32_split":
-            per = cfg.sdims + 3 + (1 if guess == "mlp_rescue" else 0)
+            per = cfg.sdims + nax + cfg.sdims + 1 + (1 if guess == "mlp_rescue" else 0)
             names = "k_face_split_mhd + k_corner_split + k_bface_split + k_c2p_mhd_split"
         else:
             per = cfg.sdims + nax + cfg.sdims + 1
@@ -94,6 +94,22 @@ def stage_kernels(cfg, form, guess="warm"):
         tiled = cfg.sdims == 3 and cfg.nx1 % 32 == 0 and cfg.nx2 % 8 == 0 and cfg.nx3 % 16 == 0
         return ("k_stage_split_tiled" if tiled else "k_stage_split") + " (FP32 fluxes, FP64 state/EoS)", s + 2
     return "k_face + k_c2p (FP64)", s * (cfg.sdims + 1) + 2
+
+
+def step_launches(cfg, form, guess="warm"):
+    """Name of what the per-stage timing covers, and the kernel launches of one step (the stage
+    kernels plus k_pre_step and k_post_step; the learned rescue adds its queue kernel to every
+    stage)."""
+    s = cfg.rk_stages
+    if form != "fp32_split":
+        return stage_kernels(cfg, form, guess)
+    if cfg.mhd:
+        # faces per direction, corners, face B, cons->prim
+        per = cfg.sdims + 3 + (1 if guess == "mlp_rescue" else 0)
+        return "k_face_split + k_corner_split + k_bface_split + k_c2p_split (one MHD stage)", s * per + 2
+    if cfg.n_cells < (220000 if cfg.sdims == 3 else 430000):
+        return "k_stage_split (FP32 fluxes, FP64 state/EoS)", s + 2
+    return "k_face_split + k_c2p_split (one hydro stage)", s * (cfg.sdims + 1) + 2
 
 
 # DRAM bytes per cell of one stage-kernel launch, from ncu captures of the 128^3 stratified box
@@ -741,7 +757,7 @@ def run_ours(args):
     model_bytes = step_bytes_per_cell(cfg.replace(precision=head_form))
     launch_ms = head["launch_ms"]
     achieved = bytes_per_cell * cells / cfg.rk_stages / (launch_ms * 1e-3) / 1e9
-    kname, launches_per_step = stage_kernels(cfg, head_form, head_guess)
+    kname, launches_per_step = step_launches(cfg, head_form, head_guess)
     tpc = TRAFFIC_PER_CELL.get((name, head_form))
     roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / peaks["hbm_gbs"], "traffic": tpc * cells if tpc else None,

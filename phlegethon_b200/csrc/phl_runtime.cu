@@ -646,7 +646,6 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
         long long nf = c->nfaces(d);
         if ((rc = c->alloc(&c->femf[d], (size_t)3 * nf))) return rc;
         if ((rc = c->alloc(&c->fsgn[d], (size_t)nf))) return rc;
-        if ((rc = c->alloc(&c->fflux[d], (size_t)nv * nf))) return rc;
       }
       for (int a = 0; a < 3; ++a) {
         if (cfg->sdims == 2 && a != 2) continue;
@@ -654,9 +653,11 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
       }
     }
   }
-  if (!c->split)
-    for (int d = 0; d < cfg->sdims; ++d)
-      if ((rc = c->alloc(&c->dflux[d], (size_t)nv * c->nfaces(d)))) return rc;
+  // face fluxes, FP64 or FP32
+  for (int d = 0; d < cfg->sdims; ++d)
+    if ((rc = c->split ? c->alloc(&c->fflux[d], (size_t)nv * c->nfaces(d))
+                       : c->alloc(&c->dflux[d], (size_t)nv * c->nfaces(d))))
+      return rc;
   if ((rc = c->alloc(&c->scal, 8))) return rc;
   if ((rc = c->alloc(&c->smax_bits, 1))) return rc;
   if ((rc = c->alloc(&c->active, 1))) return rc;

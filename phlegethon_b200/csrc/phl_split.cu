@@ -14,12 +14,11 @@
 // B / sqrt(p_ref)), fixed per run, so products of deviations never leave FP32 range whatever the
 // problem's cgs magnitudes.
 //
-// Hydro stage: one fused kernel (k_stage_split_tiled, TMA-staged planes; k_stage_split per
-// cell).  MHD stage: k_face_split_mhd_row along x1 and k_face_split_mhd_walk along x2 and x3 (PLM),
-// or k_face_split_mhd per direction (PPH, LIM5TH), k_corner_split, k_bface_split, k_c2p_mhd_split; with the
-// learned temperature guess k_c2p_mhd_split_features, k_mlp_guess, k_c2p_mhd_split_guessed.
+// Stage: k_face_split_row along x1 and k_face_split_walk along x2 and x3 (PLM), or k_face_split per
+// direction (PPH, LIM5TH); for MHD k_corner_split and k_bface_split; then k_c2p_split.  With the
+// learned temperature guess k_c2p_split_features, k_mlp_guess, k_c2p_split_guessed.  Hydro on small
+// grids: k_stage_split, one kernel.
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
@@ -87,35 +86,44 @@ __device__ __forceinline__ void riemann_hydro_split(const float *qL, const float
                                                     const float *gR, float pe, float gm, float mach_cutoff,
                                                     float *flux, bool flat = false, bool all_mach = false) {
   constexpr int IP = 1 + DIM, IAS = 2 + DIM;
-  const float igmm1 = 1.0f / (gm - 1.0f);
-  float rhoL = qL[0], inv_rhoL = 1.0f / rhoL, vx1L = qL[1], vx2L = qL[2], vx3L = DIM == 3 ? qL[3] : 0.0f;
-  float v2L = vx1L * vx1L + vx2L * vx2L + vx3L * vx3L;
-  float pLd = qL[IP], pL = pe + pLd, eint, cL, cR;
-  if (EOSM == EOS_FAST) { eint = pL / (gL[0] - 1.0f); cL = sqrtf(gL[1] * pL * inv_rhoL); }
-  else if (EOSM == EOS_GIVEN) { eint = gL[0]; cL = gL[1]; }
-  else { eint = igmm1 * pL; cL = sqrtf(gm * pL * inv_rhoL); }
-  float rhoeL = eint + 0.5f * rhoL * v2L;
-  float rhoR = qR[0], inv_rhoR = 1.0f / rhoR, vx1R = qR[1], vx2R = qR[2], vx3R = DIM == 3 ? qR[3] : 0.0f;
-  float v2R = vx1R * vx1R + vx2R * vx2R + vx3R * vx3R;
-  float pRd = qR[IP], pR = pe + pRd;
-  if (EOSM == EOS_FAST) { eint = pR / (gR[0] - 1.0f); cR = sqrtf(gR[1] * pR * inv_rhoR); }
-  else if (EOSM == EOS_GIVEN) { eint = gR[0]; cR = gR[1]; }
-  else { eint = igmm1 * pR; cR = sqrtf(gm * pR * inv_rhoR); }
-  float rhoeR = eint + 0.5f * rhoR * v2R;
-  float max_c = fmaxf(cL, cR);
-  float sL = fminf(vx1L, vx1R) - max_c;
-  float sR = fmaxf(vx1L, vx1R) + max_c;
-  float dsuL = sL - vx1L, dsuR = sR - vx1R;
-  float ustar = ((pRd - pLd) + rhoL * vx1L * dsuL - rhoR * vx1R * dsuR) / (rhoL * dsuL - rhoR * dsuR);
-  float rhostarL = rhoL * (dsuL / (sL - ustar));
-  float rhoestarL = rhostarL * (rhoeL * inv_rhoL + (ustar - vx1L) * (ustar + pL * inv_rhoL / dsuL));
-  float rhostarR = rhoR * (dsuR / (sR - ustar));
-  float rhoestarR = rhostarR * (rhoeR * inv_rhoR + (ustar - vx1R) * (ustar + pR * inv_rhoR / dsuR));
+  constexpr bool D3 = DIM == 3;
+  // pairs: .x left, .y right
+  const float2 rho2 = make_float2(qL[0], qR[0]), u2 = make_float2(qL[1], qR[1]), v2v = make_float2(qL[2], qR[2]);
+  const float2 w2 = D3 ? make_float2(qL[3], qR[3]) : f2dup(0.0f);
+  const float2 pd2 = make_float2(qL[IP], qR[IP]), p2 = f2add(f2dup(pe), pd2);
+  const float2 irho = f2rcp(rho2), pr2 = f2mul(p2, irho);
+  float2 vsq = f2fma(v2v, v2v, f2mul(u2, u2));
+  if (D3) vsq = f2fma(w2, w2, vsq);
+  float2 eint, csq, cs;
+  if (EOSM == EOS_FAST) {
+    eint = f2mul(p2, f2rcp(make_float2(gL[0] - 1.0f, gR[0] - 1.0f)));
+    csq = f2mul(make_float2(gL[1], gR[1]), pr2);
+    cs = make_float2(sqrtf(csq.x), sqrtf(csq.y));
+  } else if (EOSM == EOS_GIVEN) {
+    eint = make_float2(gL[0], gR[0]);
+    cs = make_float2(gL[1], gR[1]);
+    csq = f2mul(cs, cs);
+  } else {
+    eint = f2mul(p2, f2dup(1.0f / (gm - 1.0f)));
+    csq = f2mul(f2dup(gm), pr2);
+    cs = make_float2(sqrtf(csq.x), sqrtf(csq.y));
+  }
+  const float2 rhoe2 = f2fma(f2mul(f2dup(0.5f), rho2), vsq, eint);
+  const float max_c = fmaxf(cs.x, cs.y);
+  float sL = fminf(u2.x, u2.y) - max_c;
+  float sR = fmaxf(u2.x, u2.y) + max_c;
+  const float2 s2 = make_float2(sL, sR), dsu2 = f2sub(s2, u2), rd2 = f2mul(rho2, dsu2), rdu2 = f2mul(rd2, u2);
+  const float ustar = ((pd2.y - pd2.x) + rdu2.x - rdu2.y) / (rd2.x - rd2.y);
+  const float2 us2 = f2dup(ustar), du2 = f2sub(us2, u2);
+  const float2 rs2 = f2mul(rd2, f2rcp(f2sub(s2, us2)));  // rho*
+  const float2 rhoes2 = f2mul(rs2, f2fma(du2, f2fma(pr2, f2rcp(dsu2), us2), f2mul(rhoe2, irho)));
   if (flat) {
     // HLL on a flattened face (USE_SHOCK_FLATTENING, source.F90:15929-16010); the momentum
     // flux takes the pressure deviations, sR pe - sL pe over sR - sL being exactly pe
     sL = fminf(0.0f, sL);
     sR = fmaxf(0.0f, sR);
+    const float rhoL = rho2.x, rhoR = rho2.y, vx1L = u2.x, vx1R = u2.y, vx2L = v2v.x, vx2R = v2v.y, vx3L = w2.x;
+    const float vx3R = w2.y, rhoeL = rhoe2.x, rhoeR = rhoe2.y, pLd = pd2.x, pRd = pd2.y, pL = p2.x, pR = p2.y;
     float UL[NV], UR[NV], fL[NV], fR[NV];
     UL[0] = rhoL; UL[1] = rhoL * vx1L; UL[2] = rhoL * vx2L; if (DIM == 3) UL[3] = rhoL * vx3L; UL[IP] = rhoeL;
     UR[0] = rhoR; UR[1] = rhoR * vx1R; UR[2] = rhoR * vx2R; if (DIM == 3) UR[3] = rhoR * vx3R; UR[IP] = rhoeR;
@@ -138,44 +146,41 @@ __device__ __forceinline__ void riemann_hydro_split(const float *qL, const float
     return;
   }
   if (RIEM == R_LHLLC) {
-    float machL = sqrtf(v2L) / cL, machR = sqrtf(v2R) / cR;
-    float chi = fminf(1.0f, fmaxf(machL, machR));
-    chi = fmaxf(mach_cutoff, chi);
-    float phi = chi * (2.0f - chi);
-    float rhobar = 0.5f * (rhoL + rhoR), cbar = 0.5f * (cL + cR);
-    float pstar_d = 0.5f * (pLd + pRd) - 0.5f * phi * rhobar * cbar * (vx1R - vx1L);
+    // the Mach numbers compared as squares: one square root, for the larger
+    const float2 m2 = f2mul(vsq, f2rcp(csq));
+    const float chi = fmaxf(mach_cutoff, fminf(1.0f, sqrtf(fmaxf(m2.x, m2.y))));
+    const float phi = chi * (2.0f - chi);
+    const float pstar_d = 0.5f * (pd2.x + pd2.y) -
+                          0.125f * phi * (rho2.x + rho2.y) * (cs.x + cs.y) * (u2.y - u2.x);
     if (all_mach && (sL > 0.0f || sR < 0.0f)) {
       // FLUX_IS_ALL_MACH: the upwind state outside the wave fan, pe removed from the momentum flux
       const bool left = sL > 0.0f;
-      const float *q = left ? qL : qR;
-      float rho = left ? rhoL : rhoR, vx1 = left ? vx1L : vx1R, vx2 = left ? vx2L : vx2R, vx3 = left ? vx3L : vx3R;
-      float p = left ? pL : pR, pd = left ? pLd : pRd, rhoe = left ? rhoeL : rhoeR;
-      flux[0] = rho * vx1;
-      flux[1] = rho * vx1 * vx1 + pd;
-      flux[2] = rho * vx1 * vx2;
-      if (DIM == 3) flux[3] = rho * vx1 * vx3;
-      flux[IP] = (rhoe + p) * vx1;
+      const float m = left ? rho2.x * u2.x : rho2.y * u2.y, vx1 = left ? u2.x : u2.y;
+      flux[0] = m;
+      flux[1] = m * vx1 + (left ? pd2.x : pd2.y);
+      flux[2] = m * (left ? v2v.x : v2v.y);
+      if (D3) flux[3] = m * (left ? w2.x : w2.y);
+      flux[IP] = (left ? rhoe2.x + p2.x : rhoe2.y + p2.y) * vx1;
 #pragma unroll
-      for (int iv = IAS; iv < NV; ++iv) flux[iv] = rho * q[iv] * vx1;
+      for (int iv = IAS; iv < NV; ++iv) flux[iv] = m * (left ? qL[iv] : qR[iv]);
       return;
     }
-    float sgn = copysignf(1.0f, ustar);
-    float hp = 0.5f * (1.0f + sgn), hm = 0.5f * (1.0f - sgn);
-    float rhostar = hp * rhostarL + hm * rhostarR;
-    float mflux = rhostar * ustar;
-    flux[0] = mflux;
-    flux[1] = mflux * ustar + pstar_d;
-    flux[2] = mflux * (hp * vx2L + hm * vx2R);
-    if (DIM == 3) flux[3] = mflux * (hp * vx3L + hm * vx3R);
-    flux[IP] = (hp * rhoestarL + hm * rhoestarR + (pe + pstar_d)) * ustar;
+    const bool left = !signbit(ustar);
+    const float m = (left ? rs2.x : rs2.y) * ustar;
+    flux[0] = m;
+    flux[1] = m * ustar + pstar_d;
+    flux[2] = m * (left ? v2v.x : v2v.y);
+    if (D3) flux[3] = m * (left ? w2.x : w2.y);
+    flux[IP] = ((left ? rhoes2.x : rhoes2.y) + (pe + pstar_d)) * ustar;
 #pragma unroll
-    for (int iv = IAS; iv < NV; ++iv) flux[iv] = mflux * (hp * qL[iv] + hm * qR[iv]);
+    for (int iv = IAS; iv < NV; ++iv) flux[iv] = m * (left ? qL[iv] : qR[iv]);
   } else {
     const bool left = ustar > 0.0f;
     const float *q = left ? qL : qR;
-    float rho = left ? rhoL : rhoR, vx1 = left ? vx1L : vx1R, vx2 = left ? vx2L : vx2R, vx3 = left ? vx3L : vx3R;
-    float p = left ? pL : pR, pd = left ? pLd : pRd, rhoe = left ? rhoeL : rhoeR;
-    float rhostar = left ? rhostarL : rhostarR, rhoestar = left ? rhoestarL : rhoestarR, s = left ? sL : sR;
+    const float rho = left ? rho2.x : rho2.y, vx1 = left ? u2.x : u2.y, vx2 = left ? v2v.x : v2v.y;
+    const float vx3 = left ? w2.x : w2.y, p = left ? p2.x : p2.y, pd = left ? pd2.x : pd2.y;
+    const float rhoe = left ? rhoe2.x : rhoe2.y, rhostar = left ? rs2.x : rs2.y;
+    const float rhoestar = left ? rhoes2.x : rhoes2.y, s = left ? sL : sR;
     const bool sup = left ? (sL >= 0.0f) : (sR < 0.0f);
     float U[NV], f[NV];
     U[0] = rho; U[1] = rho * vx1; U[2] = rho * vx2; if (DIM == 3) U[3] = rho * vx3; U[IP] = rhoe;
@@ -483,23 +488,6 @@ __device__ __forceinline__ long long dir_stride(const Geo &g, int d) {
   return d == 0 ? 1 : (d == 1 ? (long long)g.nx[0] : (long long)g.nx[0] * g.nx[1]);
 }
 
-// States of the four cells m-2..m+1 around the low face of cell m: variable iv of cell s is
-// w(s, iv), FASTEOS gamma q is g(s, q).
-template <int NV>
-struct RegCells {
-  const float *w_[6], *g_[6];
-  __device__ __forceinline__ float w(int s, int iv) const { return w_[s][iv]; }
-  __device__ __forceinline__ float g(int s, int q) const { return g_[s][q]; }
-};
-// cells in a shared-memory array: variable iv of cell s at base[off[s] + iv * vs]
-template <int NV>
-struct SmemCells {
-  const float *base;
-  int off[4], vs;
-  __device__ __forceinline__ float w(int s, int iv) const { return base[off[s] + iv * vs]; }
-  __device__ __forceinline__ float g(int s, int q) const { return base[off[s] + (NV + q) * vs]; }
-};
-
 // the per-side helm_rhoP_given of the split form, out of line: the split stage kernels call it
 // twice per face, and an inlined Helmholtz evaluation at each site costs them their registers.
 // It runs the contracted-coefficient evaluation of phl_eos_fast.cuh (the FP64 form keeps the
@@ -577,91 +565,6 @@ __device__ __forceinline__ void flatten_gamma_x1(const float gv[2][6], bool fa, 
   }
 }
 
-// flux through the low face of cell m along d from the FP32 deviation states of cells m-2..m+1
-template <class C, class Cells>
-__device__ __forceinline__ void face_flux_cells(const Prm &P, int d, int fi, int fj, int fk, const Cells &cl,
-                                                float F[C::NV]) {
-  constexpr int NV = C::NV, IP = C::IP, SW = C::SW;
-  const Geo &g = P.g;
-  // cl holds cells m-SW .. m+SW-1; v[] of rec_face_f32 holds cells m-3 .. m+2
-  // USE_SHOCK_FLATTENING: is_flattened of cells m-1 (fa) and m (fb); a flagged cell's edges
-  // fall back to LIM2ND PLM, and the face takes the HLL flux
-  bool fa = false, fb = false;
-  if (C::SF) {
-    fa = P.sf_flag[sf_flag_index<C>(g, fi - (d == 0), fj - (d == 1), fk - (d == 2))] != 0;
-    fb = P.sf_flag[sf_flag_index<C>(g, fi, fj, fk)] != 0;
-  }
-  float qL[NV], qR[NV];
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    float v[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) v[q] = (q >= 3 - SW && q < 3 + SW) ? cl.w(q - (3 - SW), iv) : 0.0f;
-    rec_face_f32<C>(v, C::REC == REC_LIM5TH || iv >= C::IAS, qL[iv], qR[iv]);
-    if (C::SF && C::REC != REC_LIM2ND) flatten_face_f32(v, fa, fb, qL[iv], qR[iv]);
-  }
-  if (d == 1) {
-    float a = qL[1], b = qL[2]; qL[1] = b; qL[2] = -a;
-    a = qR[1]; b = qR[2]; qR[1] = b; qR[2] = -a;
-  } else if (C::DIM == 3 && d == 2) {
-    float a = qL[1], b = qL[2], c = qL[3]; qL[1] = c; qL[2] = a; qL[3] = b;
-    a = qR[1]; b = qR[2]; c = qR[3]; qR[1] = c; qR[2] = a; qR[3] = b;
-  }
-  float pe = 0.0f;
-  long long fbg = 0;
-  if (C::WB || C::ETOT) fbg = bg_face(g, d, fi, fj, fk);
-  float4 bg = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (C::WB) {
-    bg = __ldg(P.sf_bg[d] + fbg);
-    qL[0] = bg.x + qL[0];
-    qR[0] = bg.x + qR[0];
-    pe = bg.y;
-  }
-  float gL[2] = {0.f, 0.f}, gR[2] = {0.f, 0.f};
-  if (C::FAST) {
-    const bool late = C::SF && C::WB && d == 0;
-    float gv[2][6];
-#pragma unroll
-    for (int iv = 0; iv < 2; ++iv) {
-#pragma unroll
-      for (int q = 0; q < 6; ++q) gv[iv][q] = (q >= 3 - SW && q < 3 + SW) ? cl.g(q - (3 - SW), iv) : 0.0f;
-      rec_face_f32<C>(gv[iv], C::REC == REC_LIM5TH, gL[iv], gR[iv]);
-      if (C::SF && C::REC != REC_LIM2ND && !late) flatten_face_f32(gv[iv], fa, fb, gL[iv], gR[iv]);
-    }
-    if (C::WB) {
-      const float ge = bg.z;
-      gL[0] = gL[0] + ge;
-      gR[0] = gR[0] + ge;
-      if (late) flatten_gamma_x1(gv, fa, fb, ge, gL, gR);
-    }
-  } else if (C::HELM) {
-    // without USE_FASTEOS the first gamma slot holds the stage input's temperature
-    const float tface = 0.5f * (cl.g(SW - 1, 0) + cl.g(SW, 0));
-    split_side_eos<C>(P, qL, pe, tface, gL[0], gL[1]);
-    split_side_eos<C>(P, qR, pe, tface, gR[0], gR[1]);
-  }
-  riemann_hydro_split<C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, gL, gR, pe, (float)g.gm, (float)g.mach_cutoff, F,
-                                                    C::SF && (fa || fb), g.all_mach != 0);
-  if (d == 1) {
-    float a = F[1], b = F[2]; F[1] = -b; F[2] = a;
-  } else if (C::DIM == 3 && d == 2) {
-    float a = F[1], b = F[2], c = F[3]; F[1] = b; F[2] = c; F[3] = a;
-  }
-  if (C::ETOT) F[IP] = F[IP] + F[0] * bg.w;
-}
-
-template <class C>
-__device__ __forceinline__ void face_flux_split(const Prm &P, int d, int fi, int fj, int fk, const float *const *w,
-                                                const float *const *gm, float F[C::NV]) {
-  RegCells<C::NV> cl;
-#pragma unroll
-  for (int q = 0; q < 2 * C::SW; ++q) {
-    cl.w_[q] = w[q];
-    cl.g_[q] = gm[q];
-  }
-  face_flux_cells<C>(P, d, fi, fj, fk, cl, F);
-}
-
 // --------------------------------------------------------------------- split stage kernels
 // Per-cell statistics of a stage, reduced once per block.
 // per-thread counters (32-bit: a thread's cells times 100 iterations stay far below 2^32; the
@@ -671,113 +574,6 @@ struct SplitStat {
   unsigned calls = 0, iters = 0, nonconv = 0, clamp = 0, bad = 0;
   unsigned mlp_acc = 0, mlp_rej = 0, gevals = 0;  // learned guess in the step
 };
-
-// Everything of a stage after the flux divergence, for one cell: flux divergence to physical
-// units, gravity, RK combine (FP64), cons -> prim with the Helmholtz Newton (FP64), FP32
-// deviations out, and the cell's CFL speed in the last stage.  res: divergence in scaled units.
-template <class C>
-__device__ __forceinline__ void split_cell_update(const Prm &P, long long c, int i, int j, int k,
-                                                  const float res[C::NV], float rho_dev, SplitStat &st) {
-  constexpr int NV = C::NV, IP = C::IP, IAS = C::IAS, DIM = C::DIM;
-  const Geo &g = P.g;
-  const double dt = P.scal[1];
-  // the Newton's warm start, loaded before the state stores so that its latency overlaps them
-  const double Tw = C::HELM ? P.temp[c] : 0.0;
-  // back to physical units: mass and scalar fluxes scale with rho_ref v_ref, momentum with
-  // p_ref, energy with p_ref v_ref
-  const double fm = P.rho_ref * P.v_ref, fe = P.p_ref * P.v_ref;
-  double rd[NV];
-  rd[0] = (double)res[0] * fm;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) rd[1 + d] = (double)res[1 + d] * P.p_ref;
-  rd[IP] = (double)res[IP] * fe;
-#pragma unroll
-  for (int iv = IAS; iv < NV; ++iv) rd[iv] = (double)res[iv] * fm;
-  const long long bc = bg_cc(g, i, j, k);
-  if (C::GRAV) {
-    const double rho_dev_phys = (double)rho_dev * P.rho_ref;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d)
-      rd[1 + d] -= rho_dev_phys * __ldg(P.grav + (long long)d * (g.bg_profile ? g.nx[1] : g.N) + bc);
-  }
-  double u0[NV], u[NV];
-  if (P.first_stage) {
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) {
-      u0[iv] = P.U[(long long)iv * g.N + c];
-      u[iv] = u0[iv];
-      P.U0[(long long)iv * g.N + c] = u0[iv];
-    }
-  } else {
-#pragma unroll
-    for (int iv = 0; iv < NV; ++iv) {
-      u0[iv] = P.U0[(long long)iv * g.N + c];
-      u[iv] = P.U[(long long)iv * g.N + c];
-    }
-  }
-  if (g.use_acc) constant_acceleration<DIM, IP>(g, u, rd);
-  const double a1 = P.a1, a2 = P.a2, a3 = P.c3 * dt;
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    u[iv] = a1 * u0[iv] + a2 * u[iv] + a3 * rd[iv];
-    P.U[(long long)iv * g.N + c] = u[iv];
-  }
-  // cons -> prim + EoS in FP64
-  double rho = u[0], inv_rho = 1.0 / rho;
-  double ke = u[1] * u[1] + u[2] * u[2] + (DIM == 3 ? u[3] * u[3] : 0.0);
-  double eint = u[IP] - 0.5 * ke * inv_rho;
-  if (C::ETOT) eint = eint - rho * __ldg(P.phi_cc + bc);
-  double p, T, sound = 0.0;
-  if (C::HELM) {
-    double ye = u[IAS] * inv_rho, inv_abar = u[IAS + 1] * inv_rho;
-    T = Tw;
-    int clamped = 0;
-    bool conv = false;
-    HelmCell hc;
-    helm_cell_init_rho(P.helm, hc, rho, ye);
-    helm_cell_contract(P.helm, hc, helm_node_index(P.helm.T, P.helm.nT, P.helm.log10_T1, P.helm.dT, T));
-    int it = helm_rhoe_fast(P.helm, hc, inv_rho, eint * inv_rho, inv_abar, T, 100, clamped, conv);
-    st.calls += 1; st.iters += it; st.nonconv += !conv; st.clamp += clamped;
-    double sound2;
-    helm_cell_p_sound2(P.helm, hc, rho, inv_rho, T, inv_abar, p, sound2);
-    if (P.last_stage) sound = sqrt(sound2);
-    if (C::FAST) {
-      // gamma_e to FP32 as a deviation from equilibrium (formed in FP64), gamma_c to FP32 as it is
-      double ge = p / eint + 1.0;
-      const float gc = (float)(sound2 * rho) / (float)p;
-      if (C::WB) ge = ge - __ldg(P.eq_ge_cc + bc);
-      P.gf_out[c] = (float)ge;
-      P.gf_out[g.N + c] = gc;
-    } else {
-      P.gf_out[c] = (float)T;
-    }
-  } else {
-    p = (g.gm - 1.0) * eint;
-    T = p / (rho * CONST_RGAS * (1.0 / g.mu));
-    sound = sqrt(g.gm * p / rho);
-  }
-  double rdev = rho, pdev = p;
-  if (C::WB) {
-    rdev = rho - __ldg(P.eq_rho_cc + bc);
-    pdev = p - __ldg(P.eq_p_cc + bc);
-  }
-  P.Wf_out[c] = (float)(rdev * P.inv_rho_ref);
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) P.Wf_out[(long long)(1 + d) * g.N + c] = (float)(u[1 + d] * inv_rho * P.inv_v_ref);
-  P.Wf_out[(long long)IP * g.N + c] = (float)(pdev * P.inv_p_ref);
-#pragma unroll
-  for (int iv = IAS; iv < NV; ++iv) P.Wf_out[(long long)iv * g.N + c] = (float)(u[iv] * inv_rho);
-  P.temp[c] = T;
-  P.eint[c] = eint;
-  if (!(rho > 0.0) || !(p > 0.0) || !(T > 0.0) || !isfinite(eint)) st.bad += 1;
-  if (P.last_stage) {
-    double sx1 = (fabs(u[1] * inv_rho) + sound) * g.inv_dx[0];
-    double sx2 = (fabs(u[2] * inv_rho) + sound) * g.inv_dx[1];
-    double sm = sx1 + sx2;
-    if (DIM == 3) sm = (fabs(u[3] * inv_rho) + sound) * g.inv_dx[2] + sm;
-    st.smax = fmax(st.smax, sm);
-  }
-}
 
 template <class C>
 __device__ __forceinline__ void split_stat_flush(const Prm &P, const SplitStat &st) {
@@ -798,270 +594,13 @@ __device__ __forceinline__ void split_stat_flush(const Prm &P, const SplitStat &
   }
 }
 
-// One thread per cell; every face is solved by both of its cells.  Any grid size.
-template <class C>
-__global__ void __launch_bounds__(128) k_stage_split(Prm P) {
-  if (!*P.active) return;
-  constexpr int NV = C::NV, DIM = C::DIM;
-  const Geo &g = P.g;
-  long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  SplitStat st;
-  if (c < g.N) {
-    int i, j, k;
-    unflatten3(c, g.div0[0], g.div1[0], i, j, k);
-    float res[NV];
-    float rho_dev = 0.0f;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      // cells c-SW .. c+SW along d: the low face reads the first 2 SW, the high face the last
-      constexpr int NS = 2 * C::SW + 1;
-      float w[NS][NV], gmv[NS][2];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        int ii = i + (d == 0 ? s - C::SW : 0), jj = j + (d == 1 ? s - C::SW : 0), kk = k + (d == 2 ? s - C::SW : 0);
-        load_wf<C>(P, ii, jj, kk, w[s], gmv[s]);
-      }
-      if (d == 0) rho_dev = w[C::SW][0];
-      const float *wp[NS], *gp[NS];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        wp[s] = w[s];
-        gp[s] = gmv[s];
-      }
-      float Flo[NV], Fhi[NV];
-      face_flux_split<C>(P, d, i, j, k, wp, gp, Flo);
-      face_flux_split<C>(P, d, i + (d == 0), j + (d == 1), k + (d == 2), wp + 1, gp + 1, Fhi);
-      const float inv_dl = (float)g.inv_dx[d];
-#pragma unroll
-      for (int iv = 0; iv < NV; ++iv) {
-        float dd = (Fhi[iv] - Flo[iv]) * inv_dl;
-        res[iv] = d == 0 ? dd : res[iv] + dd;
-      }
-    }
-    split_cell_update<C>(P, c, i, j, k, res, rho_dev, st);
-  }
-  split_stat_flush<C>(P, st);
-}
-
-// 4-byte asynchronous global -> shared copy (cp.async, completes at the next wait)
-__device__ __forceinline__ void cp_async4(float *smem_dst, const float *gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
+// 8-byte asynchronous global -> shared copy (cp.async, completes at the next wait)
 __device__ __forceinline__ void cp_async8(double *smem_dst, const double *gmem_src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Start the copy of the FP32 state of a (possibly ghost) cell into shared memory (variable q at
-// dst[q * vs]); returns the velocity components to negate once the copy has landed (bit d for
-// a mirrored dimension d, as load_wf does).
-template <class C>
-__device__ __forceinline__ void load_wf_async(const Prm &P, int i, int j, int k, float *dst, int vs) {
-  const Geo &g = P.g;
-  bool f0 = false, f1 = false, f2 = false;
-  int si = map_index(i, g.nx[0], g.bc[0][0], g.bc[0][1], f0);
-  int sj = map_index(j, g.nx[1], g.bc[1][0], g.bc[1][1], f1);
-  int sk = map_index(k, g.nx[2], g.bc[2][0], g.bc[2][1], f2);
-  long long c = lin(g, si, sj, sk);
-#pragma unroll
-  for (int iv = 0; iv < C::NV; ++iv) cp_async4(dst + iv * vs, P.Wf_in + (long long)iv * g.N + c);
-  if (C::HELM) {
-    cp_async4(dst + C::NV * vs, P.gf_in + c);
-    cp_async4(dst + (C::NV + 1) * vs, P.gf_in + g.N + c);
-  }
-}
-// after the copy of cell (i, j, k) has landed: negate the velocity components of its mirrored
-// dimensions (what load_wf does on load)
-__device__ __forceinline__ void fix_mirrored(const Geo &g, int i, int j, int k, float *dst, int vs) {
-  bool f[3] = {false, false, false};
-  map_index(i, g.nx[0], g.bc[0][0], g.bc[0][1], f[0]);
-  map_index(j, g.nx[1], g.bc[1][0], g.bc[1][1], f[1]);
-  map_index(k, g.nx[2], g.bc[2][0], g.bc[2][1], f[2]);
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (f[d]) dst[(1 + d) * vs] = -dst[(1 + d) * vs];
-}
-
-// 3D, face reuse: a block owns TX x TY columns of cells in (x1, x2) and marches KZ planes along
-// x3.  Deviation states live in a shared-memory ring of five planes (k-1 .. k+3), each with a
-// 2-cell halo in x1 and x2, filled by asynchronous copies one plane ahead of use.  Each x1 and
-// x2 face of plane k is solved once into shared memory and each x3 face once per column (the
-// upper face of plane k is the lower face of plane k+1, kept in registers): 3.16 solves per cell
-// against 6 in k_stage_split.  The divergence sums the three directions in the same order as
-// k_stage_split.  Requires nx1 % TX == nx2 % TY == nx3 % KZ == 0, blockDim.x == TX * TY and
-// SplitTile<C, TX, TY>::bytes() of dynamic shared memory.
-template <class C, int TX, int TY>
-struct SplitTile {
-  static constexpr int NQ = C::NV + (C::HELM ? 2 : 0);  // stored values per cell
-  // plane rows are TX + 8 wide with the tile at x offset XO = 4: a tensor copy of the plane
-  // starts at x = i0 - 4, a multiple of 4 floats (16 bytes) as bulk tensor copies require;
-  // the faces read x offsets 2 .. TX + 5
-  static constexpr int XO = 4, SX = TX + 8, SY = TY + 4, PL = SX * SY;
-  static constexpr int NSLOT = 5;
-  static constexpr int RING = NSLOT * NQ * PL;           // floats: [slot][q][y][x]
-  static constexpr int FX = C::NV * TY * (TX + 1), FY = C::NV * (TY + 1) * TX;
-  static constexpr int PLANE_BYTES = NQ * PL * 4;        // one staged plane, all fields
-  static_assert(PLANE_BYTES % 128 == 0, "slots stay 128-byte aligned");
-  static constexpr size_t MBAR_OFFSET = sizeof(float) * (size_t)(RING + FX + FY);  // 8-byte aligned
-  static constexpr size_t bytes() { return MBAR_OFFSET + 8 * NSLOT; }
-};
-
-// Tensor maps of the stage's FP32 input for the bulk tensor copies: W' as a 4D tensor
-// (x1, x2, x3, variable) and the two FASTEOS gammas likewise; box = one plane of the tile with
-// its halo, all variables.
-struct SplitMaps {
-  CUtensorMap w, g;
-};
-constexpr int SPLIT_TMA_POLLS = 1 << 22;  // mbarrier polls before a stalled copy is reported
-
-template <class C, int TX, int TY, int KZ>
-__global__ void __launch_bounds__(TX * TY, 2) k_stage_split_tiled(Prm P, const __grid_constant__ SplitMaps maps,
-                                                                  int use_tma) {
-  if (!*P.active) return;
-  using T = SplitTile<C, TX, TY>;
-  constexpr int NV = C::NV, NQ = T::NQ, SX = T::SX, PL = T::PL, VS = PL, XO = T::XO;
-  static_assert(C::DIM == 3, "tiled stage is 3D");
-  constexpr int NHALO = 4 * TX + 4 * TY;  // halo cells the x1 and x2 faces read (no corners)
-  static_assert(NHALO <= TX * TY, "one halo cell per thread");
-  extern __shared__ __align__(128) float smem[];
-  float *ring = smem;                      // [5][NQ][SY][SX]
-  float *fx = smem + T::RING;              // [NV][TY][TX+1]
-  float *fy = fx + T::FX;                  // [NV][TY+1][TX]
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(smem) + T::MBAR_OFFSET);
-  const Geo &g = P.g;
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY, k0 = blockIdx.z * KZ;
-  const int i = i0 + tx, j = j0 + ty;
-  const float idx = (float)g.inv_dx[0], idy = (float)g.inv_dx[1], idz = (float)g.inv_dx[2];
-  const int own = (ty + 2) * SX + (tx + XO);  // own cell inside a plane
-  auto slot = [&](int k) { return ((k - k0 + 2) % T::NSLOT) * NQ * PL; };
-  SplitStat st;
-  // Interior tiles (the plane with its halo lies inside the domain in x1 and x2, x3 periodic)
-  // stage whole planes with bulk tensor copies; the others copy cell by cell with cp.async,
-  // mapping ghost indices and mirroring velocities.
-  const bool tma = use_tma && blockIdx.x >= 1 && blockIdx.x + 2 <= gridDim.x && blockIdx.y >= 1 &&
-                   blockIdx.y + 2 <= gridDim.y;
-  auto plane_copy = [&](int k) {
-    // one thread: arm the slot's barrier and copy plane k (x3 wrapped) with all variables
-    const int s = (k - k0 + 2) % T::NSLOT;
-    int kz = k % g.nx[2];
-    if (kz < 0) kz += g.nx[2];
-    mbar_arrive_expect_tx(mbar + s, T::PLANE_BYTES);
-    tma_load_4d(ring + s * NQ * PL, &maps.w, mbar + s, i0 - XO, j0 - 2, kz, 0);
-    if (NQ > NV) tma_load_4d(ring + s * NQ * PL + NV * PL, &maps.g, mbar + s, i0 - XO, j0 - 2, kz, 0);
-  };
-  auto plane_wait = [&](int k) {
-    // all threads: the n-th use of a slot completes phase n
-    const int u = k - k0 + 2, s = u % T::NSLOT;
-    if (!mbar_wait_bounded(mbar + s, (uint32_t)((u / T::NSLOT) & 1), SPLIT_TMA_POLLS) && threadIdx.x == 0)
-      atomicAdd(P.stat + STAT_TC_STALLED, 1ull);
-  };
-  // this thread's halo cell (x1/x2 halo of every plane) for the cell-by-cell path, if any
-  int hcell = -1, hx = 0, hy = 0;
-  if ((int)threadIdx.x < NHALO) {
-    const int h = threadIdx.x;
-    if (h < 4 * TX) {
-      const int r = h / TX;
-      hx = XO + h % TX;
-      hy = r < 2 ? r : TY + r;
-    } else {
-      const int h3 = h - 4 * TX, cc = h3 / TY;
-      hy = 2 + h3 % TY;
-      hx = cc < 2 ? XO - 2 + cc : XO + TX + cc - 2;
-    }
-    hcell = hy * SX + hx;
-  }
-  if (tma) {
-    if (threadIdx.x < T::NSLOT) mbar_init(mbar + threadIdx.x, 1);
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = k0 - 2; k <= k0 + 2; ++k) plane_copy(k);
-    for (int k = k0 - 2; k <= k0 + 2; ++k) plane_wait(k);
-  } else {
-    // prologue: planes k0-2 .. k0+2 of the own column, halo of plane k0
-    for (int k = k0 - 2; k <= k0 + 2; ++k) load_wf_async<C>(P, i, j, k, ring + slot(k) + own, VS);
-    if (hcell >= 0) load_wf_async<C>(P, i0 + hx - XO, j0 + hy - 2, k0, ring + slot(k0) + hcell, VS);
-    cp_async_commit();
-    cp_async_wait_all();
-    for (int k = k0 - 2; k <= k0 + 2; ++k) fix_mirrored(g, i, j, k, ring + slot(k) + own, VS);
-    if (hcell >= 0) fix_mirrored(g, i0 + hx - XO, j0 + hy - 2, k0, ring + slot(k0) + hcell, VS);
-  }
-  __syncthreads();
-  float fz_lo[NV], fz_hi[NV];
-  {
-    SmemCells<NV> cl{ring, {slot(k0 - 2) + own, slot(k0 - 1) + own, slot(k0) + own, slot(k0 + 1) + own}, VS};
-    face_flux_cells<C>(P, 2, i, j, k0, cl, fz_lo);
-  }
-
-#pragma unroll 1
-  for (int kk = 0; kk < KZ; ++kk) {
-    const int k = k0 + kk;
-    const int sk = slot(k);
-    // next copies: plane k+3 (tensor copy of the whole plane, or the own column) and the halo
-    // of plane k+1 (cell-by-cell path); neither is read during this plane
-    const bool next_own = kk + 3 <= KZ + 1, next_halo = !tma && kk + 1 < KZ && hcell >= 0;
-    if (tma) {
-      if (next_own && threadIdx.x == 0) plane_copy(k + 3);
-    } else {
-      if (next_own) load_wf_async<C>(P, i, j, k + 3, ring + slot(k + 3) + own, VS);
-      if (next_halo) load_wf_async<C>(P, i0 + hx - XO, j0 + hy - 2, k + 1, ring + slot(k + 1) + hcell, VS);
-      cp_async_commit();
-    }
-    {
-      float F[NV];
-      // low x1 face of the own cell
-      SmemCells<NV> cx{ring, {sk + own - 2, sk + own - 1, sk + own, sk + own + 1}, VS};
-      face_flux_cells<C>(P, 0, i, j, k, cx, F);
-#pragma unroll
-      for (int q = 0; q < NV; ++q) fx[(q * TY + ty) * (TX + 1) + tx] = F[q];
-      // low x2 face of the own cell
-      SmemCells<NV> cy{ring, {sk + own - 2 * SX, sk + own - SX, sk + own, sk + own + SX}, VS};
-      face_flux_cells<C>(P, 1, i, j, k, cy, F);
-#pragma unroll
-      for (int q = 0; q < NV; ++q) fy[(q * (TY + 1) + ty) * TX + tx] = F[q];
-      if (ty == 0) {
-        // upper x2 face of the tile, column tx
-        const int c = (TY + 2) * SX + tx + XO;
-        SmemCells<NV> cu{ring, {sk + c - 2 * SX, sk + c - SX, sk + c, sk + c + SX}, VS};
-        face_flux_cells<C>(P, 1, i, j0 + TY, k, cu, F);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) fy[(q * (TY + 1) + TY) * TX + tx] = F[q];
-      } else if (ty == 1 && tx < TY) {
-        // upper x1 face of the tile, row tx
-        const int c = (tx + 2) * SX + TX + XO;
-        SmemCells<NV> cr{ring, {sk + c - 2, sk + c - 1, sk + c, sk + c + 1}, VS};
-        face_flux_cells<C>(P, 0, i0 + TX, j0 + tx, k, cr, F);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) fx[(q * TY + tx) * (TX + 1) + TX] = F[q];
-      }
-      // upper x3 face of the own cell
-      SmemCells<NV> cz{ring, {slot(k - 1) + own, sk + own, slot(k + 1) + own, slot(k + 2) + own}, VS};
-      face_flux_cells<C>(P, 2, i, j, k + 1, cz, fz_hi);
-    }
-    __syncthreads();
-    float res[NV];
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      float dd = (fx[(q * TY + ty) * (TX + 1) + tx + 1] - fx[(q * TY + ty) * (TX + 1) + tx]) * idx;
-      dd = dd + (fy[(q * (TY + 1) + ty + 1) * TX + tx] - fy[(q * (TY + 1) + ty) * TX + tx]) * idy;
-      res[q] = dd + (fz_hi[q] - fz_lo[q]) * idz;
-      fz_lo[q] = fz_hi[q];
-    }
-    split_cell_update<C>(P, lin(g, i, j, k), i, j, k, res, ring[sk + own], st);
-    if (tma) {
-      if (next_own) plane_wait(k + 3);
-    } else {
-      cp_async_wait_all();
-      if (next_own) fix_mirrored(g, i, j, k + 3, ring + slot(k + 3) + own, VS);
-      if (next_halo) fix_mirrored(g, i0 + hx - XO, j0 + hy - 2, k + 1, ring + slot(k + 1) + hcell, VS);
-    }
-    __syncthreads();
-  }
-  split_stat_flush<C>(P, st);
-}
 
 // --------------------------------------------------------------------- shock detector (split)
 // USE_SHOCK_FLATTENING on the split state (source.F90:8073-8136): the full pressure of a
@@ -1117,6 +656,8 @@ __global__ void __launch_bounds__(256) k_sf_mark_split(Prm P) {
 template <class C>
 __device__ __forceinline__ void load_bccf(const Prm &P, int i, int j, int k, float b[3]) {
   const Geo &g = P.g;
+  b[0] = b[1] = b[2] = 0.0f;
+  if (!C::MHD) return;
   bool f0 = false, f1 = false, f2 = false;
   int si = map_index(i, g.nx[0], g.bc[0][0], g.bc[0][1], f0);
   int sj = map_index(j, g.nx[1], g.bc[1][0], g.bc[1][1], f1);
@@ -1132,12 +673,14 @@ __device__ __forceinline__ void load_bccf(const Prm &P, int i, int j, int k, flo
 
 template <class C>
 __device__ __forceinline__ void load_bccf_at(const Prm &P, long long c, float b[3]) {
+  b[0] = b[1] = b[2] = 0.0f;
+  if (!C::MHD) return;
   b[0] = __ldg(P.bccf + c);
   b[1] = __ldg(P.bccf + P.g.N + c);
   b[2] = C::DIM == 3 ? __ldg(P.bccf + 2 * P.g.N + c) : 0.0f;
 }
 
-// Riemann part of an MHD face along d (face index fidx, face background bg): the edge states
+// Riemann part of a face along d (face index fidx, face background bg): the edge states
 // in the cell frame (qL/qR in the order of the FP32 state, transverse B in bL/bR; FASTEOS gammas
 // gL/gR with the equilibrium gamma_e already added, or the face temperature guess tface of the
 // Helmholtz configurations without FASTEOS) are rotated to the normal frame, the WB background
@@ -1145,25 +688,31 @@ __device__ __forceinline__ void load_bccf_at(const Prm &P, long long c, float b[
 // frame with rho_L + rho_R for the CT upwinding sign (source.F90:8138-9105 with the MHD parts
 // 8327-8469, 8926-8959)
 template <class C>
-__device__ __forceinline__ void face_solve_split_mhd(const Prm &P, int d, long long fidx, const float4 &bg, float qL[C::NV],
+__device__ __forceinline__ void face_solve_split(const Prm &P, int d, long long fidx, const float4 &bg, float qL[C::NV],
                                                      float qR[C::NV], float bL[3], float bR[3], const float gLin[2],
                                                      const float gRin[2], float tface, bool flat, float F[C::NV],
                                                      float Fb[3], float &rho_sum) {
   constexpr int NV = C::NV, IP = C::IP;
   const Geo &g = P.g;
-  const float bn = (float)(P.bf[d][fidx] * P.inv_b_ref);
-  bL[d] = bn;
-  bR[d] = bn;
+  if (C::MHD) {
+    const float bn = (float)(P.bf[d][fidx] * P.inv_b_ref);
+    bL[d] = bn;
+    bR[d] = bn;
+  }
   if (d == 1) {
     float a = qL[1], c = qL[2]; qL[1] = c; qL[2] = -a;
     a = qR[1]; c = qR[2]; qR[1] = c; qR[2] = -a;
-    a = bL[0]; c = bL[1]; bL[0] = c; bL[1] = -a;
-    a = bR[0]; c = bR[1]; bR[0] = c; bR[1] = -a;
+    if (C::MHD) {
+      a = bL[0]; c = bL[1]; bL[0] = c; bL[1] = -a;
+      a = bR[0]; c = bR[1]; bR[0] = c; bR[1] = -a;
+    }
   } else if (C::DIM == 3 && d == 2) {
     float a = qL[1], c = qL[2], e = qL[3]; qL[1] = e; qL[2] = a; qL[3] = c;
     a = qR[1]; c = qR[2]; e = qR[3]; qR[1] = e; qR[2] = a; qR[3] = c;
-    a = bL[0]; c = bL[1]; e = bL[2]; bL[0] = e; bL[1] = a; bL[2] = c;
-    a = bR[0]; c = bR[1]; e = bR[2]; bR[0] = e; bR[1] = a; bR[2] = c;
+    if (C::MHD) {
+      a = bL[0]; c = bL[1]; e = bL[2]; bL[0] = e; bL[1] = a; bL[2] = c;
+      a = bR[0]; c = bR[1]; e = bR[2]; bR[0] = e; bR[1] = a; bR[2] = c;
+    }
   }
   const float pe = bg.y;
   if (C::WB) {
@@ -1175,23 +724,27 @@ __device__ __forceinline__ void face_solve_split_mhd(const Prm &P, int d, long l
     split_side_eos<C>(P, qL, pe, tface, gL[0], gL[1]);
     split_side_eos<C>(P, qR, pe, tface, gR[0], gR[1]);
   }
-  riemann_mhd_split<C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, bL, bR, gL, gR, pe, (float)g.gm, (float)g.mach_cutoff, F,
-                                                   Fb, flat, g.all_mach != 0);
+  if constexpr (C::MHD)
+    riemann_mhd_split<C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, bL, bR, gL, gR, pe, (float)g.gm, (float)g.mach_cutoff, F,
+                                                    Fb, flat, g.all_mach != 0);
+  else
+    riemann_hydro_split<C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, gL, gR, pe, (float)g.gm, (float)g.mach_cutoff, F, flat,
+                                                      g.all_mach != 0);
   if (d == 1) {
     float a = F[1], c = F[2]; F[1] = -c; F[2] = a;
-    a = Fb[0]; c = Fb[1]; Fb[0] = -c; Fb[1] = a;
+    if (C::MHD) { a = Fb[0]; c = Fb[1]; Fb[0] = -c; Fb[1] = a; }
   } else if (C::DIM == 3 && d == 2) {
     float a = F[1], c = F[2], e = F[3]; F[1] = c; F[2] = e; F[3] = a;
-    a = Fb[0]; c = Fb[1]; e = Fb[2]; Fb[0] = c; Fb[1] = e; Fb[2] = a;
+    if (C::MHD) { a = Fb[0]; c = Fb[1]; e = Fb[2]; Fb[0] = c; Fb[1] = e; Fb[2] = a; }
   }
   rho_sum = qL[0] + qR[0];
   if (C::ETOT) F[IP] = F[IP] + F[0] * bg.w;
 }
 
-// MHD flux through the low face of cell m along d from cells m-SW..m+SW-1 (w, gm, b: cells
-// m-3..m+2); reconstruction, then face_solve_split_mhd
+// flux through the low face of cell m along d from cells m-SW..m+SW-1 (w, gm, b: cells
+// m-3..m+2); reconstruction, then face_solve_split
 template <class C>
-__device__ __forceinline__ void face_flux_split_mhd(const Prm &P, int d, int fi, int fj, int fk, const float *const w[6],
+__device__ __forceinline__ void face_flux_split_rec(const Prm &P, int d, int fi, int fj, int fk, const float *const w[6],
                                                     const float *const gm[6], const float *const b[6], float F[C::NV],
                                                     float Fb[3], float &rho_sum) {
   constexpr int NV = C::NV;
@@ -1211,7 +764,7 @@ __device__ __forceinline__ void face_flux_split_mhd(const Prm &P, int d, int fi,
   float bL[3] = {0, 0, 0}, bR[3] = {0, 0, 0};
 #pragma unroll
   for (int iv = 0; iv < C::DIM; ++iv) {
-    if (iv == d) continue;
+    if (!C::MHD || iv == d) continue;
     const float v[6] = {b[0][iv], b[1][iv], b[2][iv], b[3][iv], b[4][iv], b[5][iv]};
     rec_face_f32<C>(v, C::REC == REC_LIM5TH, bL[iv], bR[iv]);
     if (C::SF && C::REC != REC_LIM2ND) flatten_face_f32(v, fa, fb, bL[iv], bR[iv]);
@@ -1237,7 +790,7 @@ __device__ __forceinline__ void face_flux_split_mhd(const Prm &P, int d, int fi,
   } else if (C::HELM) {
     tface = 0.5f * (gm[2][0] + gm[3][0]);
   }
-  face_solve_split_mhd<C>(P, d, face_lin(g, d, fi, fj, fk), bg, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F,
+  face_solve_split<C>(P, d, face_lin(g, d, fi, fj, fk), bg, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F,
                           Fb, rho_sum);
 }
 
@@ -1265,11 +818,11 @@ __device__ __forceinline__ void store_face_emf_split(const Prm &P, int d, long l
   P.fsgn[d][fidx] = sgn;
 }
 
-// MHD stage, part 1: one thread per face of direction d solves it once: the FP32 flux goes to
+// Stage, part 1: one thread per face of direction d solves it once: the FP32 flux goes to
 // P.fflux[d] ([NV][faces]), the face EMF and the CT sign to their arrays
 // (one instantiation per direction D: index strides and rotations fold into constants)
 template <class C, int D>
-__device__ __forceinline__ void face_split_mhd_at(const Prm &P, long long f) {
+__device__ __forceinline__ void face_split_at(const Prm &P, long long f) {
   constexpr int d = D;
   constexpr int NV = C::NV;
   const Geo &g = P.g;
@@ -1305,17 +858,17 @@ __device__ __forceinline__ void face_split_mhd_at(const Prm &P, long long f) {
   const float *const gv[6] = {gm4[0], gm4[1], gm4[2], gm4[3], gm4[4], gm4[5]};
   const float *const bv[6] = {b4[0], b4[1], b4[2], b4[3], b4[4], b4[5]};
   float F[NV], Fb[3], rs;
-  face_flux_split_mhd<C>(P, d, fi, fj, fk, wv, gv, bv, F, Fb, rs);
+  face_flux_split_rec<C>(P, d, fi, fj, fk, wv, gv, bv, F, Fb, rs);
   FluxPlanes<NV>::store(P.fflux[d], nf, f, F);
-  store_face_emf_split<C>(P, d, f, d == 0 ? fi : (d == 1 ? fj : fk), Fb, F[0], rs, (float)(P.scal[2] * P.inv_v_ref));
+  if (C::MHD) store_face_emf_split<C>(P, d, f, d == 0 ? fi : (d == 1 ? fj : fk), Fb, F[0], rs, (float)(P.scal[2] * P.inv_v_ref));
 }
 
 template <class C, int D>
-__global__ void __launch_bounds__(128, C::MINB_FACE32) k_face_split_mhd(Prm P) {
+__global__ void __launch_bounds__(128, C::MINB_FACE32) k_face_split(Prm P) {
   if (!*P.active) return;
   const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfaces(P.g, D)) return;
-  face_split_mhd_at<C, D>(P, f);
+  face_split_at<C, D>(P, f);
 }
 
 // faces per thread of the walking face kernels: along x (threads of a warp step K0 cells apart,
@@ -1330,14 +883,14 @@ constexpr int RESCUE_BLOCKS = 4 * 148;
 // nothing between faces and needs 72 registers.  Without USE_FASTEOS, where each face runs two FP64
 // (rho, P) -> T solves, 4 (128 registers): a 256^3 MHD step took 36.9 ms against 43.4 with the
 // registers unbounded (253 registers, 2 blocks per SM), 37.5 at 3
-constexpr int WALK_MINB = 5, WALK_MINB_GIVEN = 4, ROW_MINB = 6;
+constexpr int WALK_MINB = 5, WALK_MINB_HYDRO = 5, WALK_MINB_GIVEN = 4, ROW_MINB = 6;
 
 // Raw values of one cell for the walking face kernel along D: the FP32 state (0 .. NV-1), the
 // cell B components transverse to D (NBT of them from NV on; the component along D is not
 // reconstructed, the face carries it) and the two FASTEOS gammas or the temperature (IG, IG+1).
 template <class C, int D>
 struct WalkCell {
-  static constexpr int NBT = C::DIM - 1, IG = C::NV + NBT, NR = IG + 2;
+  static constexpr int NBT = C::MHD ? C::DIM - 1 : 0, IG = C::NV + NBT, NR = IG + 2;
   // cell B component held in transverse slot t
   static __device__ __forceinline__ constexpr int comp(int t) { return t < D ? t : t + 1; }
 };
@@ -1401,17 +954,17 @@ __device__ __forceinline__ void face_from_edges(const Prm &P, long long fidx, in
     }
   }
   float F[NV], Fb[3], rs;
-  face_solve_split_mhd<C>(P, D, fidx, bg, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F, Fb, rs);
+  face_solve_split<C>(P, D, fidx, bg, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F, Fb, rs);
   FluxPlanes<NV>::store(P.fflux[D], nfaces(g, D), fidx, F);
-  store_face_emf_split<C>(P, D, fidx, q, Fb, F[0], rs, smax_s);
+  if (C::MHD) store_face_emf_split<C>(P, D, fidx, q, Fb, F[0], rs, smax_s);
 }
 
-// MHD stage, part 1 for LIM2ND reconstruction: one thread walks K consecutive faces along D.  A
+// Stage, part 1 for LIM2ND reconstruction: one thread walks K consecutive faces along D.  A
 // cell borders two faces of the walk, so its values are loaded and its PLM slope formed once
 // (the per-face kernel does both twice) and its edge values are carried to the next face.  The
-// faces, their arithmetic and the stored results are those of k_face_split_mhd.
+// faces, their arithmetic and the stored results are those of k_face_split.
 template <class C, int D, int K>
-__global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : WALK_MINB) k_face_split_mhd_walk(Prm P) {
+__global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : (C::MHD ? WALK_MINB : WALK_MINB_HYDRO)) k_face_split_walk(Prm P) {
   static_assert(C::REC == REC_LIM2ND, "the walk carries LIM2ND edge values");
   if (!*P.active) return;
   using L = WalkCell<C, D>;
@@ -1480,7 +1033,7 @@ __global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : 
   }
 }
 
-// MHD stage, part 1 for LIM2ND along x1: a warp takes 32 neighbouring cells of a row and solves the
+// Stage, part 1 for LIM2ND along x1: a warp takes 32 neighbouring cells of a row and solves the
 // 29 faces whose stencils they hold.  A lane loads one cell (coalesced, all loads at once); the
 // differences and edge values of its neighbours come by shuffle, each slope is formed once, and
 // nothing is carried between faces, so the kernel needs no shared memory, no barrier and any row
@@ -1490,7 +1043,7 @@ __global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : 
 // instructions, two block barriers a tile) took 83 and a walk of 4 faces 1% more per stage.
 constexpr int ROW_FACES = 29;
 template <class C>
-__global__ void __launch_bounds__(128, ROW_MINB) k_face_split_mhd_row(Prm P, FastDiv chunks) {
+__global__ void __launch_bounds__(128, ROW_MINB) k_face_split_row(Prm P, FastDiv chunks) {
   static_assert(C::REC == REC_LIM2ND, "the row kernel forms LIM2ND edges");
   if (!*P.active) return;
   using L = WalkCell<C, 0>;
@@ -1736,12 +1289,13 @@ struct C2pState {
   long long bc = 0;
 };
 
-// MHD stage, part 3a: flux divergence from the face fluxes, gravity and the RK combine of U
+// Stage, part 3a: flux divergence from the face fluxes, gravity and the RK combine of U
 // (FP64), b_cc from the updated faces (FP64); stores U (U0 in the first stage), scaled b_cc and
 // what depends on the conserved state alone (FP32 velocities and scalars, cell EMFs), and
 // returns what the EoS part needs
+// (given: the flux divergence in scaled units, from the kernel that solved the faces itself)
 template <class C>
-__device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c, C2pState &cs) {
+__device__ __forceinline__ void c2p_split_combine(const Prm &P, long long c, C2pState &cs, const float *given = nullptr) {
   constexpr int NV = C::NV, IP = C::IP, IAS = C::IAS, DIM = C::DIM;
   const Geo &g = P.g;
   double &rho = cs.rho, &inv_rho = cs.inv_rho, &eint = cs.eint, &ye = cs.ye, &inv_abar = cs.inv_abar;
@@ -1764,15 +1318,19 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
     }
     cp_async_commit();
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
+    for (int d = 0; d < DIM && C::MHD; ++d) {
       int ui = i + (d == 0), uj = j + (d == 1), uk = k + (d == 2);
       bcc[d] = 0.5 * (P.bf[d][face_lin(g, d, ui, uj, uk)] + P.bf[d][face_lin(g, d, i, j, k)]);
       P.bccf[(long long)d * g.N + c] = (float)(bcc[d] * P.inv_b_ref);
     }
     // flux divergence (directions in the order of the hydro stage), gravity, RK combine
     float res[NV];
+    if (given) {
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
+      for (int iv = 0; iv < NV; ++iv) res[iv] = given[iv];
+    }
+#pragma unroll
+    for (int d = 0; d < DIM && !given; ++d) {
       const long long nf = nfaces(g, d);
       float lo[NV], hi[NV];
       FluxPlanes<NV>::load(P.fflux[d], nf, face_lin(g, d, i, j, k), lo);
@@ -1822,7 +1380,7 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
     inv_rho = 1.0 / rho;
     double ke = u[1] * u[1] + u[2] * u[2] + (DIM == 3 ? u[3] * u[3] : 0.0);
     eint = u[IP] - 0.5 * ke * inv_rho;
-    eint = eint - 0.5 * (bcc[0] * bcc[0] + bcc[1] * bcc[1] + bcc[2] * bcc[2]);
+    if (C::MHD) eint = eint - 0.5 * (bcc[0] * bcc[0] + bcc[1] * bcc[1] + bcc[2] * bcc[2]);
     if (C::ETOT) eint = eint - rho * __ldg(P.phi_cc + bc);
     float vf[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -1830,7 +1388,7 @@ __device__ __forceinline__ void c2p_mhd_split_combine(const Prm &P, long long c,
       vf[d] = (float)(u[1 + d] * inv_rho * P.inv_v_ref);
       P.Wf_out[(long long)(1 + d) * g.N + c] = vf[d];
     }
-    {
+    if (C::MHD) {
       const float bf3[3] = {(float)(bcc[0] * P.inv_b_ref), (float)(bcc[1] * P.inv_b_ref),
                             DIM == 3 ? (float)(bcc[2] * P.inv_b_ref) : 0.0f};
       store_cell_emf(P, c, vf, bf3);
@@ -1855,7 +1413,7 @@ enum { C2P_WARM = 0,    // the previous stage's temperature (the reference's war
 // ~4 more iterations, from the learned guess ~3 in all
 constexpr double RESCUE_STEP = 0.02;
 
-// MHD stage, part 3b: cons -> prim of the new state with the Helmholtz Newton (FP64) from the
+// Stage, part 3b: cons -> prim of the new state with the Helmholtz Newton (FP64) from the
 // warm guess (the previous stage's temperature), or (C2P_LEARNED) from the network's guess lT
 // (log10 T; NaN for none): the guess is accepted when the reference Newton converges from it
 // within 3 iterations without leaving the table, otherwise the Newton starts again from the
@@ -1864,7 +1422,7 @@ constexpr double RESCUE_STEP = 0.02;
 // eint, joins P.rescue_q and returns false with nothing else written (the rescue kernels finish
 // it from the learned guess); the other cells run the warm-start Newton unchanged.
 template <class C, int MODE>
-__device__ __forceinline__ bool c2p_mhd_split_eos(const Prm &P, long long c, const C2pState &cs, float lT_mlp,
+__device__ __forceinline__ bool c2p_split_eos(const Prm &P, long long c, const C2pState &cs, float lT_mlp,
                                                   SplitStat &st) {
   constexpr bool LEARNED = MODE == C2P_LEARNED;
   constexpr int IP = C::IP, DIM = C::DIM;
@@ -1954,9 +1512,11 @@ __device__ __forceinline__ bool c2p_mhd_split_eos(const Prm &P, long long c, con
       double vabs[3] = {0.0, 0.0, 0.0}, ca2 = 0.0;
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
-        const double b = 0.5 * (P.bf[d][face_lin(g, d, i + (d == 0), j + (d == 1), k + (d == 2))] +
-                                P.bf[d][face_lin(g, d, i, j, k)]);
-        ca2 = d == 0 ? b * b : ca2 + b * b;
+        if (C::MHD) {
+          const double b = 0.5 * (P.bf[d][face_lin(g, d, i + (d == 0), j + (d == 1), k + (d == 2))] +
+                                  P.bf[d][face_lin(g, d, i, j, k)]);
+          ca2 = d == 0 ? b * b : ca2 + b * b;
+        }
         vabs[d] = fabs(P.U[(long long)(1 + d) * g.N + c] * inv_rho);
       }
       double csnd = sqrt(sound2 + ca2 * inv_rho);
@@ -1971,7 +1531,7 @@ __device__ __forceinline__ bool c2p_mhd_split_eos(const Prm &P, long long c, con
 }
 
 template <class C, int MODE>
-__global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_mhd_split(Prm P) {
+__global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_split(Prm P) {
   if (!*P.active) return;
   SplitStat st;
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1979,8 +1539,59 @@ __global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_mhd_split(Prm 
     C2pState cs;
     // the warm start first: its load then overlaps the combine instead of following its stores
     if (C::HELM) cs.Tw = P.temp[c];
-    c2p_mhd_split_combine<C>(P, c, cs);
-    c2p_mhd_split_eos<C, MODE>(P, c, cs, 0.0f, st);
+    c2p_split_combine<C>(P, c, cs);
+    c2p_split_eos<C, MODE>(P, c, cs, 0.0f, st);
+  }
+  split_stat_flush<C>(P, st);
+}
+
+// A whole hydro stage in one kernel, one thread per cell: every face is solved by both of its cells,
+// nothing goes through memory but the state.  On small grids, whose kernels are all latency, one
+// launch beats the face kernels and cons->prim (SplitRunnerT::one_kernel has the line).
+template <class C>
+__global__ void __launch_bounds__(C2P_BLOCK) k_stage_split(Prm P) {
+  if (!*P.active) return;
+  constexpr int NV = C::NV, DIM = C::DIM, SW = C::SW, NS = 2 * SW + 1;
+  const Geo &g = P.g;
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  SplitStat st;
+  if (c < g.N) {
+    C2pState cs;
+    if (C::HELM) cs.Tw = P.temp[c];
+    int i, j, k;
+    unflatten3(c, g.div0[0], g.div1[0], i, j, k);
+    float res[NV];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      // cells c-SW .. c+SW along d: the low face reads the first 2 SW, the high face the last
+      float w[NS][NV], gmv[NS][2];
+#pragma unroll
+      for (int s = 0; s < NS; ++s)
+        load_wf<C>(P, i + (d == 0 ? s - SW : 0), j + (d == 1 ? s - SW : 0), k + (d == 2 ? s - SW : 0), w[s], gmv[s]);
+      const float none[3] = {0.0f, 0.0f, 0.0f};
+      const float *const nb[6] = {none, none, none, none, none, none};
+      float F[2][NV], Fb[3], rs;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        // cells m-3 .. m+2 of the face; the outer pair is read by LIM5TH only
+        const float *wp[6], *gp[6];
+#pragma unroll
+        for (int s = 0; s < 6; ++s) {
+          const int q = s + e + SW - 3;
+          wp[s] = w[q < 0 ? 0 : (q < NS ? q : NS - 1)];
+          gp[s] = gmv[q < 0 ? 0 : (q < NS ? q : NS - 1)];
+        }
+        face_flux_split_rec<C>(P, d, i + (e && d == 0), j + (e && d == 1), k + (e && d == 2), wp, gp, nb, F[e], Fb, rs);
+      }
+      const float inv_dl = (float)g.inv_dx[d];
+#pragma unroll
+      for (int iv = 0; iv < NV; ++iv) {
+        const float dd = (F[1][iv] - F[0][iv]) * inv_dl;
+        res[iv] = d == 0 ? dd : res[iv] + dd;
+      }
+    }
+    c2p_split_combine<C>(P, c, cs, res);
+    c2p_split_eos<C, C2P_WARM>(P, c, cs, 0.0f, st);
   }
   split_stat_flush<C>(P, st);
 }
@@ -2022,18 +1633,18 @@ __device__ __forceinline__ float4 c2p_features(const Prm &P, const C2pState &cs)
 // barriers): (1) the combine, storing eint and the network's features, (2) k_mlp_guess over
 // all cells, (3) the EoS part from the stored state and guess.
 template <class C>
-__global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_mhd_split_features(Prm P) {
+__global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_split_features(Prm P) {
   if (!*P.active) return;
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= P.g.N) return;
   C2pState cs;
-  c2p_mhd_split_combine<C>(P, c, cs);
+  c2p_split_combine<C>(P, c, cs);
   P.eint[c] = cs.eint;
   reinterpret_cast<float4 *>(P.mlp_feat)[c] = c2p_features<C>(P, cs);
 }
 
 template <class C>
-__global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_mhd_split_guessed(Prm P) {
+__global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_split_guessed(Prm P) {
   if (!*P.active) return;
   SplitStat st;
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2042,7 +1653,7 @@ __global__ void __launch_bounds__(128, C::MINB_C2P32) k_c2p_mhd_split_guessed(Pr
     C2pState cs;
     c2p_state_from_u<C>(P, c, cs);
     st.gevals += 1;
-    c2p_mhd_split_eos<C, C2P_LEARNED>(P, c, cs, P.mlp_out[c], st);
+    c2p_split_eos<C, C2P_LEARNED>(P, c, cs, P.mlp_out[c], st);
   }
   split_stat_flush<C>(P, st);
 }
@@ -2069,7 +1680,7 @@ static __global__ void __launch_bounds__(128) k_mlp_guess(const __grid_constant_
 }
 
 // ---- learned rescue of poor warm starts (eos_guess = PHL_GUESS_MLP_RESCUE): one kernel on a
-// fixed grid over the queue that k_c2p_mhd_split<C, C2P_RESCUE> fills.  Tiles of 128 queue
+// fixed grid over the queue that k_c2p_split<C, C2P_RESCUE> fills.  Tiles of 128 queue
 // slots, strided over the blocks: each thread reads its cell's state back (U, eint) and forms
 // the network's features, the block runs one tensor-core product for the tile, and each thread
 // finishes its cell from the judged guess.  With an empty queue every block reads the count and
@@ -2101,7 +1712,7 @@ __global__ void __launch_bounds__(128) k_c2p_rescue(Prm P, const __grid_constant
     parity ^= 1u;
     if (c >= 0) {
       st.gevals += 1;
-      c2p_mhd_split_eos<C, C2P_LEARNED>(P, c, cs, have ? y : __int_as_float(0x7fc00000), st);
+      c2p_split_eos<C, C2P_LEARNED>(P, c, cs, have ? y : __int_as_float(0x7fc00000), st);
     }
   }
   mlp_cta_teardown(S);
@@ -2218,91 +1829,36 @@ __global__ void k_split_to_prim(Prm P) {
 namespace {
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// cuTensorMapEncodeTiled from the driver, found through the runtime (no link to libcuda)
-PFN_cuTensorMapEncodeTiled tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
-  }
-  return fn;
-}
-
-// 4D map (x1, x2, x3, variable) over an FP32 SoA field block, box = (bx, by, bz, nvar)
-bool encode_box_map(CUtensorMap *m, const float *base, int nvar, const Geo &g, int bx, int by, int bz) {
-  PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
-  if (!enc || !base) return false;
-  const cuuint64_t nx = (cuuint64_t)g.nx[0], ny = (cuuint64_t)g.nx[1], nz = (cuuint64_t)g.nx[2];
-  const cuuint64_t dims[4] = {nx, ny, nz, (cuuint64_t)nvar};
-  const cuuint64_t strides[3] = {nx * 4, nx * ny * 4, (cuuint64_t)g.N * 4};
-  const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)nvar};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-bool encode_plane_map(CUtensorMap *m, const float *base, int nvar, const Geo &g, int bx, int by) {
-  return encode_box_map(m, base, nvar, g, bx, by, 1);
-}
 }
 
 template <class C>
 struct SplitRunnerT : Runner {
-  static constexpr int TX = 32, TY = 8, KZ = 16;
-  bool attr_set = false;
-  // tensor maps of the two FP32 state buffers (the stage input alternates between them)
-  struct MapEntry {
-    const float *w = nullptr;
-    SplitMaps maps;
-    bool ok = false;
-  } map_cache[2];
-  // maps of this stage's input, or false when interior tiles must also copy cell by cell
-  bool stage_maps(const Prm &P, SplitMaps &out) {
-    using T = SplitTile<C, TX, TY>;
-    const Geo &g = P.g;
-    // bulk copies need a periodic x3 (the plane index wraps) and interior tiles in x1 and x2
-    if (g.bc[2][0] != BC_PERIODIC || g.nx[0] < 3 * TX || g.nx[1] < 3 * TY) return false;
-    for (auto &e : map_cache)
-      if (e.w == P.Wf_in) {
-        out = e.maps;
-        return e.ok;
-      }
-    MapEntry &e = map_cache[map_cache[0].w ? 1 : 0];
-    e.w = P.Wf_in;
-    e.ok = encode_plane_map(&e.maps.w, P.Wf_in, C::NV, g, T::SX, T::SY);
-    if (e.ok && C::HELM) e.ok = encode_plane_map(&e.maps.g, P.gf_in, 2, g, T::SX, T::SY);
-    out = e.maps;
-    return e.ok;
-  }
   // PHL_FACE_KERNEL=walk runs the walking kernel along x1 as well (comparison)
   const bool walk_x1 = [] {
     const char *e = getenv("PHL_FACE_KERNEL");
     return e && strcmp(e, "walk") == 0;
   }();
-  // PHL_STAGE_KERNEL=cell selects the per-cell kernel on any grid, =tiled_cpasync the tiled
-  // kernel with cell-by-cell copies only (comparisons of the three)
-  const bool allow_tiled = [] {
+  // A hydro stage in one per-cell kernel on grids of up to about one and a half (3D) or three (2D)
+  // waves of its blocks; with more cells the face kernels, which solve each face once, pay for their
+  // launches.  us per stage, one kernel / face kernels: Helmholtz box 20^3 21 / 32, 32^3 22 / 33, 48^3
+  // 34 / 40, 150x101x70 201 / 162; hot bubble 64^2 9 / 15, 400^2 16 / 19, 700^2 32 / 31, 1024^2 68 / 61.
+  // PHL_STAGE_KERNEL=cell / =faces select one of them on any grid (comparisons).
+  const int stage_kind = [] {
     const char *e = getenv("PHL_STAGE_KERNEL");
-    return !(e && strcmp(e, "cell") == 0);
+    return e && strcmp(e, "cell") == 0 ? 1 : (e && strcmp(e, "faces") == 0 ? 2 : 0);
   }();
-  const bool allow_tma = [] {
-    const char *e = getenv("PHL_STAGE_KERNEL");
-    return !(e && strcmp(e, "tiled_cpasync") == 0);
-  }();
-  bool tiled(const Geo &g) const {
-    return allow_tiled && C::DIM == 3 && g.nx[0] % TX == 0 && g.nx[1] % TY == 0 && g.nx[2] % KZ == 0;
+  bool one_kernel(const Geo &g) const {
+    if (stage_kind) return stage_kind == 1;
+    return g.N < (C::DIM == 3 ? 220000 : 430000);
   }
   void stage(const Prm &P, cudaStream_t s) override {
     if constexpr (C::SF) {
       k_sf_mark_split<C><<<nblk(sf_mark_cells<C>(P.g), 256), 256, 0, s>>>(P);
       k_sf_flag<C><<<nblk(sf_flag_cells<C>(P.g), 256), 256, 0, s>>>(P);
     }
-    if constexpr (C::MHD) {
+    if (!C::MHD && one_kernel(P.g)) {
+      if constexpr (!C::MHD) k_stage_split<C><<<nblk(P.g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
+    } else {
       const Geo &g = P.g;
       auto nfc = [&](int d) {
         return (long long)(g.nx[0] + (d == 0)) * (g.nx[1] + (d == 1)) * (g.nx[2] + (d == 2));
@@ -2318,41 +1874,41 @@ struct SplitRunnerT : Runner {
         // without USE_FASTEOS a face is two FP64 (rho, P) -> T solves, and the row kernel's three idle
         // lanes in 32 cost more than its loads save (96^3 MHD step 2.50 ms against 2.28)
         if (walk_x1 || C::EOSM == EOS_GIVEN) {
-          k_face_split_mhd_walk<C, 0, WALK_K0><<<nblk(nwalk(0, WALK_K0), 128), 128, 0, s>>>(P);
+          k_face_split_walk<C, 0, WALK_K0><<<nblk(nwalk(0, WALK_K0), 128), 128, 0, s>>>(P);
         } else if constexpr (C::EOSM != EOS_GIVEN) {
           const unsigned chunks = nblk(g.nx[0] + 1, ROW_FACES);
-          k_face_split_mhd_row<C><<<nblk((long long)chunks * g.nx[1] * g.nx[2], 4), 128, 0, s>>>(P, FastDiv::by(chunks));
+          k_face_split_row<C><<<nblk((long long)chunks * g.nx[1] * g.nx[2], 4), 128, 0, s>>>(P, FastDiv::by(chunks));
         }
-        k_face_split_mhd_walk<C, 1, WALK_K><<<nblk(nwalk(1, WALK_K), 128), 128, 0, s>>>(P);
+        k_face_split_walk<C, 1, WALK_K><<<nblk(nwalk(1, WALK_K), 128), 128, 0, s>>>(P);
         if constexpr (C::DIM == 3)
-          k_face_split_mhd_walk<C, 2, WALK_K><<<nblk(nwalk(2, WALK_K), 128), 128, 0, s>>>(P);
+          k_face_split_walk<C, 2, WALK_K><<<nblk(nwalk(2, WALK_K), 128), 128, 0, s>>>(P);
       } else {
-        k_face_split_mhd<C, 0><<<nblk(nfc(0), 128), 128, 0, s>>>(P);
-        k_face_split_mhd<C, 1><<<nblk(nfc(1), 128), 128, 0, s>>>(P);
-        if constexpr (C::DIM == 3) k_face_split_mhd<C, 2><<<nblk(nfc(2), 128), 128, 0, s>>>(P);
+        k_face_split<C, 0><<<nblk(nfc(0), 128), 128, 0, s>>>(P);
+        k_face_split<C, 1><<<nblk(nfc(1), 128), 128, 0, s>>>(P);
+        if constexpr (C::DIM == 3) k_face_split<C, 2><<<nblk(nfc(2), 128), 128, 0, s>>>(P);
       }
-      corners(P, s);
-      const long long nodes = (long long)(g.nx[0] + 1) * (g.nx[1] + 1) * (C::DIM == 3 ? g.nx[2] + 1 : 1);
-      k_bface_split<C><<<nblk(nodes, 256), 256, 0, s>>>(P);
-      if constexpr (C::HELM) {
+      if constexpr (C::MHD) {
+        corners(P, s);
+        const long long nodes = (long long)(g.nx[0] + 1) * (g.nx[1] + 1) * (C::DIM == 3 ? g.nx[2] + 1 : 1);
+        k_bface_split<C><<<nblk(nodes, 256), 256, 0, s>>>(P);
+      }
+      if constexpr (C::HELM && C::MHD) {
         if (P.mlp_w && P.mlp_small && P.rescue_q) {
           // warm start everywhere; cells with a poor warm start through the learned guess
           cudaMemsetAsync(P.rescue_q, 0, sizeof(unsigned), s);
-          k_c2p_mhd_split<C, C2P_RESCUE><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
+          k_c2p_split<C, C2P_RESCUE><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
           k_c2p_rescue<C><<<RESCUE_BLOCKS, 128, sizeof(MlpUmmaSmem), s>>>(P, *P.mlp_small);
           return;
         }
         if (P.mlp_w && P.mlp_small && P.mlp_feat && P.mlp_out) {
-          k_c2p_mhd_split_features<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
+          k_c2p_split_features<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
           k_mlp_guess<<<nblk(g.N, 128), 128, sizeof(MlpUmmaSmem), s>>>(*P.mlp_small, P.mlp_w2bf, g.N, P.mlp_feat,
                                                                        P.mlp_out, P.active, P.stat + STAT_TC_STALLED);
-          k_c2p_mhd_split_guessed<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
+          k_c2p_split_guessed<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
           return;
         }
       }
-      k_c2p_mhd_split<C, C2P_WARM><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
-    } else {
-      hydro_stage(P, s);
+      k_c2p_split<C, C2P_WARM><<<nblk(g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
     }
   }
   // corner EMFs: the interior nodes' blocks, then those of the nodes on the domain's faces
@@ -2364,25 +1920,6 @@ struct SplitRunnerT : Runner {
     const unsigned bin = nblk(nin, 256);
     k_corner_split<C><<<bin + nblk(nrim, 256), 256, 0, s>>>(P, bin, FastDiv::by((unsigned)n0 - 1),
                                                             FastDiv::by((unsigned)n1 - 1));
-  }
-  void hydro_stage(const Prm &P, cudaStream_t s) {
-    if constexpr (C::DIM == 3 && C::SW == 2) {
-      if (tiled(P.g)) {
-        constexpr size_t sm = SplitTile<C, TX, TY>::bytes();
-        if (!attr_set) {
-          cudaFuncSetAttribute(k_stage_split_tiled<C, TX, TY, KZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sm);
-          attr_set = true;
-        }
-        dim3 grid(P.g.nx[0] / TX, P.g.nx[1] / TY, P.g.nx[2] / KZ);
-        SplitMaps maps;
-        memset(&maps, 0, sizeof(maps));
-        const int use_tma = allow_tma && stage_maps(P, maps) ? 1 : 0;
-        k_stage_split_tiled<C, TX, TY, KZ><<<grid, TX * TY, sm, s>>>(P, maps, use_tma);
-        return;
-      }
-    }
-    k_stage_split<C><<<nblk(P.g.N, 128), 128, 0, s>>>(P);
   }
   void split_from_prim(const Prm &P, cudaStream_t s) override {
     k_split_from_prim<C><<<nblk(P.g.N, 256), 256, 0, s>>>(P);

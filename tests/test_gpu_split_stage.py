@@ -1,0 +1,82 @@
+"""The split form's stage kernels against one another where their work splits: the warp rows along
+x1 (29 faces each), the walks of 8 faces along x2 and x3, and the one-kernel hydro stage of small
+grids, which solves every face from both of its cells with the ghost mapping of single loads.
+
+Two kernels that do the same FP32 arithmetic sit at the same rounding distance from the FP64 form and
+apart by rounding noise only, so each must be no further from FP64 than 1.5 times the other, and the
+two no further apart than the sum of their distances.  A wrong stencil, ghost or face index moves a
+field by its own size."""
+import numpy as np
+import pytest
+
+from phlegethon_b200 import problems
+from test_gpu_split import run_form
+from util import div_b_max, field_errors, permute_axes
+
+pytestmark = pytest.mark.gpu
+
+
+def check(ha, hb, h64):
+    ea, eb, diff = field_errors(ha, h64), field_errors(hb, h64), field_errors(ha, hb)
+    for f in ea:
+        assert ea[f] <= 1.5 * eb[f] + 1e-12 and eb[f] <= 1.5 * ea[f] + 1e-12, (f, ea, eb)
+        assert diff[f] <= ea[f] + eb[f] + 1e-12, (f, diff, ea, eb)
+
+
+def both(cfg, h, table, monkeypatch, var, a, b, steps=3):
+    monkeypatch.setenv(var, a)
+    ha, sta = run_form(cfg, h, steps, table, "fp32_split")
+    monkeypatch.setenv(var, b)
+    hb, stb = run_form(cfg, h, steps, table, "fp32_split")
+    h64, _ = run_form(cfg, h, steps, table, "fp64")
+    for st in (sta, stb):
+        assert st["nonfinite"] == 0 and st["newton_calls"] in (0, steps * 3 * cfg.n_cells)
+    check(ha, hb, h64)
+    return ha, hb
+
+
+# row lengths around multiples of 29 faces (nx1 + 1 of them) and walks around multiples of 8
+@pytest.mark.parametrize("n,ny,nz", [(4, 4, 5), (27, 7, 8), (28, 8, 7), (29, 9, 16), (57, 15, 5), (58, 16, 4)])
+def test_hydro_face_kernels_equal_one_kernel(gpu_lib, table, monkeypatch, n, ny, nz):
+    cfg, h = problems.stratified_3d(n, ny=ny, nz=nz, seed=n)
+    both(cfg, h, table, monkeypatch, "PHL_STAGE_KERNEL", "faces", "cell")
+
+
+@pytest.mark.parametrize("perm", [(1, 0, 2), (0, 2, 1)])
+def test_hydro_walls_along_x1_and_x3(gpu_lib, table, monkeypatch, perm):
+    cfg, h = problems.stratified_3d(10, ny=30, nz=9)
+    h = permute_axes(h, perm)
+    both(h.cfg, h, table, monkeypatch, "PHL_STAGE_KERNEL", "faces", "cell")
+
+
+@pytest.mark.parametrize("n", [28, 31, 58])
+def test_hydro_2d(gpu_lib, monkeypatch, n):
+    cfg, h = problems.hot_bubble_2d(n)
+    both(cfg, h, None, monkeypatch, "PHL_STAGE_KERNEL", "faces", "cell", steps=6)
+
+
+@pytest.mark.parametrize("rec", ["pph", "lim5th"])
+def test_hydro_other_reconstructions(gpu_lib, table, monkeypatch, rec):
+    cfg, h = problems.stratified_3d(30, ny=9, nz=10, rec=rec)
+    both(cfg, h, table, monkeypatch, "PHL_STAGE_KERNEL", "faces", "cell")
+
+
+@pytest.mark.parametrize("case", ["28", "29", "58", "walls_x1", "walls_x3", "2d"])
+def test_mhd_rows_equal_walks(gpu_lib, table, monkeypatch, case):
+    if case == "2d":
+        cfg, h = problems.orszag_tang_2d(59)
+        tab = None
+    else:
+        cfg, h = problems.stratified_3d(int(case) if case.isdigit() else 12, ny=17, nz=7, mhd=True)
+        # a field with all three components: a loop in the (x1, x3) plane adds to the uniform b1
+        B = h.b_x[0][0, 0, 0]
+        i, k = np.arange(-1, cfg.nx1 + 2), np.arange(-1, cfg.nx3 + 2)
+        dx = cfg.dx()
+        A = 0.1 * B * cfg.x1u * np.cos(2 * np.pi * i / cfg.nx1)[:, None] * np.cos(2 * np.pi * k / cfg.nx3)[None, :]
+        h.b_x[0][...] += ((A[:, 1:] - A[:, :-1]) / dx[2])[:, None, :]
+        h.b_x[2][...] += (-(A[1:, :] - A[:-1, :]) / dx[0])[:, None, :]
+        tab = table
+    if case.startswith("walls"):
+        h = permute_axes(h, (1, 0, 2) if case == "walls_x1" else (0, 2, 1))
+    ha, hb = both(h.cfg, h, tab, monkeypatch, "PHL_FACE_KERNEL", "row", "walk")
+    assert div_b_max(ha) <= 1e-13 and div_b_max(hb) <= 1e-13
