@@ -523,33 +523,93 @@ struct HelmTable {
   double Tl, Th;
 };
 
-struct HelmPos {
-  int ih, jh;  // 1-based like the reference
-  double Ye, rhos, x, y, omx, omy, drho, dT, drho2, dT2, idrho, idT, idT2;
-};
+// ---- The FP64 evaluations below follow the reference operation by operation, so their results are
+// its results to the last bit; what they leave out are operations whose result is already known.  Of
+// a Newton iteration's twelve divisions and two double-precision logarithms one division remains:
+// the density part (cell, bases, reciprocals) is formed once per solve, a table cell is found
+// without a logarithm away from the nodes, and a quotient by a value with a known reciprocal takes
+// five multiply-adds (div_by).  The FP64 pipe was busy 61% of the time in cons->prim (3,000 FP64
+// instructions a cell), which ran 241 us on 96^3 cells.
 
-__device__ __forceinline__ void helm_locate(const HelmTable &h, double rho, double T, double abar,
-                                            double zbar, HelmPos &p) {
-  p.Ye = zbar / abar;
-  p.rhos = rho * p.Ye;
-  p.ih = (int)((log10(p.rhos) - h.log10_rho1) / h.drho) + 1;
-  p.jh = (int)((log10(T) - h.log10_T1) / h.dT) + 1;
-  // stay inside the table like the reference's arrays would (the reference does not check)
-  p.ih = max(1, min(p.ih, h.nrho - 1));
-  p.jh = max(1, min(p.jh, h.nT - 1));
-  double tmp = __ldg(h.rho + p.ih - 1);
-  p.drho = __ldg(h.rho + p.ih) - tmp;
-  p.x = (p.rhos - tmp) / p.drho;
-  p.omx = 1.0 - p.x;
-  tmp = __ldg(h.T + p.jh - 1);
-  p.dT = __ldg(h.T + p.jh) - tmp;
-  p.y = (T - tmp) / p.dT;
-  p.omy = 1.0 - p.y;
-  p.drho2 = p.drho * p.drho;
-  p.dT2 = p.dT * p.dT;
-  p.idrho = 1.0 / p.drho;
-  p.idT = 1.0 / p.dT;
-  p.idT2 = p.idT * p.idT;
+// a / b correctly rounded from rb = RN(1 / b): two Newton steps on the quotient with exact residuals
+// (Markstein, IBM J. Res. Dev. 34, 1990: with RN(1/b) and a faithful quotient the last step rounds
+// correctly, and the first step makes the quotient faithful).  For finite a, b well inside the
+// exponent range (HELM_LO .. HELM_HI below); callers divide plainly otherwise.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+  double q = __dmul_rn(a, rb);
+  q = __fma_rn(__fma_rn(-b, q, a), rb, q);
+  return __fma_rn(__fma_rn(-b, q, a), rb, q);
+}
+constexpr double HELM_LO = 1.0e-30, HELM_HI = 1.0e60;
+__device__ __forceinline__ bool helm_in_range(double x) { return x > HELM_LO && x < HELM_HI; }
+
+// table node index (1-based like the reference) of x in the log-spaced nodes: an estimate in
+// single precision (within one node of the cell for any x in the table's range), then exact
+// comparisons against the node values
+__device__ __forceinline__ int helm_node_index(const double *nodes, int n, double log10_first, double dlog,
+                                               double x) {
+  const float lx = __log2f((float)x) * 0.30102999566398120f;
+  int i = (int)(__fdividef(lx - (float)log10_first, (float)dlog)) + 1;
+  i = max(1, min(i, n - 1));
+  if (i < n - 1 && __ldg(nodes + i) <= x) ++i;
+  if (i > 1 && __ldg(nodes + i - 1) > x) --i;
+  return i;
+}
+// the reference's index (source.F90:23702-23709); the reference does not check the table's ends
+static __device__ __noinline__ int helm_log_index(int n, double log10_first, double dlog, double x) {
+  const int i = (int)((log10(x) - log10_first) / dlog) + 1;
+  return max(1, min(i, n - 1));
+}
+// The same index without the logarithm: x more than HELM_EDGE (relative) inside the cell of its node
+// index has the reference's index there (the logarithm, the nodes and the quotient are off by less
+// than 1e-13 of a cell together); next to a node, outside the table or for NaN the logarithm decides.
+constexpr double HELM_EDGE = 1.0e-12;
+__device__ __forceinline__ int helm_index(const double *nodes, int n, double log10_first, double dlog, double x) {
+  const int i = helm_node_index(nodes, n, log10_first, dlog, x);
+  if (x >= __ldg(nodes + i - 1) * (1.0 + HELM_EDGE) && x <= __ldg(nodes + i) * (1.0 - HELM_EDGE)) return i;
+  return helm_log_index(n, log10_first, dlog, x);
+}
+
+// density part of an evaluation: table row, position in it, and the reciprocals the others divide by
+struct HelmRho {
+  int ih;
+  bool ok;  // rho within the range of div_by
+  double rho, irho, iabar, Ye, rhos, x, omx, drho, drho2;
+};
+__device__ __forceinline__ HelmRho helm_rho_part(const HelmTable &h, double rho, double abar, double zbar) {
+  HelmRho r;
+  r.rho = rho;
+  r.irho = 1.0 / rho;
+  r.ok = helm_in_range(rho);
+  r.iabar = 1.0 / abar;
+  r.Ye = zbar / abar;
+  r.rhos = rho * r.Ye;
+  r.ih = helm_index(h.rho, h.nrho, h.log10_rho1, h.drho, r.rhos);
+  const double tmp = __ldg(h.rho + r.ih - 1);
+  r.drho = __ldg(h.rho + r.ih) - tmp;
+  r.x = (r.rhos - tmp) / r.drho;
+  r.omx = 1.0 - r.x;
+  r.drho2 = r.drho * r.drho;
+  return r;
+}
+// temperature part: the cell, kept while T stays inside it (lo <= T <= hi: HELM_EDGE off its nodes)
+struct HelmTemp {
+  int jh = 0;
+  double T0, dT, idT, lo = 1.0, hi = 0.0, y, omy;
+};
+__device__ __forceinline__ void helm_temp_part(const HelmTable &h, double T, HelmTemp &t) {
+  if (!(T >= t.lo && T <= t.hi)) {
+    t.jh = helm_index(h.T, h.nT, h.log10_T1, h.dT, T);
+    const double up = __ldg(h.T + t.jh);
+    t.T0 = __ldg(h.T + t.jh - 1);
+    t.dT = up - t.T0;
+    t.idT = __ldg(h.inv_dT + t.jh - 1);
+    t.lo = t.T0 * (1.0 + HELM_EDGE);
+    t.hi = up * (1.0 - HELM_EDGE);
+  }
+  const double a = T - t.T0;
+  t.y = helm_in_range(T) ? div_by(a, t.dT, t.idT) : a / t.dT;
+  t.omy = 1.0 - t.y;
 }
 
 // quintic Hermite bases (source.F90:24708-24738) and their derivatives
@@ -626,111 +686,145 @@ __device__ __forceinline__ void helm_load36(const HelmTable &h, int ih, int jh, 
   }
 }
 
-// helm_rhoT_given2 (source.F90:24571-24941): E and dE/dT
-__device__ __forceinline__ void helm_given2(const HelmTable &h, double rho, double T, double abar,
-                                            double zbar, double &E, double &dEdT, bool want_deriv) {
-  HelmPos p;
-  helm_locate(h, rho, T, abar, zbar, p);
+// helm_rhoT_given2 (source.F90:24571-24941): E and dE/dT; r0, r1 the density bases of the row
+__device__ __forceinline__ void helm_rho_bases(const HelmRho &r, double r0[3], double r1[3]) {
+  hb0(r.x, r.drho, r.drho2, r0);
+  hb0m(r.omx, r.drho, r.drho2, r1);
+}
+template <bool DERIV>
+__device__ __forceinline__ void helm_energy(const HelmTable &h, const HelmRho &r, const double r0[3],
+                                            const double r1[3], HelmTemp &t, double T, double &E, double &dEdT) {
+  helm_temp_part(h, T, t);
   double c[36];
-  helm_load36(h, p.ih, p.jh, c);
-  double r0[3], r1[3], t0[3], t1[3];
-  hb0(p.x, p.drho, p.drho2, r0);
-  hb0m(p.omx, p.drho, p.drho2, r1);
-  hb0(p.y, p.dT, p.dT2, t0);
-  hb0m(p.omy, p.dT, p.dT2, t1);
+  helm_load36(h, r.ih, t.jh, c);
+  const double dT2 = t.dT * t.dT;
+  double t0[3], t1[3];
+  hb0(t.y, t.dT, dT2, t0);
+  hb0m(t.omy, t.dT, dT2, t1);
   double f = helm_sum36(c, r0, r1, t0, t1);
   double d0[3], d1[3];
-  hb1(p.y, p.idT, p.dT, d0);
-  hb1m(p.omy, p.idT, p.dT, d1);
+  hb1(t.y, t.idT, t.dT, d0);
+  hb1m(t.omy, t.idT, t.dT, d1);
   double df_dT = helm_sum36(c, r0, r1, d0, d1);
   double df_dT2 = 0.0;
-  if (want_deriv) {
+  if (DERIV) {
+    const double idT2 = t.idT * t.idT;
     double e0[3], e1[3];
-    hb2(p.y, p.idT2, p.idT, e0);
-    hb2m(p.omy, p.idT2, p.idT, e1);
+    hb2(t.y, idT2, t.idT, e0);
+    hb2m(t.omy, idT2, t.idT, e1);
     df_dT2 = helm_sum36(c, r0, r1, e0, e1);
   }
-  double s = -p.Ye * df_dT;
-  double ds_dT = -p.Ye * df_dT2;
-  double e = p.Ye * f + T * s;
-  double de = T * ds_dT;
+  const bool safe = r.ok && helm_in_range(T);
+  double s = -r.Ye * df_dT;
+  double e = r.Ye * f + T * s;
   double T2 = T * T, T3 = T2 * T, T4 = T3 * T;
-  double tmp = 1.0 / abar;
-  e = e + 1.5 * CONST_RGAS * T * tmp + CONST_RAD * T4 / rho;
-  de = de + 1.5 * CONST_RGAS * tmp + 4.0 * CONST_RAD * T3 / rho;
+  const double aT4 = CONST_RAD * T4;
+  e = e + 1.5 * CONST_RGAS * T * r.iabar + (safe ? div_by(aT4, r.rho, r.irho) : aT4 / r.rho);
   E = e;
-  dEdT = de;
+  if (DERIV) {
+    double ds_dT = -r.Ye * df_dT2;
+    double de = T * ds_dT;
+    const double aT3 = 4.0 * CONST_RAD * T3;
+    dEdT = de + 1.5 * CONST_RGAS * r.iabar + (safe ? div_by(aT3, r.rho, r.irho) : aT3 / r.rho);
+  }
+}
+// E at table temperature node j (1-based).  There the position in the cell is exactly 0 (or 1 in the
+// cell below), the T bases are exactly 1 and 0, and of the 36 terms of f and df/dT only the node's
+// own 6 are left, in the reference's order: 12 coefficients instead of 36 and no T basis.
+__device__ __forceinline__ double helm_energy_at_node(const HelmTable &h, const HelmRho &r, const double r0[3],
+                                                      const double r1[3], int j) {
+  const double *lo = h.tab + 9 * ((long long)(r.ih - 1) + (long long)h.nrho * (j - 1)), *hi = lo + 9;
+  const double T = __ldg(h.T + j - 1);
+  double f = __ldg(lo) * r0[0];
+  f = f + __ldg(hi) * r1[0];
+  f = f + __ldg(lo + 3) * r0[1];
+  f = f + __ldg(hi + 3) * r1[1];
+  f = f + __ldg(lo + 4) * r0[2];
+  f = f + __ldg(hi + 4) * r1[2];
+  double df_dT = __ldg(lo + 1) * r0[0];
+  df_dT = df_dT + __ldg(hi + 1) * r1[0];
+  df_dT = df_dT + __ldg(lo + 5) * r0[1];
+  df_dT = df_dT + __ldg(hi + 5) * r1[1];
+  df_dT = df_dT + __ldg(lo + 6) * r0[2];
+  df_dT = df_dT + __ldg(hi + 6) * r1[2];
+  double s = -r.Ye * df_dT;
+  double e = r.Ye * f + T * s;
+  double T2 = T * T, T3 = T2 * T, T4 = T3 * T;
+  const double aT4 = CONST_RAD * T4;
+  return e + 1.5 * CONST_RGAS * T * r.iabar + (r.ok && helm_in_range(T) ? div_by(aT4, r.rho, r.irho) : aT4 / r.rho);
+}
+__device__ __forceinline__ double helm_given2_energy(const HelmTable &h, double rho, double T, double abar, double zbar) {
+  const HelmRho r = helm_rho_part(h, rho, abar, zbar);
+  double r0[3], r1[3], E, dE;
+  helm_rho_bases(r, r0, r1);
+  HelmTemp t;
+  helm_energy<false>(h, r, r0, r1, t, T, E, dE);
+  return E;
 }
 
-// helm_rhoT_given1 (source.F90:24234-24569): P and dP/dT
-__device__ __forceinline__ void helm_given1(const HelmTable &h, double rho, double T, double abar,
-                                            double zbar, double &P, double &dPdT, bool want_deriv) {
-  HelmPos p;
-  helm_locate(h, rho, T, abar, zbar, p);
+// helm_rhoT_given1 (source.F90:24234-24569): P and dP/dT; dr0, dr1 the derivative density bases
+__device__ __forceinline__ void helm_rho_dbases(const HelmTable &h, const HelmRho &r, double dr0[3], double dr1[3]) {
+  const double idrho = __ldg(h.inv_drho + r.ih - 1);
+  hb1(r.x, idrho, r.drho, dr0);
+  hb1m(r.omx, idrho, r.drho, dr1);
+}
+__device__ __forceinline__ void helm_pressure(const HelmTable &h, const HelmRho &r, const double dr0[3],
+                                              const double dr1[3], HelmTemp &t, double T, double &P, double &dPdT) {
+  helm_temp_part(h, T, t);
   double c[36];
-  helm_load36(h, p.ih, p.jh, c);
-  double r0[3], r1[3], t0[3], t1[3];
-  hb1(p.x, p.idrho, p.drho, r0);
-  hb1m(p.omx, p.idrho, p.drho, r1);
-  hb0(p.y, p.dT, p.dT2, t0);
-  hb0m(p.omy, p.dT, p.dT2, t1);
-  double df_drho = helm_sum36(c, r0, r1, t0, t1);
-  double df_drhodT = 0.0;
-  if (want_deriv) {
-    double d0[3], d1[3];
-    hb1(p.y, p.idT, p.dT, d0);
-    hb1m(p.omy, p.idT, p.dT, d1);
-    df_drhodT = helm_sum36(c, r0, r1, d0, d1);
-  }
-  double tmp = p.rhos * p.rhos;
+  helm_load36(h, r.ih, t.jh, c);
+  const double dT2 = t.dT * t.dT;
+  double t0[3], t1[3];
+  hb0(t.y, t.dT, dT2, t0);
+  hb0m(t.omy, t.dT, dT2, t1);
+  double df_drho = helm_sum36(c, dr0, dr1, t0, t1);
+  double d0[3], d1[3];
+  hb1(t.y, t.idT, t.dT, d0);
+  hb1m(t.omy, t.idT, t.dT, d1);
+  double df_drhodT = helm_sum36(c, dr0, dr1, d0, d1);
+  double tmp = r.rhos * r.rhos;
   double pp = tmp * df_drho;
   double dp = tmp * df_drhodT;
   double T2 = T * T, T3 = T2 * T, T4 = T3 * T;
-  tmp = 1.0 / abar;
-  double pion = CONST_RGAS * rho * T * tmp;
-  double dpiondt = CONST_RGAS * rho * tmp;
-  pp = pp + pion + CONST_RAD * T4 * (1.0 / 3.0);
-  dp = dp + dpiondt + (4.0 / 3.0) * CONST_RAD * T3;
-  P = pp;
-  dPdT = dp;
+  double pion = CONST_RGAS * r.rho * T * r.iabar;
+  double dpiondt = CONST_RGAS * r.rho * r.iabar;
+  P = pp + pion + CONST_RAD * T4 * (1.0 / 3.0);
+  dPdT = dp + dpiondt + (4.0 / 3.0) * CONST_RAD * T3;
 }
 
 // helm_rhoT_given_full (source.F90:23686-24232): P, E, relativistic sound speed, cv
-__device__ __forceinline__ void helm_given_full(const HelmTable &h, double rho, double T, double abar,
-                                                double zbar, double &P, double &E, double &sound,
-                                                double &cv) {
-  HelmPos p;
-  helm_locate(h, rho, T, abar, zbar, p);
+__device__ __forceinline__ void helm_full(const HelmTable &h, const HelmRho &r, HelmTemp &t, double T, double &P,
+                                          double &E, double &sound, double &cv) {
+  helm_temp_part(h, T, t);
   double c[36];
-  helm_load36(h, p.ih, p.jh, c);
+  helm_load36(h, r.ih, t.jh, c);
+  const double dT2 = t.dT * t.dT, idT2 = t.idT * t.idT;
   double r0[3], r1[3], t0[3], t1[3], dr0[3], dr1[3], dt0[3], dt1[3], et0[3], et1[3];
-  hb0(p.x, p.drho, p.drho2, r0);
-  hb0m(p.omx, p.drho, p.drho2, r1);
-  hb0(p.y, p.dT, p.dT2, t0);
-  hb0m(p.omy, p.dT, p.dT2, t1);
+  helm_rho_bases(r, r0, r1);
+  hb0(t.y, t.dT, dT2, t0);
+  hb0m(t.omy, t.dT, dT2, t1);
   double f = helm_sum36(c, r0, r1, t0, t1);
-  hb1(p.x, p.idrho, p.drho, dr0);
-  hb1m(p.omx, p.idrho, p.drho, dr1);
+  helm_rho_dbases(h, r, dr0, dr1);
   double df_drho = helm_sum36(c, dr0, dr1, t0, t1);
-  hb1(p.y, p.idT, p.dT, dt0);
-  hb1m(p.omy, p.idT, p.dT, dt1);
+  hb1(t.y, t.idT, t.dT, dt0);
+  hb1m(t.omy, t.idT, t.dT, dt1);
   double df_dT = helm_sum36(c, r0, r1, dt0, dt1);
   double df_drhodT = helm_sum36(c, dr0, dr1, dt0, dt1);
-  hb2(p.y, p.idT2, p.idT, et0);
-  hb2m(p.omy, p.idT2, p.idT, et1);
+  hb2(t.y, idT2, t.idT, et0);
+  hb2m(t.omy, idT2, t.idT, et1);
   double df_dT2 = helm_sum36(c, r0, r1, et0, et1);
   // bicubic Hermite of dP/d(rho Ye) (source.F90:24082-24118)
-  double x = p.x, x2 = x * x, x3 = x2 * x, omx = p.omx, omx2 = omx * omx, omx3 = omx2 * omx;
-  double y = p.y, y2 = y * y, y3 = y2 * y, omy = p.omy, omy2 = omy * omy, omy3 = omy2 * omy;
+  double x = r.x, x2 = x * x, x3 = x2 * x, omx = r.omx, omx2 = omx * omx, omx3 = omx2 * omx;
+  double y = t.y, y2 = y * y, y3 = y2 * y, omy = t.omy, omy2 = omy * omy, omy3 = omy2 * omy;
   double p0r = 2.0 * x3 - 3.0 * x2 + 1.0;
-  double p1r = (x3 - 2.0 * x2 + x) * p.drho;
+  double p1r = (x3 - 2.0 * x2 + x) * r.drho;
   double p0mr = 2.0 * omx3 - 3.0 * omx2 + 1.0;
-  double p1mr = -(omx3 - 2.0 * omx2 + omx) * p.drho;
+  double p1mr = -(omx3 - 2.0 * omx2 + omx) * r.drho;
   double p0t = 2.0 * y3 - 3.0 * y2 + 1.0;
-  double p1t = (y3 - 2.0 * y2 + y) * p.dT;
+  double p1t = (y3 - 2.0 * y2 + y) * t.dT;
   double p0mt = 2.0 * omy3 - 3.0 * omy2 + 1.0;
-  double p1mt = -(omy3 - 2.0 * omy2 + omy) * p.dT;
-  const double *q00 = h.dpdr + 4 * ((long long)(p.ih - 1) + (long long)h.nrho * (p.jh - 1));
+  double p1mt = -(omy3 - 2.0 * omy2 + omy) * t.dT;
+  const double *q00 = h.dpdr + 4 * ((long long)(r.ih - 1) + (long long)h.nrho * (t.jh - 1));
   const double *q10 = q00 + 4, *q01 = q00 + 4 * (long long)h.nrho, *q11 = q01 + 4;
   double l[16];
 #pragma unroll
@@ -744,24 +838,26 @@ __device__ __forceinline__ void helm_given_full(const HelmTable &h, double rho, 
                    l[4] * p0r * p1t + l[5] * p0mr * p1t + l[6] * p0r * p1mt + l[7] * p0mr * p1mt +
                    l[8] * p1r * p0t + l[9] * p1mr * p0t + l[10] * p1r * p0mt + l[11] * p1mr * p0mt +
                    l[12] * p1r * p1t + l[13] * p1mr * p1t + l[14] * p1r * p1mt + l[15] * p1mr * p1mt;
-  dP_drho = p.Ye * dP_drho;
-  double tmp = p.rhos * p.rhos;
+  dP_drho = r.Ye * dP_drho;
+  const double rho = r.rho, tmp2 = r.iabar;
+  double tmp = r.rhos * r.rhos;
   double pp = tmp * df_drho;
   double dP_dT = tmp * df_drhodT;
-  double s = -p.Ye * df_dT;
-  double ds_dT = -p.Ye * df_dT2;
-  double e = p.Ye * f + T * s;
+  double s = -r.Ye * df_dT;
+  double ds_dT = -r.Ye * df_dT2;
+  double e = r.Ye * f + T * s;
   double dE_dT = T * ds_dT;
-  tmp = 1.0 / abar;
   double T2 = T * T, T3 = T2 * T, T4 = T3 * T;
-  double pion = CONST_RGAS * rho * T * tmp;
-  double dpiondt = CONST_RGAS * rho * tmp;
-  double dpiondd = CONST_RGAS * T * tmp;
+  double pion = CONST_RGAS * rho * T * tmp2;
+  double dpiondt = CONST_RGAS * rho * tmp2;
+  double dpiondd = CONST_RGAS * T * tmp2;
   pp = pp + pion + CONST_RAD * T4 * (1.0 / 3.0);
   dP_dT = dP_dT + dpiondt + (4.0 / 3.0) * CONST_RAD * T3;
   dP_drho = dP_drho + dpiondd;
-  e = e + 1.5 * CONST_RGAS * T * tmp + CONST_RAD * T4 / rho;
-  dE_dT = dE_dT + 1.5 * CONST_RGAS * tmp + 4.0 * CONST_RAD * T3 / rho;
+  const bool safe = r.ok && helm_in_range(T);
+  const double aT4 = CONST_RAD * T4, aT3 = 4.0 * CONST_RAD * T3;
+  e = e + 1.5 * CONST_RGAS * T * tmp2 + (safe ? div_by(aT4, rho, r.irho) : aT4 / rho);
+  dE_dT = dE_dT + 1.5 * CONST_RGAS * tmp2 + (safe ? div_by(aT3, rho, r.irho) : aT3 / rho);
   double zz = pp / rho;
   double c_v = dE_dT;
   double chiT = T / pp * dP_dT;
@@ -774,19 +870,26 @@ __device__ __forceinline__ void helm_given_full(const HelmTable &h, double rho, 
   cv = c_v;
   sound = CONST_C * sqrt(gam1 / z);
 }
+__device__ __forceinline__ void helm_given_full(const HelmTable &h, double rho, double T, double abar,
+                                                double zbar, double &P, double &E, double &sound,
+                                                double &cv) {
+  HelmTemp t;
+  helm_full(h, helm_rho_part(h, rho, abar, zbar), t, T, P, E, sound, cv);
+}
 
 // helm_rhoe_given Newton (source.F90:24982-25019).  Returns the iterations used; `clamped`
 // counts resets to the starting guess after leaving [Tl_eos, Th_eos].
-__device__ __forceinline__ int helm_rhoe_newton(const HelmTable &h, double rho, double E0, double abar,
-                                                double zbar, double &T, int max_iter, int &clamped,
-                                                bool *converged = nullptr) {
+__device__ __forceinline__ int helm_rhoe_newton(const HelmTable &h, const HelmRho &r, HelmTemp &t, double E0, double &T,
+                                                int max_iter, int &clamped, bool *converged = nullptr) {
   double Told = T;
   int used = 0;
   bool conv = false;
+  double r0[3], r1[3];
+  helm_rho_bases(r, r0, r1);
   for (int iter = 1; iter <= max_iter; ++iter) {
     used = iter;
     double E, dE;
-    helm_given2(h, rho, T, abar, zbar, E, dE, true);
+    helm_energy<true>(h, r, r0, r1, t, T, E, dE);
     double res = E - E0;
     T = T - res / dE;
     double error = fabs(res / E0);
@@ -802,14 +905,16 @@ __device__ __forceinline__ int helm_rhoe_newton(const HelmTable &h, double rho, 
 }
 
 // helm_rhoP_given Newton (source.F90:24943-24980)
-__device__ __forceinline__ int helm_rhoP_newton(const HelmTable &h, double rho, double P0, double abar,
-                                                double zbar, double &T, int &clamped) {
+__device__ __forceinline__ int helm_rhoP_newton(const HelmTable &h, const HelmRho &r, HelmTemp &t, double P0, double &T,
+                                                int &clamped) {
   double Told = T;
   int used = 0;
+  double dr0[3], dr1[3];
+  helm_rho_dbases(h, r, dr0, dr1);
   for (int iter = 1; iter <= 100; ++iter) {
     used = iter;
     double P, dP;
-    helm_given1(h, rho, T, abar, zbar, P, dP, true);
+    helm_pressure(h, r, dr0, dr1, t, T, P, dP);
     double res = P - P0;
     T = T - res / dP;
     double error = fabs(res / P0);
@@ -828,9 +933,11 @@ __device__ __forceinline__ int helm_rhoP_newton(const HelmTable &h, double rho, 
 __device__ __forceinline__ void helm_side_eos_inl(const HelmTable &h, double rho, double p, double abar,
                                                   double zbar, double T, double &rhoe, double &sound) {
   int clamped = 0;
-  helm_rhoP_newton(h, rho, p, abar, zbar, T, clamped);
+  const HelmRho r = helm_rho_part(h, rho, abar, zbar);
+  HelmTemp t;
+  helm_rhoP_newton(h, r, t, p, T, clamped);
   double Pd, E, cv;
-  helm_given_full(h, rho, T, abar, zbar, Pd, E, sound, cv);
+  helm_full(h, r, t, T, Pd, E, sound, cv);
   rhoe = E * rho;
 }
 

@@ -21,22 +21,25 @@
 
 namespace phl {
 
-constexpr int EOS_MINB_DEFAULT = 4;
+// Resident blocks of 128 threads per SM the inversion kernels are compiled for: 3 (168 registers).
+// 2^22 samples on B200, learned guess 2.62 ms against 2.84 at 4 (128 registers, 850 B of spills) and
+// 2.91 at 2 (unbounded); 10^6 samples, bracket guess 0.49 ms against 0.55 and 0.55.  The 36
+// coefficients kept in shared memory between the evaluations of a solve ran 3 to 5% slower.
+constexpr int EOS_MINB = 3;
 
 // cold guess; returns the number of EoS evaluations the search used
-__device__ __forceinline__ int bracket_guess(const HelmTable &h, double rho, double e, double abar, double zbar,
-                                             double &Tg) {
+__device__ __forceinline__ int bracket_guess(const HelmTable &h, const HelmRho &r, HelmTemp &t, double e, double &Tg) {
   int lo = 0, hi = h.nT - 1;
-  double elo, ehi, dd;
-  helm_given2(h, rho, __ldg(h.T + lo), abar, zbar, elo, dd, false);
+  double r0[3], r1[3], elo, ehi, dd;
+  helm_rho_bases(r, r0, r1);
+  elo = helm_energy_at_node(h, r, r0, r1, lo + 1);
   if (e <= elo) { Tg = __ldg(h.T + lo); return 1; }
-  helm_given2(h, rho, __ldg(h.T + hi) * 0.999999, abar, zbar, ehi, dd, false);
+  helm_energy<false>(h, r, r0, r1, t, __ldg(h.T + hi) * 0.999999, ehi, dd);
   if (e >= ehi) { Tg = __ldg(h.T + hi) * 0.999999; return 2; }
   int evals = 2;
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
-    double em;
-    helm_given2(h, rho, __ldg(h.T + mid), abar, zbar, em, dd, false);
+    const double em = helm_energy_at_node(h, r, r0, r1, mid + 1);
     ++evals;
     if (em <= e) { lo = mid; elo = em; } else { hi = mid; ehi = em; }
   }
@@ -50,9 +53,7 @@ __global__ void k_eos_energy(HelmTable h, long long n, const double *rho, const 
                              const double *zbar, double *e) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  double E, dd;
-  helm_given2(h, rho[t], T[t], abar[t], zbar[t], E, dd, false);
-  e[t] = E;
+  e[t] = helm_given2_energy(h, rho[t], T[t], abar[t], zbar[t]);
 }
 
 // per-warp sums of the batch statistics into the context's counters
@@ -73,12 +74,12 @@ struct EosStat {
 };
 
 // outputs of one finished inversion
-__device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, double r, double ab, double zb,
+__device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, const HelmRho &r, HelmTemp &ht,
                                            double Tg, int used, double *T, double *p, double *cs, int *iters) {
   T[t] = Tg;
   if (p || cs) {
     double P, E, snd, cv;
-    helm_given_full(h, r, Tg, ab, zb, P, E, snd, cv);
+    helm_full(h, r, ht, Tg, P, E, snd, cv);
     if (p) p[t] = P;
     if (cs) cs[t] = snd;
   }
@@ -91,8 +92,8 @@ __device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, doub
 // appended to `queue` (queue[0] = count, then index | judged iterations << 56) for phase 2, so
 // that the fallback runs in converged warps instead of stalling the accepted lanes.
 // LEARNED selects the learned-guess instantiation (guess 1); the other carries no tensor-core code.
-template <bool LEARNED, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_eos_invert(HelmTable h, long long n, const double *rho, const double *e,
+template <bool LEARNED>
+__global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long long n, const double *rho, const double *e,
                                                     const double *abar, const double *zbar, double *T,
                                                     double *p, double *cs, int *iters, int guess, MlpWeights mw,
                                                     unsigned long long *stat, unsigned long long *queue) {
@@ -114,33 +115,35 @@ __global__ void __launch_bounds__(128, MINB) k_eos_invert(HelmTable h, long long
   bool reject = false;
   int judged = 0;
   if (t < n) {
-    const double r = rho[t], ee = e[t], ab = abar[t], zb = zbar[t];
+    const double ee = e[t];
+    const HelmRho r = helm_rho_part(h, rho[t], abar[t], zbar[t]);
+    HelmTemp ht;
     double Tg;
     int used = 0, clamped = 0;
     bool conv = false;
     if constexpr (LEARNED) {
       Tg = fmin(fmax(exp10((double)lT_mlp), h.Tl * 1.000001), h.Th * 0.999999);
-      used = helm_rhoe_newton(h, r, ee, ab, zb, Tg, 3, clamped, &conv);
+      used = helm_rhoe_newton(h, r, ht, ee, Tg, 3, clamped, &conv);
       st.v[3] = clamped;
       if (conv && clamped == 0) {
         st.v[0] = 1;
         st.v[1] = used;
         st.v[4] = 1;
-        eos_finish(h, t, r, ab, zb, Tg, used, T, p, cs, iters);
+        eos_finish(h, t, r, ht, Tg, used, T, p, cs, iters);
       } else {
         reject = true;
         judged = used;
         st.v[5] = 1;
       }
     } else {
-      if (guess == PHL_GUESS_BRACKET) st.v[6] = bracket_guess(h, r, ee, ab, zb, Tg);
+      if (guess == PHL_GUESS_BRACKET) st.v[6] = bracket_guess(h, r, ht, ee, Tg);
       else Tg = T[t];
-      used = helm_rhoe_newton(h, r, ee, ab, zb, Tg, 100, clamped, &conv);
+      used = helm_rhoe_newton(h, r, ht, ee, Tg, 100, clamped, &conv);
       st.v[0] = 1;
       st.v[1] = used;
       st.v[2] = !conv;
       st.v[3] = clamped;
-      eos_finish(h, t, r, ab, zb, Tg, used, T, p, cs, iters);
+      eos_finish(h, t, r, ht, Tg, used, T, p, cs, iters);
     }
   }
   if constexpr (LEARNED) {
@@ -161,8 +164,7 @@ __global__ void __launch_bounds__(128, MINB) k_eos_invert(HelmTable h, long long
 
 // Phase 2 of the learned guess: the reference Newton from the bracket guess for the rejected
 // samples (grid-stride over the queue written by phase 1)
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) k_eos_fallback(HelmTable h, const unsigned long long *queue,
+__global__ void __launch_bounds__(128, EOS_MINB) k_eos_fallback(HelmTable h, const unsigned long long *queue,
                                                       const double *rho, const double *e, const double *abar,
                                                       const double *zbar, double *T, double *p, double *cs,
                                                       int *iters, unsigned long long *stat) {
@@ -178,17 +180,19 @@ __global__ void __launch_bounds__(128, MINB) k_eos_fallback(HelmTable h, const u
       const unsigned long long ent = queue[1 + q];
       const long long t = (long long)(ent & ((1ull << 56) - 1));
       const int judged = (int)(ent >> 56);
-      const double r = rho[t], ee = e[t], ab = abar[t], zb = zbar[t];
+      const double ee = e[t];
+      const HelmRho r = helm_rho_part(h, rho[t], abar[t], zbar[t]);
+      HelmTemp ht;
       double Tg;
-      st.v[6] += bracket_guess(h, r, ee, ab, zb, Tg);
+      st.v[6] += bracket_guess(h, r, ht, ee, Tg);
       int clamped = 0;
       bool conv = false;
-      const int used = helm_rhoe_newton(h, r, ee, ab, zb, Tg, 100, clamped, &conv);
+      const int used = helm_rhoe_newton(h, r, ht, ee, Tg, 100, clamped, &conv);
       st.v[0] += 1;
       st.v[1] += judged + used;
       st.v[2] += !conv;
       st.v[3] += clamped;
-      eos_finish(h, t, r, ab, zb, Tg, judged + used, T, p, cs, iters);
+      eos_finish(h, t, r, ht, Tg, judged + used, T, p, cs, iters);
     }
   }
   st.flush(stat);
@@ -196,50 +200,24 @@ __global__ void __launch_bounds__(128, MINB) k_eos_fallback(HelmTable h, const u
 
 // Launch the inversion on stream s (no synchronisation).  `queue` (n + 1 entries) is needed for
 // the learned guess only.  Returns 0 or a cudaError_t.
-// Resident blocks per SM the inversion kernels are compiled for: 4 caps them at 128 registers
-// (2^24 samples on B200: learned guess 1.66e9 inversions/s, bracket 1.39e9, against 1.34e9 and
-// 1.07e9 with 1, which lets the compiler keep the whole inlined evaluation in ~190 registers at
-// two blocks per SM, and 1.17e9 / 1.04e9 with 6); PHL_EOS_MINB=1 or 3 selects the others.
-inline int eos_minb() {
-  static const int v = [] {
-    const char *e = getenv("PHL_EOS_MINB");
-    const int m = e ? atoi(e) : EOS_MINB_DEFAULT;
-    return (m == 1 || m == 3 || m == 4) ? m : EOS_MINB_DEFAULT;
-  }();
-  return v;
-}
-
-template <int MINB>
-inline int eos_launch_t(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *e,
-                        const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters,
-                        int guess, MlpWeights mw, unsigned long long *stat, unsigned long long *queue, int nsm) {
+inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *e,
+                      const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters,
+                      int guess, MlpWeights mw, unsigned long long *stat, unsigned long long *queue, int nsm) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
   if (guess != PHL_GUESS_MLP) {
-    k_eos_invert<false, MINB><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat,
+    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat,
                                                       nullptr);
     return (int)cudaGetLastError();
   }
   const size_t sm = sizeof(MlpUmmaSmem);
-  cudaError_t err = cudaFuncSetAttribute(k_eos_invert<true, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t err = cudaFuncSetAttribute(k_eos_invert<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (err == cudaSuccess) err = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (err != cudaSuccess) return (int)err;
-  k_eos_invert<true, MINB><<<blocks, 128, sm, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue);
+  k_eos_invert<true><<<blocks, 128, sm, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue);
   // enough resident blocks to cover every SM several times; the loop covers any queue length
   const unsigned fb = (unsigned)std::min<long long>((long long)nsm * 8, (long long)blocks);
-  k_eos_fallback<MINB><<<fb, 128, 0, s>>>(h, queue, rho, e, abar, zbar, T, p, cs, iters, stat);
+  k_eos_fallback<<<fb, 128, 0, s>>>(h, queue, rho, e, abar, zbar, T, p, cs, iters, stat);
   return (int)cudaGetLastError();
-}
-
-// Launch the inversion on stream s (no synchronisation).  `queue` (n + 1 entries) is needed for
-// the learned guess only.  Returns 0 or a cudaError_t.
-inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *e,
-                      const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters,
-                      int guess, MlpWeights mw, unsigned long long *stat, unsigned long long *queue, int nsm) {
-  switch (eos_minb()) {
-    case 3: return eos_launch_t<3>(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue, nsm);
-    case 4: return eos_launch_t<4>(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue, nsm);
-    default: return eos_launch_t<1>(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue, nsm);
-  }
 }
 
 struct EosBatch {

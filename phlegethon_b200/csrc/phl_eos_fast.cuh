@@ -15,19 +15,6 @@
 
 namespace phl {
 
-// table node index (1-based like the reference) of x in the log-spaced nodes: an estimate in
-// single precision (within one node of the cell for any x in the table's range), then exact
-// comparisons against the node values
-__device__ __forceinline__ int helm_node_index(const double *nodes, int n, double log10_first, double dlog,
-                                               double x) {
-  const float lx = __log2f((float)x) * 0.30102999566398120f;
-  int i = (int)(__fdividef(lx - (float)log10_first, (float)dlog)) + 1;
-  i = max(1, min(i, n - 1));
-  if (i < n - 1 && __ldg(nodes + i) <= x) ++i;
-  if (i > 1 && __ldg(nodes + i - 1) > x) --i;
-  return i;
-}
-
 // The quintic Hermite bases of the table interpolation (source.F90:24708-24738) and their first
 // derivatives, in nested (Horner) form with fused multiply-adds: the same polynomials as hb0 ..
 // hb1m of phl_device.cuh, which keep the reference's term order for the FP64 form; here they

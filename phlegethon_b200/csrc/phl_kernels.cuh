@@ -810,10 +810,12 @@ __global__ void __launch_bounds__(128, C::MINB_C2P64) k_c2p(Prm P) {
       double zbar = ye * abar;
       T = P.temp[c];
       int clamped = 0;
-      int it = helm_rhoe_newton(P.helm, rho, eint * inv_rho, abar, zbar, T, 100, clamped);
+      const HelmRho hr = helm_rho_part(P.helm, rho, abar, zbar);
+      HelmTemp ht;
+      int it = helm_rhoe_newton(P.helm, hr, ht, eint * inv_rho, T, 100, clamped);
       n_calls += 1; n_iters += it; n_nonconv += (it == 100); n_clamp += clamped;
       double E, cv;
-      helm_given_full(P.helm, rho, T, abar, zbar, p, E, sound, cv);
+      helm_full(P.helm, hr, ht, T, p, E, sound, cv);
       if (C::FAST) {
         P.gout[c] = p / eint + 1.0;
         P.gout[g.N + c] = sound * sound * rho / p;
@@ -926,8 +928,10 @@ __global__ void __launch_bounds__(128) k_init_thermo(Prm P) {
     double zbar = abar * ye, sound, cv, Pdummy;
     T = P.temp[c];
     int clamped = 0;
-    helm_rhoP_newton(P.helm, rho, p, abar, zbar, T, clamped);
-    helm_given_full(P.helm, rho, T, abar, zbar, Pdummy, eint, sound, cv);
+    const HelmRho hr = helm_rho_part(P.helm, rho, abar, zbar);
+    HelmTemp ht;
+    helm_rhoP_newton(P.helm, hr, ht, p, T, clamped);
+    helm_full(P.helm, hr, ht, T, Pdummy, eint, sound, cv);
     eint = rho * eint;
     if (C::FAST) {
       P.gout[c] = p / eint + 1.0;

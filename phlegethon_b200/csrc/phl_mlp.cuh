@@ -38,9 +38,10 @@ __host__ __device__ __forceinline__ void mlp_features(double rho, double e_th, d
 }
 // cold (lowest-table-temperature) specific energy of the mixture at rho
 __device__ __forceinline__ double mlp_cold_energy(const HelmTable &h, double rho, double abar, double zbar) {
-  double E, dE;
-  helm_given2(h, rho, __ldg(h.T), abar, zbar, E, dE, false);
-  return E;
+  const HelmRho r = helm_rho_part(h, rho, abar, zbar);
+  double r0[3], r1[3];
+  helm_rho_bases(r, r0, r1);
+  return helm_energy_at_node(h, r, r0, r1, 1);
 }
 // Fixed (non-trained) skip connection: log10 of the temperature at which ideal ions plus
 // radiation alone would hold e_th, (T_ion^-4 + T_rad^-4)^(-1/4) with T_ion = e_th Abar / (3/2 R)
@@ -91,8 +92,8 @@ static __global__ void k_mlp_make_samples(HelmTable h, long long n, unsigned lon
   double abar = r.abar[0] + (r.abar[1] - r.abar[0]) * u01(seed, i, 2);
   double zbar = r.zbar[1] > 0.0 ? r.zbar[0] + (r.zbar[1] - r.zbar[0]) * u01(seed, i, 3)
                                 : 1.0 + fmax(abar * 0.5 - 1.0, 0.0) * u01(seed, i, 3);
-  double rho = exp10(lrho), T = exp10(lT), E, dE;
-  helm_given2(h, rho, T, abar, zbar, E, dE, false);
+  double rho = exp10(lrho), T = exp10(lT);
+  const double E = helm_given2_energy(h, rho, T, abar, zbar);
   float f[4];
   mlp_features(rho, E - mlp_cold_energy(h, rho, abar, zbar), abar, zbar, f);
   for (int k = 0; k < 4; ++k) feat[i * 4 + k] = f[k];
