@@ -8,12 +8,13 @@
 // Training (all on the device): samples are drawn with a counter-based hash over the EoS
 // benchmark ranges and labelled by the forward EoS (helm_rhoT_given2); each step a CTA takes 64
 // samples through forward and backward passes (three 64x64x64 tensor-core products: layer-2
-// forward, dH1 = dH2 W2, dW2 = dH2^T H1), writes its partial gradient, a second kernel sums the
-// partials in a fixed order (deterministic), and a third applies Adam.
+// forward, dH1 = dH2 W2, dW2 = dH2^T H1) and writes its partial gradient; a second kernel sums the
+// partials in a fixed order (deterministic) and applies Adam.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <mma.h>
+#include <cmath>
 #include "phl_device.cuh"
 #include "phl_umma.cuh"
 
@@ -101,179 +102,219 @@ static __global__ void k_mlp_make_samples(HelmTable h, long long n, unsigned lon
 }
 
 // ------------------------------------------------------------------ training step (one CTA = 64 samples)
-// shared layout (bytes): X 64x4 f32 | T 64 f32 | H1 64x64 f32 | H1b 64x64 bf16 | W2b 64x64 bf16 |
-// Z 64x64 f32 (Z2, later dH1) | G 64x64 bf16 (dH2) | Gf 64x64 f32 (dH2) | y 64 f32
+// Rows of the FP32 scratch are 68 floats long and those of the BF16 tiles 72 elements, so that the
+// 16-row tensor-core accesses and the column walks both spread over the banks.
+constexpr int MLP_LDF = 68, MLP_LDB = 72;
+constexpr int MLP_TRAIN_THREADS = 256, MLP_TRAIN_Q = MLP_TRAIN_THREADS / MLP_H;  // 4 threads per hidden unit
+constexpr int MLP_PSTRIDE = 4608;  // floats per partial gradient (tiles of dW2 start on 32 bytes)
 struct MlpTrainSmem {
+  alignas(32) float Z[MLP_TILE][MLP_LDF];  // layer-2 product, later dH1
+  alignas(32) __nv_bfloat16 H1b[MLP_TILE][MLP_LDB];
+  alignas(32) __nv_bfloat16 W2b[MLP_H][MLP_LDB];
+  alignas(32) __nv_bfloat16 Gb[MLP_TILE][MLP_LDB];  // dH2
   float X[MLP_TILE][4];
-  float T[MLP_TILE];
-  float y[MLP_TILE];
-  float H1[MLP_TILE][MLP_H];
-  float Z[MLP_TILE][MLP_H];
-  float Gf[MLP_TILE][MLP_H];
-  alignas(32) __nv_bfloat16 H1b[MLP_TILE][MLP_H];
-  alignas(32) __nv_bfloat16 W2b[MLP_H][MLP_H];
-  alignas(32) __nv_bfloat16 Gb[MLP_TILE][MLP_H];
-  alignas(32) float dW2[MLP_H][MLP_H];
+  float y[MLP_TILE];                       // dL/dy
+  float part[MLP_TRAIN_Q][5][MLP_H];       // column sums of the 4 threads of a hidden unit
 };
 
-static __global__ void __launch_bounds__(128) k_mlp_train_step(const float *params, const __nv_bfloat16 *w2bf,
+// Forward and backward pass of 64 samples, the partial gradient to partial[block].  8 warps: a thread
+// owns one hidden unit and a quarter of the samples in the FP32 parts (its weights stay in registers,
+// the column sums need one exchange), two 16 x 16 tiles of each product in the tensor-core parts.
+// Bound by the chain of its phases, not by a rate: 128 such blocks are one block on most SMs.
+static __global__ void __launch_bounds__(MLP_TRAIN_THREADS) k_mlp_train_step(const float *params, const __nv_bfloat16 *w2bf,
                                                         const float *feat, const float *target, long long n,
                                                         long long offset, int batch, float *partial,
                                                         float *loss_partial) {
   using namespace nvcuda;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   MlpTrainSmem &S = *reinterpret_cast<MlpTrainSmem *>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const float *W1 = params + MLP_OFF_W1, *b1 = params + MLP_OFF_B1, *b2 = params + MLP_OFF_B2;
-  const float *W3 = params + MLP_OFF_W3, b3 = params[MLP_OFF_B3];
+  const int tid = threadIdx.x, warp = tid >> 5, o = tid % MLP_H, q4 = tid / MLP_H;
+  constexpr int NS = MLP_TILE / MLP_TRAIN_Q;  // samples per thread in the FP32 parts
   const long long base = offset + (long long)blockIdx.x * MLP_TILE;
-  // samples (wrapping around the training set)
-  for (int q = tid; q < MLP_TILE * 4; q += blockDim.x) {
-    long long s = (base + q / 4) % n;
-    S.X[q / 4][q % 4] = feat[s * 4 + q % 4];
-  }
-  for (int q = tid; q < MLP_TILE; q += blockDim.x) S.T[q] = target[(base + q) % n];
-  for (int q = tid; q < MLP_H * MLP_H; q += blockDim.x) S.W2b[q / MLP_H][q % MLP_H] = w2bf[q];
+  // samples (wrapping around the training set), W2
+  if (tid < MLP_TILE) *reinterpret_cast<float4 *>(S.X[tid]) = __ldg(reinterpret_cast<const float4 *>(feat) + (base + tid) % n);
+  for (int q = tid; q < MLP_H * MLP_H / 8; q += MLP_TRAIN_THREADS)
+    *reinterpret_cast<uint4 *>(&S.W2b[q / 8][8 * (q % 8)]) = reinterpret_cast<const uint4 *>(w2bf)[q];
+  const float4 w1 = reinterpret_cast<const float4 *>(params + MLP_OFF_W1)[o];
+  const float b1 = params[MLP_OFF_B1 + o], b2 = params[MLP_OFF_B2 + o], w3 = params[MLP_OFF_W3 + o];
   __syncthreads();
   // layer 1 (FP32)
-  for (int q = tid; q < MLP_TILE * MLP_H; q += blockDim.x) {
-    int s = q / MLP_H, o = q % MLP_H;
-    float a = b1[o];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a = fmaf(W1[o * 4 + k], S.X[s][k], a);
-    a = fmaxf(a, 0.0f);
-    S.H1[s][o] = a;
-    S.H1b[s][o] = __float2bfloat16(a);
+#pragma unroll 4
+  for (int k = 0; k < NS; ++k) {
+    const int s = q4 * NS + k;
+    const float4 x = *reinterpret_cast<const float4 *>(S.X[s]);
+    const float a = fmaf(w1.w, x.w, fmaf(w1.z, x.z, fmaf(w1.y, x.y, fmaf(w1.x, x.x, b1))));
+    S.H1b[s][o] = __float2bfloat16(fmaxf(a, 0.0f));
   }
   __syncthreads();
-  // layer 2 on the tensor cores: Z[s][o] = sum_i H1[s][i] W2[o][i]; warp w owns rows 16w..16w+15
+  // layer 2 on the tensor cores: Z[s][o] = sum_i H1[s][i] W2[o][i]; warp w owns the tiles of rows
+  // 16 (w / 2) and columns 32 (w % 2) .. + 31
+  const int r0 = 16 * (warp >> 1), c0 = 32 * (warp & 1);
   {
     wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major> a;
     wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::col_major> b;
-    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
+    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc[2];
+    wmma::fill_fragment(acc[0], 0.0f);
+    wmma::fill_fragment(acc[1], 0.0f);
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      wmma::fill_fragment(acc, 0.0f);
+    for (int kt = 0; kt < 4; ++kt) {
+      wmma::load_matrix_sync(a, &S.H1b[r0][16 * kt], MLP_LDB);
 #pragma unroll
-      for (int kt = 0; kt < 4; ++kt) {
-        wmma::load_matrix_sync(a, &S.H1b[16 * warp][16 * kt], MLP_H);
-        wmma::load_matrix_sync(b, &S.W2b[16 * nt][16 * kt], MLP_H);  // B(k=i, n=o) = W2[o][i]
-        wmma::mma_sync(acc, a, b, acc);
+      for (int t = 0; t < 2; ++t) {
+        wmma::load_matrix_sync(b, &S.W2b[c0 + 16 * t][16 * kt], MLP_LDB);  // B(k=i, n=o) = W2[o][i]
+        wmma::mma_sync(acc[t], a, b, acc[t]);
       }
-      wmma::store_matrix_sync(&S.Z[16 * warp][16 * nt], acc, MLP_H, wmma::mem_row_major);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) wmma::store_matrix_sync(&S.Z[r0][c0 + 16 * t], acc[t], MLP_LDF, wmma::mem_row_major);
+  }
+  __syncthreads();
+  // bias + ReLU and the output layer: 4 threads per sample, 16 hidden units each, then the loss
+  {
+    const int s = tid >> 2, part = tid & 3;
+    float a = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < 16; ++k) {
+      const int u = part + 4 * k;
+      a = fmaf(__ldg(params + MLP_OFF_W3 + u), fmaxf(S.Z[s][u] + __ldg(params + MLP_OFF_B2 + u), 0.0f), a);
+    }
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    if (part == 0) {
+      const float d = a + params[MLP_OFF_B3] - target[(base + s) % n];
+      S.y[s] = 2.0f * d / (float)batch;  // dL/dy for L = mean (y - t)^2
+      loss_partial[blockIdx.x * MLP_TILE + s] = d * d;
     }
   }
   __syncthreads();
-  // bias + ReLU -> H2 (kept in Z), output layer, loss gradient
-  for (int q = tid; q < MLP_TILE * MLP_H; q += blockDim.x) {
-    int s = q / MLP_H, o = q % MLP_H;
-    S.Z[s][o] = fmaxf(S.Z[s][o] + b2[o], 0.0f);
-  }
-  __syncthreads();
-  if (tid < MLP_TILE) {
-    float a = b3;
-    for (int o = 0; o < MLP_H; ++o) a = fmaf(W3[o], S.Z[tid][o], a);
-    float d = a - S.T[tid];
-    S.y[tid] = 2.0f * d / (float)batch;  // dL/dy for L = mean (y - t)^2
-    loss_partial[blockIdx.x * MLP_TILE + tid] = d * d;
-  }
-  __syncthreads();
-  // dH2 = dy W3 * relu'(H2)
-  for (int q = tid; q < MLP_TILE * MLP_H; q += blockDim.x) {
-    int s = q / MLP_H, o = q % MLP_H;
-    float g = S.Z[s][o] > 0.0f ? S.y[s] * W3[o] : 0.0f;
-    S.Gf[s][o] = g;
+  float *P = partial + (long long)blockIdx.x * MLP_PSTRIDE;
+  // dH2 = dy W3 relu'(H2); column sums of dW3 and db2 from FP32 H2 / dH2
+  float gw3 = 0.0f, gb2 = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < NS; ++k) {
+    const int s = q4 * NS + k;
+    const float h2 = fmaxf(S.Z[s][o] + b2, 0.0f), dy = S.y[s];
+    const float g = h2 > 0.0f ? dy * w3 : 0.0f;
     S.Gb[s][o] = __float2bfloat16(g);
+    gw3 = fmaf(dy, h2, gw3);
+    gb2 += g;
   }
+  S.part[q4][0][o] = gw3;
+  S.part[q4][1][o] = gb2;
   __syncthreads();
-  float *P = partial + (long long)blockIdx.x * MLP_NPARAM;
-  // dW3, b3, b2 from FP32 H2 / dH2
-  for (int o = tid; o < MLP_H; o += blockDim.x) {
-    float gw3 = 0.0f, gb2 = 0.0f;
-    for (int s = 0; s < MLP_TILE; ++s) {
-      gw3 = fmaf(S.y[s], S.Z[s][o], gw3);
-      gb2 += S.Gf[s][o];
-    }
-    P[MLP_OFF_W3 + o] = gw3;
-    P[MLP_OFF_B2 + o] = gb2;
+  if (tid < 2 * MLP_H) {
+    const int v = tid / MLP_H;
+    const float g = (S.part[0][v][o] + S.part[1][v][o]) + (S.part[2][v][o] + S.part[3][v][o]);
+    P[(v ? MLP_OFF_B2 : MLP_OFF_W3) + o] = g;
+  } else if (warp == 4) {
+    float g = S.y[tid & 31] + S.y[32 + (tid & 31)];
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) g += __shfl_xor_sync(0xffffffffu, g, m);
+    if ((tid & 31) == 0) P[MLP_OFF_B3] = g;
   }
-  if (tid == 0) {
-    float g = 0.0f;
-    for (int s = 0; s < MLP_TILE; ++s) g += S.y[s];
-    P[MLP_OFF_B3] = g;
-  }
-  __syncthreads();
   // tensor cores: dH1pre[s][i] = sum_o dH2[s][o] W2[o][i] (into Z) and
-  // dW2[o][i] = sum_s dH2[s][o] H1[s][i]
+  // dW2[o][i] = sum_s dH2[s][o] H1[s][i] (to the partial gradient)
   {
     wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major> a;
     wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::row_major> b;
     wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::col_major> at;
-    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
+    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc[2], dw[2];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      wmma::fill_fragment(acc, 0.0f);
-#pragma unroll
-      for (int kt = 0; kt < 4; ++kt) {
-        wmma::load_matrix_sync(a, &S.Gb[16 * warp][16 * kt], MLP_H);     // A(s, o) = dH2[s][o]
-        wmma::load_matrix_sync(b, &S.W2b[16 * kt][16 * nt], MLP_H);      // B(k=o, n=i) = W2[o][i]
-        wmma::mma_sync(acc, a, b, acc);
-      }
-      wmma::store_matrix_sync(&S.Z[16 * warp][16 * nt], acc, MLP_H, wmma::mem_row_major);
+    for (int t = 0; t < 2; ++t) {
+      wmma::fill_fragment(acc[t], 0.0f);
+      wmma::fill_fragment(dw[t], 0.0f);
     }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      wmma::fill_fragment(acc, 0.0f);
+    for (int kt = 0; kt < 4; ++kt) {
+      wmma::load_matrix_sync(a, &S.Gb[r0][16 * kt], MLP_LDB);   // A(s, o) = dH2[s][o]
+      wmma::load_matrix_sync(at, &S.Gb[16 * kt][r0], MLP_LDB);  // A(o, s) = dH2[s][o]
 #pragma unroll
-      for (int kt = 0; kt < 4; ++kt) {
-        wmma::load_matrix_sync(at, &S.Gb[16 * kt][16 * warp], MLP_H);    // A(o, s) = dH2[s][o]
-        wmma::load_matrix_sync(b, &S.H1b[16 * kt][16 * nt], MLP_H);      // B(k=s, n=i) = H1[s][i]
-        wmma::mma_sync(acc, at, b, acc);
+      for (int t = 0; t < 2; ++t) {
+        wmma::load_matrix_sync(b, &S.W2b[16 * kt][c0 + 16 * t], MLP_LDB);  // B(k=o, n=i) = W2[o][i]
+        wmma::mma_sync(acc[t], a, b, acc[t]);
+        wmma::load_matrix_sync(b, &S.H1b[16 * kt][c0 + 16 * t], MLP_LDB);  // B(k=s, n=i) = H1[s][i]
+        wmma::mma_sync(dw[t], at, b, dw[t]);
       }
-      wmma::store_matrix_sync(&S.dW2[16 * warp][16 * nt], acc, MLP_H, wmma::mem_row_major);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      wmma::store_matrix_sync(P + MLP_OFF_W2 + r0 * MLP_H + c0 + 16 * t, dw[t], MLP_H, wmma::mem_row_major);
+      wmma::store_matrix_sync(&S.Z[r0][c0 + 16 * t], acc[t], MLP_LDF, wmma::mem_row_major);
     }
   }
   __syncthreads();
-  for (int q = tid; q < MLP_H * MLP_H; q += blockDim.x) P[MLP_OFF_W2 + q] = S.dW2[q / MLP_H][q % MLP_H];
-  // dH1 = dH1pre * relu'(H1); dW1, db1 (FP32)
-  for (int q = tid; q < MLP_TILE * MLP_H; q += blockDim.x) {
-    int s = q / MLP_H, i = q % MLP_H;
-    S.Z[s][i] = S.H1[s][i] > 0.0f ? S.Z[s][i] : 0.0f;
+  // dH1 = dH1pre relu'(H1) (the BF16 H1 is positive where H1 is); column sums of dW1, db1 (FP32)
+  float g[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+  for (int k = 0; k < NS; ++k) {
+    const int s = q4 * NS + k;
+    const float d = __bfloat162float(S.H1b[s][o]) > 0.0f ? S.Z[s][o] : 0.0f;
+    const float4 x = *reinterpret_cast<const float4 *>(S.X[s]);
+    g[0] = fmaf(d, x.x, g[0]);
+    g[1] = fmaf(d, x.y, g[1]);
+    g[2] = fmaf(d, x.z, g[2]);
+    g[3] = fmaf(d, x.w, g[3]);
+    g[4] += d;
   }
-  __syncthreads();
-  for (int o = tid; o < MLP_H; o += blockDim.x) {
-    float g[4] = {0, 0, 0, 0}, gb = 0.0f;
-    for (int s = 0; s < MLP_TILE; ++s) {
-      float d = S.Z[s][o];
-      gb += d;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) g[k] = fmaf(d, S.X[s][k], g[k]);
-    }
-    for (int k = 0; k < 4; ++k) P[MLP_OFF_W1 + o * 4 + k] = g[k];
-    P[MLP_OFF_B1 + o] = gb;
+  for (int v = 0; v < 5; ++v) S.part[q4][v][o] = g[v];
+  __syncthreads();
+  for (int t = tid; t < 5 * MLP_H; t += MLP_TRAIN_THREADS) {
+    const int v = t / MLP_H, u = t % MLP_H;
+    const float sum = (S.part[0][v][u] + S.part[1][v][u]) + (S.part[2][v][u] + S.part[3][v][u]);
+    if (v < 4) P[MLP_OFF_W1 + 4 * u + v] = sum;
+    else P[MLP_OFF_B1 + u] = sum;
   }
 }
 
-// fixed-order sum of the per-CTA partial gradients
-static __global__ void k_mlp_reduce(const float *partial, int nblocks, float *grad) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= MLP_NPARAM) return;
+// Sum of the partial gradients of one parameter in a fixed order: 8 warps take every eighth partial
+// (coalesced over 32 parameters), their sums meet in shared memory.  Valid in warp 0.
+constexpr int MLP_UPD_THREADS = 256;
+__device__ __forceinline__ float mlp_sum_partials(const float *partial, int nblocks, int p, float (&red)[8][32]) {
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
   float s = 0.0f;
-  for (int b = 0; b < nblocks; ++b) s += partial[(long long)b * MLP_NPARAM + p];
-  grad[p] = s;
+  if (p < MLP_NPARAM) {
+#pragma unroll 8
+    for (int b = seg; b < nblocks; b += 8) s += partial[(long long)b * MLP_PSTRIDE + p];
+  }
+  red[seg][lane] = s;
+  __syncthreads();
+  float r = 0.0f;
+  if (seg == 0)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) r += red[q][lane];
+  return r;
 }
 
-static __global__ void k_mlp_adam(float *params, const float *grad, float *m, float *v, float lr, float b1, float b2,
-                           float eps, int step, __nv_bfloat16 *w2bf) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= MLP_NPARAM) return;
-  float g = grad[p];
-  float mm = b1 * m[p] + (1.0f - b1) * g;
-  float vv = b2 * v[p] + (1.0f - b2) * g * g;
+// the summed gradient of every parameter
+static __global__ void __launch_bounds__(MLP_UPD_THREADS) k_mlp_reduce(const float *partial, int nblocks, float *grad) {
+  __shared__ float red[8][32];
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+  const float g = mlp_sum_partials(partial, nblocks, p, red);
+  if (threadIdx.x < 32 && p < MLP_NPARAM) grad[p] = g;
+}
+
+// The same sum and the Adam update of the parameter in one launch; c1, c2: 1 - beta^step.  One update
+// of the fit (8,192 samples) took 40 us in three launches (27.6 for the gradient, 8.1 and 4.4).
+static __global__ void __launch_bounds__(MLP_UPD_THREADS) k_mlp_adam(const float *partial, int nblocks, float *params, float *m, float *v,
+                                                          float lr, float b1, float b2, float eps, float c1, float c2,
+                                                          __nv_bfloat16 *w2bf) {
+  __shared__ float red[8][32];
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+  const bool mine = threadIdx.x < 32 && p < MLP_NPARAM;
+  float mm = 0.0f, vv = 0.0f, w = 0.0f;
+  if (mine) {
+    mm = m[p];
+    vv = v[p];
+    w = params[p];
+  }
+  const float g = mlp_sum_partials(partial, nblocks, p, red);
+  if (!mine) return;
+  mm = b1 * mm + (1.0f - b1) * g;
+  vv = b2 * vv + (1.0f - b2) * g * g;
   m[p] = mm;
   v[p] = vv;
-  float mh = mm / (1.0f - powf(b1, (float)step)), vh = vv / (1.0f - powf(b2, (float)step));
-  float w = params[p] - lr * mh / (sqrtf(vh) + eps);
+  w = w - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
   params[p] = w;
   if (p >= MLP_OFF_W2 && p < MLP_OFF_B2) w2bf[p - MLP_OFF_W2] = __float2bfloat16(w);
 }
@@ -548,8 +589,8 @@ struct Mlp {
   int gradient(cudaStream_t s, long long offset, int batch, double *loss) {
     int nb = batch / MLP_TILE;
     size_t sm = sizeof(MlpTrainSmem);
-    k_mlp_train_step<<<nb, 128, sm, s>>>(params, w2bf, feat, target, nsamp, offset, batch, partial, lossp);
-    k_mlp_reduce<<<(MLP_NPARAM + 255) / 256, 256, 0, s>>>(partial, nb, grad);
+    k_mlp_train_step<<<nb, MLP_TRAIN_THREADS, sm, s>>>(params, w2bf, feat, target, nsamp, offset, batch, partial, lossp);
+    k_mlp_reduce<<<(MLP_NPARAM + 31) / 32, MLP_UPD_THREADS, 0, s>>>(partial, nb, grad);
     if (cudaGetLastError() != cudaSuccess) return -2;
     if (loss) {
       float *h = new float[batch];
@@ -578,7 +619,7 @@ struct Mlp {
       if (partial) cudaFree(partial);
       if (lossp) cudaFree(lossp);
       partial = lossp = nullptr;
-      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_NPARAM) || cudaMalloc(&lossp, sizeof(float) * batch))
+      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_PSTRIDE) || cudaMalloc(&lossp, sizeof(float) * batch))
         return -2;
       npart = nb;
     }
@@ -600,9 +641,11 @@ struct Mlp {
         ++step;
         double frac = (double)(ep * steps_per_epoch + k) / (double)(epochs * steps_per_epoch);
         float lr_t = (float)(frac < 0.5 ? lr : lr * (1.0 - 1.9 * (frac - 0.5)));
-        if (gradient(s, k * batch, batch, nullptr)) return -2;
-        k_mlp_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, s>>>(params, grad, m, v, lr_t, 0.9f, 0.999f, 1e-8f, step,
-                                                           w2bf);
+        k_mlp_train_step<<<nb, MLP_TRAIN_THREADS, sizeof(MlpTrainSmem), s>>>(params, w2bf, feat, target, nsamp, k * batch,
+                                                                             batch, partial, lossp);
+        k_mlp_adam<<<(MLP_NPARAM + 31) / 32, MLP_UPD_THREADS, 0, s>>>(
+            partial, nb, params, m, v, lr_t, 0.9f, 0.999f, 1e-8f, (float)(1.0 - std::pow(0.9, step)),
+            (float)(1.0 - std::pow(0.999, step)), w2bf);
       }
     }
     if (cudaGetLastError() != cudaSuccess) return -2;
@@ -628,7 +671,7 @@ struct Mlp {
       if (partial) cudaFree(partial);
       if (lossp) cudaFree(lossp);
       partial = lossp = nullptr;
-      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_NPARAM) || cudaMalloc(&lossp, sizeof(float) * n))
+      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_PSTRIDE) || cudaMalloc(&lossp, sizeof(float) * n))
         return -2;
       npart = nb;
     }
