@@ -42,6 +42,11 @@ struct Cfg {
   static constexpr int MINB_C2P32 = HELM_ ? 7 : 1;
 };
 
+// resident blocks of 128 threads per SM of the FP64 walks and rows, and faces per walk.  Walks at 4
+// (128 registers): a magnetised 128^3 step took 3.88 ms against 4.09 at 5 (96), 4.17 at 6 and more at 3
+// and 2, with little to choose between 8 and 16 faces; rows at 6 (80) 91 us against 97 at 5 for 96^3.
+constexpr int FACE64_WALK_MINB = 4, FACE64_ROW_MINB = 6, FACE64_K = 8;
+
 struct MlpSmall;
 
 struct Prm {
@@ -288,27 +293,16 @@ __device__ __forceinline__ void flatten_face(const R *const c[6], int iv, bool f
   }
 }
 
-// fa, fb: is_flattened of cells m-1 and m (always false without USE_SHOCK_FLATTENING)
+// Riemann part of a face along d from the edge states of its two sides in the cell frame (qL/qR
+// deviations under WB, transverse B in bL/bR, FASTEOS gammas with the equilibrium gamma_e added, or the
+// face temperature guess tface of Helmholtz without USE_FASTEOS): rotation, background, solver, WB fix
 template <class C>
-__device__ __forceinline__ void face_flux(const Prm &P, int d, int fi, int fj, int fk, const double *const w[6],
-                                          const double *const gmv[6], const double *const bc[6], double F[C::NV],
-                                          double Fb[3], double &rho_face_sum, bool fa = false, bool fb = false) {
+__device__ __forceinline__ void face_solve(const Prm &P, int d, int fi, int fj, int fk, double qL[C::NV], double qR[C::NV],
+                                           double bL[3], double bR[3], double gL[2], double gR[2], double tface,
+                                           bool flat, double F[C::NV], double Fb[3], double &rho_face_sum) {
   constexpr int NV = C::NV, IP = C::IP;
   const Geo &g = P.g;
-  double qL[NV], qR[NV];
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    rec_face<C>(w, iv, C::REC == REC_LIM5TH || iv >= C::IAS, qL[iv], qR[iv]);
-    if (C::SF) flatten_face<C>(w, iv, fa, fb, qL[iv], qR[iv]);
-  }
-  double bL[3] = {0, 0, 0}, bR[3] = {0, 0, 0};
   if (C::MHD) {
-#pragma unroll
-    for (int iv = 0; iv < C::DIM; ++iv) {
-      if (iv == d) continue;
-      rec_face<C>(bc, iv, C::REC == REC_LIM5TH, bL[iv], bR[iv]);
-      if (C::SF) flatten_face<C>(bc, iv, fa, fb, bL[iv], bR[iv]);
-    }
     double bn = P.bf[d][face_lin(g, d, fi, fj, fk)];
     bL[d] = bn;
     bR[d] = bn;
@@ -338,6 +332,62 @@ __device__ __forceinline__ void face_flux(const Prm &P, int d, int fi, int fj, i
     qL[IP] = qL[IP] + p_eq;
     qR[IP] = qR[IP] + p_eq;
   }
+  if (C::HELM && !C::FAST) {
+    // Helmholtz without USE_FASTEOS: helm_rhoP_given on each side of the face from the guess
+    // 1/2 (T(m-1) + T(m)) (source.F90:8488-8495, 15705-15720, 15777-15781); passes rho*e and c
+    double *gs[2] = {gL, gR};
+    const double *qs[2] = {qL, qR};
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const double *q = qs[side];
+      const double ye = q[C::IAS], abar = 1.0 / q[C::IAS + 1], zbar = ye * abar;
+      helm_side_eos_inl(P.helm, q[0], q[IP], abar, zbar, tface, gs[side][0], gs[side][1]);
+    }
+  }
+  const double gm = P.g.gm, mc = P.g.mach_cutoff;
+  if (C::MHD) {
+    riemann_mhd<double, C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, bL, bR, gL, gR, gm, mc, F, Fb, flat,
+                                                      g.all_mach != 0);
+  } else {
+    riemann_hydro<double, C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, gL, gR, gm, mc, F, flat,
+                                                        g.all_mach != 0);
+  }
+  // back to the lab frame
+  if (d == 1) {
+    double a = F[1], b = F[2]; F[1] = -b; F[2] = a;
+    if (C::MHD) { a = Fb[0]; b = Fb[1]; Fb[0] = -b; Fb[1] = a; }
+  } else if (C::DIM == 3 && d == 2) {
+    double a = F[1], b = F[2], c = F[3]; F[1] = b; F[2] = c; F[3] = a;
+    if (C::MHD) { a = Fb[0]; b = Fb[1]; c = Fb[2]; Fb[0] = b; Fb[1] = c; Fb[2] = a; }
+  }
+  rho_face_sum = qL[0] + qR[0];
+  // MHD: the EMF/sign are taken before the WB momentum fix (source.F90:8926-8959)
+  if (C::WB) F[1 + d] = F[1 + d] - __ldg(P.eq_p_f[d] + fbg);
+  if (C::ETOT) F[IP] = F[IP] + F[0] * __ldg(P.phi_f[d] + fbg);
+}
+
+// fa, fb: is_flattened of cells m-1 and m (always false without USE_SHOCK_FLATTENING)
+template <class C>
+__device__ __forceinline__ void face_flux(const Prm &P, int d, int fi, int fj, int fk, const double *const w[6],
+                                          const double *const gmv[6], const double *const bc[6], double F[C::NV],
+                                          double Fb[3], double &rho_face_sum, bool fa = false, bool fb = false) {
+  constexpr int NV = C::NV;
+  const Geo &g = P.g;
+  double qL[NV], qR[NV];
+#pragma unroll
+  for (int iv = 0; iv < NV; ++iv) {
+    rec_face<C>(w, iv, C::REC == REC_LIM5TH || iv >= C::IAS, qL[iv], qR[iv]);
+    if (C::SF) flatten_face<C>(w, iv, fa, fb, qL[iv], qR[iv]);
+  }
+  double bL[3] = {0, 0, 0}, bR[3] = {0, 0, 0};
+  if (C::MHD) {
+#pragma unroll
+    for (int iv = 0; iv < C::DIM; ++iv) {
+      if (iv == d) continue;
+      rec_face<C>(bc, iv, C::REC == REC_LIM5TH, bL[iv], bR[iv]);
+      if (C::SF) flatten_face<C>(bc, iv, fa, fb, bL[iv], bR[iv]);
+    }
+  }
   double gL[2] = {0, 0}, gR[2] = {0, 0};
   if (C::FAST) {
     // the x1 sweep flattens the gammas after the WB add-back, x2 and x3 before it
@@ -348,7 +398,7 @@ __device__ __forceinline__ void face_flux(const Prm &P, int d, int fi, int fj, i
       if (C::SF && !late) flatten_face<C>(gmv, iv, fa, fb, gL[iv], gR[iv]);
     }
     if (C::WB) {
-      double ge = __ldg(P.eq_ge_f[d] + fbg);
+      double ge = __ldg(P.eq_ge_f[d] + bg_face(g, d, fi, fj, fk));
       gL[0] = gL[0] + ge;
       gR[0] = gR[0] + ge;
       if (late) {
@@ -374,39 +424,9 @@ __device__ __forceinline__ void face_flux(const Prm &P, int d, int fi, int fj, i
         }
       }
     }
-  } else if (C::HELM) {
-    // Helmholtz without USE_FASTEOS: helm_rhoP_given on each side of the face from the guess
-    // 1/2 (T(m-1) + T(m)) (source.F90:8488-8495, 15705-15720, 15777-15781); passes rho*e and c
-    const double tface = 0.5 * (gmv[2][0] + gmv[3][0]);
-    double *gs[2] = {gL, gR};
-    const double *qs[2] = {qL, qR};
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const double *q = qs[side];
-      const double ye = q[C::IAS], abar = 1.0 / q[C::IAS + 1], zbar = ye * abar;
-      helm_side_eos_inl(P.helm, q[0], q[IP], abar, zbar, tface, gs[side][0], gs[side][1]);
-    }
   }
-  const double gm = P.g.gm, mc = P.g.mach_cutoff;
-  if (C::MHD) {
-    riemann_mhd<double, C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, bL, bR, gL, gR, gm, mc, F, Fb, C::SF && (fa || fb),
-                                                      g.all_mach != 0);
-  } else {
-    riemann_hydro<double, C::DIM, NV, C::EOSM, C::RIEM>(qL, qR, gL, gR, gm, mc, F, C::SF && (fa || fb),
-                                                        g.all_mach != 0);
-  }
-  // back to the lab frame
-  if (d == 1) {
-    double a = F[1], b = F[2]; F[1] = -b; F[2] = a;
-    if (C::MHD) { a = Fb[0]; b = Fb[1]; Fb[0] = -b; Fb[1] = a; }
-  } else if (C::DIM == 3 && d == 2) {
-    double a = F[1], b = F[2], c = F[3]; F[1] = b; F[2] = c; F[3] = a;
-    if (C::MHD) { a = Fb[0]; b = Fb[1]; c = Fb[2]; Fb[0] = b; Fb[1] = c; Fb[2] = a; }
-  }
-  rho_face_sum = qL[0] + qR[0];
-  // MHD: the EMF/sign are taken before the WB momentum fix (source.F90:8926-8959)
-  if (C::WB) F[1 + d] = F[1 + d] - __ldg(P.eq_p_f[d] + fbg);
-  if (C::ETOT) F[IP] = F[IP] + F[0] * __ldg(P.phi_f[d] + fbg);
+  const double tface = C::HELM && !C::FAST ? 0.5 * (gmv[2][0] + gmv[3][0]) : 0.0;
+  face_solve<C>(P, d, fi, fj, fk, qL, qR, bL, bR, gL, gR, tface, C::SF && (fa || fb), F, Fb, rho_face_sum);
 }
 
 // EMF components of a face flux and the mass-flux sign (source.F90:8926-8951)
@@ -582,6 +602,145 @@ __global__ void __launch_bounds__(128, C::MINB_FACE64) k_face(Prm P) {
 #pragma unroll
   for (int iv = 0; iv < NV; ++iv) P.dflux[d][(long long)iv * nf + f] = F[iv];
   if (C::MHD) store_face_emf<C>(P, d, f, Fb, F[0], rs, P.scal[2]);
+}
+
+// The same faces for LIM2ND with FASTEOS or the ideal gas, without forming every cell's slopes (a
+// division each) twice.  Values of a cell in the kernels below: the NV deviations, the cell B
+// components transverse to D, and the two gammas; comp(t) is the B component in transverse slot t.
+template <class C, int D>
+struct EdgeCell {
+  static constexpr int NBT = C::MHD ? C::DIM - 1 : 0, IG = C::NV + NBT, NR = IG + (C::FAST ? 2 : 0);
+  static __device__ __forceinline__ constexpr int comp(int t) { return t < D ? t : t + 1; }
+  // cell q along D of the row through (c[0], c[1], c[2]); ghosts are mapped
+  static __device__ __forceinline__ void load(const Prm &P, const int c[3], int q, double r[NR]) {
+    const Geo &g = P.g;
+    const int i = D == 0 ? q : c[0], j = D == 1 ? q : c[1], k = D == 2 ? q : c[2];
+    double w[C::NV], gm_[2] = {0.0, 0.0}, b[3] = {0.0, 0.0, 0.0};
+    if (q >= 0 && q < g.nx[D]) {
+      load_cell_at<C>(P, lin(g, i, j, k), j, w, gm_, b);
+    } else {
+      load_wdev<C>(P, i, j, k, w);
+      if (C::HELM) load_gdev<C>(P, i, j, k, gm_);
+      if (C::MHD) load_bcc<C>(P, i, j, k, b);
+    }
+#pragma unroll
+    for (int v = 0; v < C::NV; ++v) r[v] = w[v];
+#pragma unroll
+    for (int t = 0; t < NBT; ++t) r[C::NV + t] = b[comp(t)];
+    if (C::FAST) { r[IG] = gm_[0]; r[IG + 1] = gm_[1]; }
+  }
+  // slope of plm from the forward and backward differences
+  static __device__ __forceinline__ double half_slope(double sf, double sb) {
+    const double prod = sf * sb;
+    double slope = 0.0;
+    if (prod > 0.0) slope = prod / (sf + sb);
+    return 0.5 * slope;
+  }
+  // solve and store face q of the row from the high edges of cell q-1 and the low edges of cell q
+  static __device__ __forceinline__ void face(const Prm &P, const int c[3], int q, const double *hip, const double *lo,
+                                              double smax) {
+    const Geo &g = P.g;
+    const int i = D == 0 ? q : c[0], j = D == 1 ? q : c[1], k = D == 2 ? q : c[2];
+    double qL[C::NV], qR[C::NV], bL[3] = {0, 0, 0}, bR[3] = {0, 0, 0}, gL[2] = {0, 0}, gR[2] = {0, 0};
+#pragma unroll
+    for (int v = 0; v < C::NV; ++v) { qL[v] = hip[v]; qR[v] = lo[v]; }
+#pragma unroll
+    for (int t = 0; t < NBT; ++t) { bL[comp(t)] = hip[C::NV + t]; bR[comp(t)] = lo[C::NV + t]; }
+    if (C::FAST) {
+      gL[0] = hip[IG]; gL[1] = hip[IG + 1];
+      gR[0] = lo[IG]; gR[1] = lo[IG + 1];
+      if (C::WB) {
+        const double ge = __ldg(P.eq_ge_f[D] + bg_face(g, D, i, j, k));
+        gL[0] = gL[0] + ge;
+        gR[0] = gR[0] + ge;
+      }
+    }
+    double F[C::NV], Fb[3], rs;
+    face_solve<C>(P, D, i, j, k, qL, qR, bL, bR, gL, gR, 0.0, false, F, Fb, rs);
+    const long long nf = nfaces(g, D), f = face_lin(g, D, i, j, k);
+#pragma unroll
+    for (int v = 0; v < C::NV; ++v) P.dflux[D][(long long)v * nf + f] = F[v];
+    if (C::MHD) store_face_emf<C>(P, D, f, Fb, F[0], rs, smax);
+  }
+};
+
+// along x2 or x3: a thread walks K faces and carries the cell, its backward difference and the high
+// edges of the cell before (e0, e1: extents of the threads' index space in x1 and x2)
+template <class C, int D, int K>
+__global__ void __launch_bounds__(128, FACE64_WALK_MINB) k_face_walk(Prm P, FastDiv e0, FastDiv e1) {
+  if (!*P.active) return;
+  using E = EdgeCell<C, D>;
+  constexpr int NR = E::NR;
+  const Geo &g = P.g;
+  const int nd = g.nx[D] + 1, nch = (nd + K - 1) / K;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)e0.d * e1.d * (D == 2 ? nch : (C::DIM == 3 ? g.nx[2] : 1))) return;
+  int c[3];
+  unflatten3(t, e0, e1, c[0], c[1], c[2]);
+  const int q0 = c[D] * K, qend = min(q0 + K, nd);
+  c[D] = 0;
+  const double smax = P.scal[2];
+  double rc[NR], sb[NR], hip[NR];
+  {
+    double rm[NR], rp[NR];
+    E::load(P, c, q0 - 2, rm);
+    E::load(P, c, q0 - 1, rc);
+    E::load(P, c, q0, rp);
+#pragma unroll
+    for (int v = 0; v < NR; ++v) {
+      const double sf = rp[v] - rc[v];
+      hip[v] = rc[v] + E::half_slope(sf, rc[v] - rm[v]);
+      sb[v] = sf;
+      rc[v] = rp[v];
+    }
+  }
+#pragma unroll 1
+  for (int q = q0; q < qend; ++q) {
+    double rp[NR], lo[NR], hi[NR];
+    E::load(P, c, q + 1, rp);
+#pragma unroll
+    for (int v = 0; v < NR; ++v) {
+      const double sf = rp[v] - rc[v], h = E::half_slope(sf, sb[v]);
+      lo[v] = rc[v] - h;
+      hi[v] = rc[v] + h;
+      sb[v] = sf;
+      rc[v] = rp[v];
+    }
+    E::face(P, c, q, hip, lo, smax);
+#pragma unroll
+    for (int v = 0; v < NR; ++v) hip[v] = hi[v];
+  }
+}
+
+// along x1: a warp takes 32 neighbouring cells of a row and solves the 29 faces whose stencils they
+// hold, the neighbours' differences and edges coming by shuffle.  Any row length; 91 us for the x1
+// faces of a magnetised 96^3 box where one thread per face took 139 (every cell loaded four times and
+// its 11 slopes, a division each, formed twice).
+constexpr int ROW_FACES = 29;
+template <class C>
+__global__ void __launch_bounds__(128, FACE64_ROW_MINB) k_face_row(Prm P, FastDiv chunks) {
+  if (!*P.active) return;
+  using E = EdgeCell<C, 0>;
+  constexpr int NR = E::NR;
+  constexpr unsigned ALL = 0xffffffffu;
+  const Geo &g = P.g;
+  const unsigned w = (unsigned)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  int c[3], ch;
+  unflatten3(w, chunks, g.div1[0], ch, c[1], c[2]);
+  if (c[2] >= g.nx[2]) return;
+  c[0] = 0;
+  const int f = ch * ROW_FACES - 2 + (int)lane, i = min(f, g.nx[0] + 1);
+  double rc[NR], hip[NR], lo[NR];
+  E::load(P, c, i, rc);
+#pragma unroll
+  for (int v = 0; v < NR; ++v) {
+    const double sf = __shfl_down_sync(ALL, rc[v], 1) - rc[v];
+    const double h = E::half_slope(sf, __shfl_up_sync(ALL, sf, 1));
+    lo[v] = rc[v] - h;
+    hip[v] = __shfl_up_sync(ALL, rc[v] + h, 1);
+  }
+  if (lane < 2 || lane > 30 || f > g.nx[0]) return;
+  E::face(P, c, i, hip, lo, P.scal[2]);
 }
 
 // --------------------------------------------------------------------- MHD: corner EMFs

@@ -41,6 +41,12 @@ inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 // ----------------------------------------------------------------------------- runners
 template <class C>
 struct RunnerT : Runner {
+  // options whose edges the row and walk kernels form
+  static constexpr bool EDGES = C::REC == REC_LIM2ND && !C::SF && C::EOSM != EOS_GIVEN;
+  // A walk has an eighth of the threads: with fewer cells than this they do not fill the GPU (two
+  // waves of 4 blocks per SM).  Faces along x2 of a magnetised 96^3 box 109 us either way; a step of
+  // 128^3 4.28 ms with one thread per face, 3.85 walking; 2D grids lose 10% by walking.
+  static constexpr long long WALK64_CELLS = 1000000;
   void stage(const Prm &P, cudaStream_t s) override {
     const Geo &g = P.g;
     // each face once, then (MHD) corners and face B, then divergence + RK + cons->prim per cell
@@ -48,9 +54,23 @@ struct RunnerT : Runner {
       k_sf_mark<C><<<nblk(sf_mark_cells<C>(g), 256), 256, 0, s>>>(P);
       k_sf_flag<C><<<nblk(sf_flag_cells<C>(g), 256), 256, 0, s>>>(P);
     }
-    k_face<C, 0><<<nblk(nfaces_host(g, 0), 128), 128, 0, s>>>(P);
-    k_face<C, 1><<<nblk(nfaces_host(g, 1), 128), 128, 0, s>>>(P);
-    if constexpr (C::DIM == 3) k_face<C, 2><<<nblk(nfaces_host(g, 2), 128), 128, 0, s>>>(P);
+    if constexpr (EDGES) {
+      const unsigned chunks = nblk(g.nx[0] + 1, ROW_FACES);
+      k_face_row<C><<<nblk((long long)chunks * g.nx[1] * g.nx[2], 4), 128, 0, s>>>(P, FastDiv::by(chunks));
+    } else {
+      k_face<C, 0><<<nblk(nfaces_host(g, 0), 128), 128, 0, s>>>(P);
+    }
+    bool walked = false;
+    if constexpr (EDGES && C::DIM == 3)
+      if (g.N >= WALK64_CELLS) {
+        walk<1>(P, s);
+        walk<2>(P, s);
+        walked = true;
+      }
+    if (!walked) {
+      k_face<C, 1><<<nblk(nfaces_host(g, 1), 128), 128, 0, s>>>(P);
+      if constexpr (C::DIM == 3) k_face<C, 2><<<nblk(nfaces_host(g, 2), 128), 128, 0, s>>>(P);
+    }
     if constexpr (C::MHD) {
       auto ncor = [&](int a) {
         return (long long)(g.nx[0] + (a != 0)) * (g.nx[1] + (a != 1)) * (C::DIM == 3 ? g.nx[2] + (a != 2) : 1);
@@ -65,6 +85,14 @@ struct RunnerT : Runner {
       if constexpr (C::DIM == 3) k_bface<C, 2><<<nblk(nfaces_host(g, 2), 256), 256, 0, s>>>(P);
     }
     k_c2p<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
+  }
+  template <int D>
+  static void walk(const Prm &P, cudaStream_t s) {
+    const Geo &g = P.g;
+    unsigned e[3] = {(unsigned)g.nx[0], (unsigned)g.nx[1], (unsigned)g.nx[2]};
+    e[D] = nblk(g.nx[D] + 1, FACE64_K);
+    k_face_walk<C, D, FACE64_K><<<nblk((long long)e[0] * e[1] * e[2], 128), 128, 0, s>>>(P, FastDiv::by(e[0]),
+                                                                                         FastDiv::by(e[1]));
   }
   void dt(const Prm &P, cudaStream_t s) override { k_dt<C><<<nblk(P.g.N, 256), 256, 0, s>>>(P); }
   void init_thermo(const Prm &P, cudaStream_t s) override {

@@ -1041,7 +1041,6 @@ __global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : 
 // below its cell.  Bound by issue slots (70% of the cycles issue, 690 instructions a face); 67 us
 // for the x1 faces of a 128^3 MHD stage, where tiles staged in shared memory by bulk copies (766
 // instructions, two block barriers a tile) took 83 and a walk of 4 faces 1% more per stage.
-constexpr int ROW_FACES = 29;
 template <class C>
 __global__ void __launch_bounds__(128, ROW_MINB) k_face_split_row(Prm P, FastDiv chunks) {
   static_assert(C::REC == REC_LIM2ND, "the row kernel forms LIM2ND edges");
