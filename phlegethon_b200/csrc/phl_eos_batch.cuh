@@ -22,7 +22,7 @@
 namespace phl {
 
 // Resident blocks of 128 threads per SM the inversion kernels are compiled for: 3 (168 registers).
-// 2^22 samples on B200, learned guess 2.62 ms against 2.84 at 4 (128 registers, 850 B of spills) and
+// 2^22 samples on B200, learned guess (guess in the same kernel) 2.62 ms against 2.84 at 4 (128 registers, 850 B of spills) and
 // 2.91 at 2 (unbounded); 10^6 samples, bracket guess 0.49 ms against 0.55 and 0.55.  The 36
 // coefficients kept in shared memory between the evaluations of a solve ran 3 to 5% slower.
 constexpr int EOS_MINB = 3;
@@ -86,32 +86,39 @@ __device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, cons
   if (iters) iters[t] = used;
 }
 
-// Phase 1.  guess 0 / 2: warm or bracket guess and the full Newton.  guess 1: the learned guess
-// (computed per block of 128 samples on the tensor cores), judged by at most 3 reference
-// Newton iterations; a sample whose guess did not converge within them without a reset is
-// appended to `queue` (queue[0] = count, then index | judged iterations << 56) for phase 2, so
-// that the fallback runs in converged warps instead of stalling the accepted lanes.
-// LEARNED selects the learned-guess instantiation (guess 1); the other carries no tensor-core code.
+// Learned guess, phase 0: the network's temperature of every sample, left in T for phase 1.  A block
+// takes 128 samples: features (the cold energy from 12 table coefficients), one tensor-core product,
+// the FP32 layers as constant-bank operands.  A kernel of its own, so that the waits of the product and
+// the block's barriers are hidden by 8 blocks an SM instead of the 3 that the Newton's registers leave
+// (in one kernel, and with the FP32 layers read from memory, 2^22 samples took 2.62 ms, now 2.07).
+static __global__ void __launch_bounds__(128, 8) k_eos_guess(HelmTable h, const __grid_constant__ MlpSmall w,
+                                                             const __nv_bfloat16 *w2bf, long long n, const double *rho,
+                                                             const double *e, const double *abar, const double *zbar,
+                                                             double *T, unsigned long long *stat) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  MlpUmmaSmem &S = *reinterpret_cast<MlpUmmaSmem *>(sm);
+  mlp_cta_setup(w2bf, S);
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  float feat[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (t < n) mlp_features(rho[t], e[t] - mlp_cold_energy(h, rho[t], abar[t], zbar[t]), abar[t], zbar[t], feat);
+  bool ok = true, have = false;
+  const float lT = mlp_forward_tile(w, feat, S, 0u, ok, have, stat + STAT_TC_STALLED);
+  mlp_cta_teardown(S);
+  if (t < n) T[t] = fmin(fmax(exp10((double)lT), h.Tl * 1.000001), h.Th * 0.999999);
+}
+
+// Phase 1.  guess 0 / 2: warm or bracket guess and the full Newton.  LEARNED: the guess that phase 0
+// left in T, judged by at most 3 reference Newton iterations; a sample whose guess did not
+// converge within them without a reset is appended to `queue` (queue[0] = count, then
+// index | judged iterations << 56) for phase 2, so that the fallback runs in converged warps
+// instead of stalling the accepted lanes.
 template <bool LEARNED>
 __global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long long n, const double *rho, const double *e,
                                                     const double *abar, const double *zbar, double *T,
-                                                    double *p, double *cs, int *iters, int guess, MlpWeights mw,
+                                                    double *p, double *cs, int *iters, int guess,
                                                     unsigned long long *stat, unsigned long long *queue) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   EosStat st;
-  float lT_mlp = 0.0f;
-  double ecold = 0.0;
-  if constexpr (LEARNED) {
-    extern __shared__ __align__(128) unsigned char sm[];
-    MlpUmmaSmem &S = *reinterpret_cast<MlpUmmaSmem *>(sm);
-    float feat[4] = {0, 0, 0, 0};
-    if (t < n) {
-      ecold = mlp_cold_energy(h, rho[t], abar[t], zbar[t]);
-      st.v[6] = 1;
-      mlp_features(rho[t], e[t] - ecold, abar[t], zbar[t], feat);
-    }
-    lT_mlp = mlp_forward_cta(mw, feat, S, stat + STAT_TC_STALLED);
-  }
   bool reject = false;
   int judged = 0;
   if (t < n) {
@@ -122,7 +129,8 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long 
     int used = 0, clamped = 0;
     bool conv = false;
     if constexpr (LEARNED) {
-      Tg = fmin(fmax(exp10((double)lT_mlp), h.Tl * 1.000001), h.Th * 0.999999);
+      Tg = T[t];
+      st.v[6] = 1;  // the cold energy of phase 0
       used = helm_rhoe_newton(h, r, ht, ee, Tg, 3, clamped, &conv);
       st.v[3] = clamped;
       if (conv && clamped == 0) {
@@ -202,18 +210,17 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_fallback(HelmTable h, con
 // the learned guess only.  Returns 0 or a cudaError_t.
 inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *e,
                       const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters,
-                      int guess, MlpWeights mw, unsigned long long *stat, unsigned long long *queue, int nsm) {
+                      int guess, const Mlp &mlp, unsigned long long *stat, unsigned long long *queue, int nsm) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
   if (guess != PHL_GUESS_MLP) {
-    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat,
-                                                      nullptr);
+    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, stat, nullptr);
     return (int)cudaGetLastError();
   }
   const size_t sm = sizeof(MlpUmmaSmem);
-  cudaError_t err = cudaFuncSetAttribute(k_eos_invert<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (err == cudaSuccess) err = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
+  const cudaError_t err = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (err != cudaSuccess) return (int)err;
-  k_eos_invert<true><<<blocks, 128, sm, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, mw, stat, queue);
+  k_eos_guess<<<blocks, 128, sm, s>>>(h, mlp.small, mlp.w2bf, n, rho, e, abar, zbar, T, stat);
+  k_eos_invert<true><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, stat, queue);
   // enough resident blocks to cover every SM several times; the loop covers any queue length
   const unsigned fb = (unsigned)std::min<long long>((long long)nsm * 8, (long long)blocks);
   k_eos_fallback<<<fb, 128, 0, s>>>(h, queue, rho, e, abar, zbar, T, p, cs, iters, stat);
@@ -270,7 +277,7 @@ struct EosBatch {
       if (cudaMalloc(&queue, sizeof(unsigned long long) * (size_t)(n + 1)) != cudaSuccess) return -2;
       qcap = n + 1;
     }
-    if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp.weights(), stat, queue, sm_count()))
+    if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp, stat, queue, sm_count()))
       return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
     return 0;

@@ -351,76 +351,6 @@ struct MlpUmmaSmem {
 constexpr int MLP_UMMA_COLS = 64;         // FP32 accumulator columns (N)
 constexpr int MLP_UMMA_POLLS = 1 << 22;   // mbarrier polls before a stalled MMA is reported
 
-// All 128 threads of the block call this with uniform control flow.  A product that does not
-// complete within the poll limit increments *stalled (once per warp) and leaves layer 2 at zero.
-__device__ __forceinline__ float mlp_forward_cta(const MlpWeights &m, const float x[4], MlpUmmaSmem &S,
-                                                 unsigned long long *stalled) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 0) {
-    tmem_alloc(&S.tmem, MLP_UMMA_COLS);
-    tmem_relinquish();
-  }
-  if (tid == 0) mbar_init(&S.mbar, 1);
-  // W2 (row-major bf16 [out][in]) into the core-matrix layout, 16-byte pieces
-  for (int q = tid; q < MLP_H * 8; q += blockDim.x) {
-    const int n = q >> 3, c = q & 7;
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(m.w2bf + n * MLP_H) + c);
-    *reinterpret_cast<uint4 *>(S.B + umma_kmajor_offset(n, 8 * c)) = v;
-  }
-  // layer 1 (FP32) -> BF16 row tid of A
-  const float *W1 = m.w + MLP_OFF_W1, *b1 = m.w + MLP_OFF_B1;
-#pragma unroll 2
-  for (int c = 0; c < MLP_H / 8; ++c) {
-    __align__(16) __nv_bfloat16 v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int o = 8 * c + j;
-      float a = __ldg(b1 + o);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) a = fmaf(__ldg(W1 + o * 4 + k), x[k], a);
-      v[j] = __float2bfloat16(fmaxf(a, 0.0f));
-    }
-    *reinterpret_cast<uint4 *>(S.A + umma_kmajor_offset(tid, 8 * c)) = *reinterpret_cast<const uint4 *>(v);
-  }
-  fence_proxy_async_smem();
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tbase = S.tmem;
-  if (tid == 0) {
-    const uint32_t a0 = smem_u32(S.A), b0 = smem_u32(S.B);
-    constexpr uint32_t idesc = umma_idesc_bf16(128, MLP_H);
-#pragma unroll
-    for (int kk = 0; kk < MLP_H / 16; ++kk)
-      umma_bf16_f32(tbase, umma_desc(a0 + kk * UMMA_KSTEP_BYTES, UMMA_KCORE_BYTES, UMMA_ROW_GROUP_BYTES),
-                    umma_desc(b0 + kk * UMMA_KSTEP_BYTES, UMMA_KCORE_BYTES, UMMA_ROW_GROUP_BYTES), idesc, kk > 0);
-    umma_commit(&S.mbar);
-  }
-  // a phase seen complete by any lane is complete for the whole warp
-  const bool done = __any_sync(0xffffffffu, mbar_wait_bounded(&S.mbar, 0, MLP_UMMA_POLLS));
-  tc_fence_after_sync();
-  float out = __ldg(m.w + MLP_OFF_B3);
-  if (done) {
-    const float *W3 = m.w + MLP_OFF_W3, *b2 = m.w + MLP_OFF_B2;
-    const uint32_t row_addr = tbase + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-    for (int c = 0; c < MLP_H / 16; ++c) {
-      float z[16];
-      tmem_ld16(row_addr + 16 * c, z);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) out = fmaf(__ldg(W3 + 16 * c + q), fmaxf(z[q] + __ldg(b2 + 16 * c + q), 0.0f), out);
-    }
-  } else {
-    if (lane == 0 && stalled) atomicAdd(stalled, 1ull);
-    // give the product a second bounded chance to land before its columns are released
-    mbar_wait_bounded(&S.mbar, 0, MLP_UMMA_POLLS);
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, MLP_UMMA_COLS);
-  return mlp_prior(x) + out * MLP_OUT_SCALE + MLP_OUT_SHIFT;
-}
-
 // The FP32 parameters of layers 1 and 3 by value: passed as a __grid_constant__ kernel argument
 // they sit in the constant bank, and the fully unrolled layer arithmetic takes them as operands
 // instead of loading them.
@@ -437,11 +367,10 @@ inline void mlp_small_from_params(const float *p, MlpSmall &w) {
   w.b3 = p[MLP_OFF_B3];
 }
 
-// mlp_forward_cta in three pieces, with the FP32 layers taken from an MlpSmall: the block sets up
-// its tensor-memory columns, mbarrier and W2 in shared memory once (mlp_cta_setup), runs tiles of
-// 128 samples (mlp_forward_tile: all 128 threads, uniform control flow; tile n of the block waits
-// on the mbarrier phase of parity n & 1) and releases the columns (mlp_cta_teardown).  The step's
-// guess kernel (k_mlp_guess) runs one tile per block.
+// A block of 128 threads sets up its tensor-memory columns, mbarrier and W2 in shared memory once
+// (mlp_cta_setup), runs tiles of 128 samples (mlp_forward_tile: all threads, uniform control flow;
+// tile n of the block waits on the mbarrier phase of parity n & 1) and releases the columns
+// (mlp_cta_teardown).  The guess and inference kernels run one tile per block.
 __device__ __forceinline__ void mlp_cta_setup(const __nv_bfloat16 *w2bf, MlpUmmaSmem &S) {
   const int tid = threadIdx.x;
   if ((tid >> 5) == 0) {
@@ -533,19 +462,24 @@ __device__ __forceinline__ void mlp_cta_teardown(MlpUmmaSmem &S) {
 }
 
 // per-sample inference kernel (features n x 4 -> log10 T), 128 threads per block
-static __global__ void __launch_bounds__(128) k_mlp_infer(MlpWeights m, long long n, const float *feat, float *out,
+static __global__ void __launch_bounds__(128) k_mlp_infer(const __grid_constant__ MlpSmall w, const __nv_bfloat16 *w2bf,
+                                                   long long n, const float *feat, float *out,
                                                    unsigned long long *stalled) {
   __shared__ MlpUmmaSmem S;
+  mlp_cta_setup(w2bf, S);
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float x[4] = {0, 0, 0, 0};
   if (t < n)
     for (int k = 0; k < 4; ++k) x[k] = feat[t * 4 + k];
-  float y = mlp_forward_cta(m, x, S, stalled);
+  bool ok = true, have = false;
+  const float y = mlp_forward_tile(w, x, S, 0u, ok, have, stalled);
+  mlp_cta_teardown(S);
   if (t < n) out[t] = y;
 }
 
 struct Mlp {
   bool ready = false;
+  MlpSmall small;  // host copy of the FP32 layers of params, an argument of the inference kernels
   MlpRange range;
   float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *partial = nullptr, *lossp = nullptr;
   float *feat = nullptr, *target = nullptr;
@@ -575,6 +509,7 @@ struct Mlp {
     if (cudaMemcpyAsync(params, h, sizeof(float) * MLP_NPARAM, cudaMemcpyHostToDevice, s) != cudaSuccess) return -2;
     k_mlp_to_bf16<<<(MLP_H * MLP_H + 255) / 256, 256, 0, s>>>(params, w2bf);
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
+    mlp_small_from_params(h, small);
     ready = true;
     return 0;
   }
@@ -652,7 +587,9 @@ struct Mlp {
     if (final_loss) {
       if (gradient(s, 0, batch, final_loss)) return -2;
     }
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
+    float host[MLP_NPARAM];
+    if (get(s, host)) return -2;  // waits for the stream
+    mlp_small_from_params(host, small);
     ready = true;
     return 0;
   }
@@ -689,7 +626,7 @@ struct Mlp {
   int infer(cudaStream_t s, long long n, const float *f, float *o, unsigned long long *stalled) {
     if (!ready) return -4;
     if (n == 0) return 0;
-    k_mlp_infer<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(weights(), n, f, o, stalled);
+    k_mlp_infer<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(small, w2bf, n, f, o, stalled);
     if (cudaGetLastError() != cudaSuccess) return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
     return 0;

@@ -260,9 +260,6 @@ struct phl_ctx {
   double *htab = nullptr, *hdpd = nullptr, *hrho = nullptr, *hT = nullptr, *hirho = nullptr, *hiT = nullptr;
   HelmTable helm{};
   bool table_loaded = false, uploaded = false, bg_uploaded = false;
-  // host copy of the network's FP32 layers 1 and 3 (argument of the learned cons->prim kernel)
-  MlpSmall mlp_small{};
-  bool mlp_small_ok = false;
   // staging
   double *stage_buf = nullptr;
   size_t stage_bytes = 0;
@@ -387,7 +384,7 @@ struct phl_ctx {
       MlpWeights mw = eos.mlp.weights();
       P.mlp_w = mw.w;
       P.mlp_w2bf = mw.w2bf;
-      P.mlp_small = mlp_small_ok ? &mlp_small : nullptr;
+      P.mlp_small = &eos.mlp.small;
       P.rescue_q = cfg.eos_guess == PHL_GUESS_MLP_RESCUE ? rescue_q : nullptr;
     }
     P.sf_flag = sf_flag;
@@ -1407,7 +1404,7 @@ extern "C" int phl_eos_invert_batch_noalloc(phl_ctx *ctx, long long n, const dou
   CK(cudaMemcpyAsync(d_z, zbar, b, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_T, T_inout, b, cudaMemcpyHostToDevice, s));
   CK((cudaError_t)eos_launch(ctx->helm, s, n, d_rho, d_e, d_a, d_z, d_T, p ? d_p : nullptr, cs ? d_c : nullptr,
-                             iters ? ibuf : nullptr, guess, ctx->eos.mlp.weights(), ctx->stat, queue,
+                             iters ? ibuf : nullptr, guess, ctx->eos.mlp, ctx->stat, queue,
                              ctx->eos.sm_count()));
   CK(cudaMemcpyAsync(T_inout, d_T, b, cudaMemcpyDeviceToHost, s));
   if (p) CK(cudaMemcpyAsync(p, d_p, b, cudaMemcpyDeviceToHost, s));
@@ -1426,15 +1423,6 @@ int phl_mlp_train(phl_ctx *ctx, long long n, unsigned long long seed, int epochs
   CK(cudaSetDevice(ctx->cfg.device));
   int rc = ctx->eos.mlp_train(ctx->helm, ctx->stream, n, seed, epochs, batch, lr, final_loss);
   ctx->drop_graphs();  // step graphs bake the network's parameters into their kernels
-  ctx->mlp_small_ok = false;
-  if (rc == 0) {
-    std::vector<float> p(MLP_NPARAM);
-    rc = ctx->eos.mlp_get(ctx->stream, p.data());
-    if (rc == 0) {
-      mlp_small_from_params(p.data(), ctx->mlp_small);
-      ctx->mlp_small_ok = true;
-    }
-  }
   return rc;
 }
 
@@ -1477,8 +1465,6 @@ int phl_mlp_set_params(phl_ctx *ctx, const float *params) {
   CK(cudaSetDevice(ctx->cfg.device));
   int rc = ctx->eos.mlp_set(ctx->stream, params);
   ctx->drop_graphs();
-  ctx->mlp_small_ok = rc == 0;
-  if (rc == 0) mlp_small_from_params(params, ctx->mlp_small);
   return rc;
 }
 
