@@ -265,6 +265,18 @@ struct phl_ctx {
   size_t stage_bytes = 0;
   // graphs: one per parity of the W ping-pong
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  // the same of hydro_step alone, captured once a caller has made HYDRO_GRAPH_AFTER calls (a graph
+  // costs about as much to make as it saves in that many)
+  static constexpr int HYDRO_GRAPH_AFTER = 8;
+  cudaGraphExec_t hydro_graph[2] = {nullptr, nullptr};
+  int hydro_calls = 0;
+  // page-locked mailbox of the calls that return scalars: with pageable memory every 8-byte copy is a
+  // wait of its own.  A call waits for its copies before it returns, so the next one may reuse it.
+  struct Mailbox {
+    double scal[4];      // time, dt, smax; [3] tmax on its way to the device
+    long long step[2];   // steps before and after the call
+  };
+  Mailbox *mail = nullptr;
   // asynchronous host-state pipeline (phl_run_steps_host_async): copy streams, staging images
   // of the dynamic host arrays, and the events that order one call's uploads after the previous
   // call's downloads chunk by chunk
@@ -289,8 +301,8 @@ struct phl_ctx {
   std::vector<void *> allocs;
 
   ~phl_ctx() {
-    for (int p = 0; p < 2; ++p)
-      if (graph[p]) cudaGraphExecDestroy(graph[p]);
+    drop_graphs();
+    if (mail) cudaFreeHost(mail);
     eos.release();
     for (cudaEvent_t e : ev_chunk_out) cudaEventDestroy(e);
     for (int q = 0; q < HOST_SLOTS; ++q) {
@@ -440,8 +452,10 @@ struct phl_ctx {
     runner->split_to_prim(P, stream);
   }
   void drop_graphs() {
-    for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < 2; ++p) {
       if (graph[p]) { cudaGraphExecDestroy(graph[p]); graph[p] = nullptr; }
+      if (hydro_graph[p]) { cudaGraphExecDestroy(hydro_graph[p]); hydro_graph[p] = nullptr; }
+    }
   }
   // hydro_step: all RK stages starting from W[cur]
   void launch_stages() {
@@ -449,23 +463,48 @@ struct phl_ctx {
   }
   // one time_loop iteration as a CUDA graph (captured on first use per W parity): tmax clamp,
   // the RK stages, time += dt, the next dt
-  int launch_step_graph() {
-    int p = cur;
-    if (!graph[p]) {
+  template <class Body>
+  int run_graph(cudaGraphExec_t &g, Body body) {
+    if (!g) {
       cudaGraph_t gph;
       CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      k_pre_step<<<1, 1, 0, stream>>>(scal, active, smax_bits, step, (long long)1 << 62);
-      launch_stages();
-      k_post_step<<<1, 1, 0, stream>>>(scal, active, smax_bits, step, cfg.cfl);
+      body();
       CK(cudaStreamEndCapture(stream, &gph));
-      cudaError_t e = cudaGraphInstantiate(&graph[p], gph, 0);
+      cudaError_t e = cudaGraphInstantiate(&g, gph, 0);
       cudaGraphDestroy(gph);
       if (e != cudaSuccess) {
+        g = nullptr;
         g_last_error = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
         return PHL_E_CUDA;
       }
     }
-    CK(cudaGraphLaunch(graph[p], stream));
+    CK(cudaGraphLaunch(g, stream));
+    return PHL_OK;
+  }
+  int launch_step_graph() {
+    if (int rc = run_graph(graph[cur], [&] {
+          k_pre_step<<<1, 1, 0, stream>>>(scal, active, smax_bits, step, (long long)1 << 62);
+          launch_stages();
+          k_post_step<<<1, 1, 0, stream>>>(scal, active, smax_bits, step, cfg.cfl);
+        }))
+      return rc;
+    cur = (cur + cfg.rk_stages) & 1;
+    return PHL_OK;
+  }
+  // hydro_step with the current dt: launched kernel by kernel at first, as a graph for callers that
+  // keep stepping this way
+  int launch_hydro_step() {
+    auto body = [&] {
+      k_set_active<<<1, 1, 0, stream>>>(active, smax_bits);
+      launch_stages();
+    };
+    if (hydro_calls < HYDRO_GRAPH_AFTER) {
+      ++hydro_calls;
+      body();
+      CK(cudaGetLastError());
+    } else if (int rc = run_graph(hydro_graph[cur], body)) {
+      return rc;
+    }
     cur = (cur + cfg.rk_stages) & 1;
     return PHL_OK;
   }
@@ -598,6 +637,7 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
   }
   if (!c->runner) return PHL_E_UNSUPPORTED;
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  CK(cudaMallocHost(&c->mail, sizeof(phl_ctx::Mailbox)));
   Geo &g = c->geo;
   memset(&g, 0, sizeof(g));
   g.sdims = cfg->sdims;
@@ -913,9 +953,7 @@ int phl_upload_state(phl_ctx *ctx, const phl_fields *f) {
   CK(cudaStreamSynchronize(s));
   if (strat && f->eq_prim_cc) {
     ctx->bg_uploaded = true;
-    // graphs bake the background layout into their kernel arguments
-    for (int p = 0; p < 2; ++p)
-      if (ctx->graph[p]) { cudaGraphExecDestroy(ctx->graph[p]); ctx->graph[p] = nullptr; }
+    ctx->drop_graphs();  // they bake the background layout into their kernel arguments
   }
   ctx->uploaded = true;
   return PHL_OK;
@@ -1013,8 +1051,8 @@ int phl_compute_hyperbolic_dt(phl_ctx *ctx, double *dt, double *smax) {
   ctx->thermo()->dt(P, ctx->stream);
   k_finish_dt<<<1, 1, 0, ctx->stream>>>(ctx->scal, ctx->smax_bits, ctx->cfg.cfl);
   CK(cudaGetLastError());
-  double sc[3];
-  CK(cudaMemcpyAsync(sc, ctx->scal, sizeof(sc), cudaMemcpyDeviceToHost, ctx->stream));
+  const double *sc = ctx->mail->scal;
+  CK(cudaMemcpyAsync(ctx->mail->scal, ctx->scal, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (dt) *dt = sc[1];
   if (smax) *smax = sc[2];
@@ -1025,10 +1063,7 @@ int phl_hydro_step(phl_ctx *ctx) {
   int rc = ready(ctx, true);
   if (rc) return rc;
   CK(cudaSetDevice(ctx->cfg.device));
-  k_set_active<<<1, 1, 0, ctx->stream>>>(ctx->active, ctx->smax_bits);
-  ctx->launch_stages();
-  CK(cudaGetLastError());
-  ctx->cur = (ctx->cur + ctx->cfg.rk_stages) & 1;
+  if ((rc = ctx->launch_hydro_step())) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   return PHL_OK;
 }
@@ -1060,20 +1095,20 @@ int phl_run_steps(phl_ctx *ctx, int nsteps, double tmax, int *steps_done, double
   if (nsteps < 0) return PHL_E_INVALID;
   CK(cudaSetDevice(ctx->cfg.device));
   cudaStream_t s = ctx->stream;
-  long long step0 = 0;
-  CK(cudaMemcpyAsync(&step0, ctx->step, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(ctx->scal + 3, &tmax, sizeof(double), cudaMemcpyHostToDevice, s));
-  CK(cudaStreamSynchronize(s));
+  phl_ctx::Mailbox &m = *ctx->mail;
+  m.scal[3] = tmax;
+  CK(cudaMemcpyAsync(&m.step[0], ctx->step, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(ctx->scal + 3, &m.scal[3], sizeof(double), cudaMemcpyHostToDevice, s));
   // graphs run with no device-side step limit: the host launches exactly nsteps of them and
   // the device stops by itself once time >= tmax.
   for (int n = 0; n < nsteps; ++n)
     if ((rc = ctx->launch_step_graph())) return rc;
-  long long step1 = 0;
-  double t = 0;
-  CK(cudaMemcpyAsync(&step1, ctx->step, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&t, ctx->scal, sizeof(double), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&m.step[1], ctx->step, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(m.scal, ctx->scal, sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   CK(cudaGetLastError());
+  const long long step0 = m.step[0], step1 = m.step[1];
+  const double t = m.scal[0];
   // steps skipped by the device (time >= tmax) did not swap the W buffers: recover parity
   long long skipped = (long long)nsteps - (step1 - step0);
   if (skipped > 0 && (ctx->cfg.rk_stages & 1)) ctx->cur = (int)((ctx->cur + skipped) & 1);
