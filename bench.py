@@ -102,7 +102,9 @@ def step_launches(cfg, form, guess="warm"):
     stage)."""
     s = cfg.rk_stages
     if form != "fp32_split":
-        return stage_kernels(cfg, form, guess)
+        if cfg.mhd:
+            return "k_face + k_corner + k_bface + k_c2p (one MHD stage)", s * (cfg.sdims + 3) + 2
+        return "k_face + k_c2p (FP64)", s * (cfg.sdims + 1) + 2
     if cfg.mhd:
         # faces per direction, corners, face B, cons->prim
         per = cfg.sdims + 3 + (1 if guess == "mlp_rescue" else 0)

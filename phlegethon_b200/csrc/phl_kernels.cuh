@@ -35,7 +35,8 @@ struct Cfg {
   // run faster with more warps resident, even with a few registers spilled to L1 (measured on
   // B200 for the Helmholtz boxes); the variants whose inlined EoS or fifth-order stencil would
   // spill kilobytes keep the compiler's own budget (1).
-  static constexpr int MINB_FACE64 = (EOSM == EOS_GIVEN || REC_ == REC_LIM5TH) ? 1 : 6;
+  // (LIM5TH at 4, 128 registers: 333^2 Orszag-Tang, 5 steps, 614 us against 640 at the compiler's 142)
+  static constexpr int MINB_FACE64 = EOSM == EOS_GIVEN ? 1 : (REC_ == REC_LIM5TH ? 4 : 6);
   static constexpr int MINB_C2P64 = HELM_ ? 4 : 1;
   static constexpr int MINB_FACE32 = (EOSM == EOS_GIVEN || REC_ == REC_LIM5TH) ? 1 : 8;
   // split cons->prim: 7 (72 registers), 256^3 MHD step 12.2 ms against 12.4 at 6 and 12.5 at 8
@@ -793,33 +794,49 @@ __device__ __forceinline__ double emf_cell(const Prm &P, int a, int i, int j, in
   return v[0] * b[2] - v[2] * b[0];
 }
 
-// corner EMF along axis a (source.F90:11966-12206); one thread per corner
-template <class C, int A>
-__global__ void __launch_bounds__(256) k_corner(Prm P) {
-  constexpr int a = A;  // one instantiation per corner axis
-  if (!*P.active) return;
+__device__ __forceinline__ long long cor_lin(const Geo &g, int a, int i, int j, int k) {
+  return lin3(g.nx[0] + (a != 0), g.nx[1] + (a != 1), i, j, k);
+}
+
+// corner EMF along axis A (source.F90:11966-12206) at node (c[0], c[1], c[2]); INTERIOR: all four faces
+// and cells lie inside the domain (linear indices, no wrap or mirror)
+template <class C, int A, bool INTERIOR>
+__device__ __forceinline__ double corner_emf(const Prm &P, const int c[3]) {
+  constexpr int a = A, pa = A == 2 ? 0 : (A == 0 ? 1 : 2), qa = A == 2 ? 1 : (A == 0 ? 2 : 0);
   const Geo &g = P.g;
-  int pa, qa;
-  if (a == 2) { pa = 0; qa = 1; } else if (a == 0) { pa = 1; qa = 2; } else { pa = 2; qa = 0; }
-  int n0 = g.nx[0] + (a != 0), n1 = g.nx[1] + (a != 1), n2 = C::DIM == 3 ? g.nx[2] + (a != 2) : 1;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n0 * n1 * n2) return;
-  int c[3];
-  unflatten3(t, g.div0[a != 0], g.div1[a != 1], c[0], c[1], c[2]);
   int cqm[3] = {c[0], c[1], c[2]}; cqm[qa] -= 1;
   int cpm[3] = {c[0], c[1], c[2]}; cpm[pa] -= 1;
   int cpq[3] = {c[0], c[1], c[2]}; cpq[pa] -= 1; cpq[qa] -= 1;
-  double emf_N, emf_E, emf_S, emf_W, s_dummy;
-  double sgS, sgN, sgW, sgE;
-  face_emf_at<C>(P, pa, a, c[0], c[1], c[2], emf_N, sgN);
-  face_emf_at<C>(P, qa, a, c[0], c[1], c[2], emf_E, sgE);
-  face_emf_at<C>(P, pa, a, cqm[0], cqm[1], cqm[2], emf_S, sgS);
-  face_emf_at<C>(P, qa, a, cpm[0], cpm[1], cpm[2], emf_W, sgW);
-  (void)s_dummy;
-  double emf_SW = emf_cell<C>(P, a, cpq[0], cpq[1], cpq[2]);
-  double emf_NW = emf_cell<C>(P, a, cpm[0], cpm[1], cpm[2]);
-  double emf_NE = emf_cell<C>(P, a, c[0], c[1], c[2]);
-  double emf_SE = emf_cell<C>(P, a, cqm[0], cqm[1], cqm[2]);
+  double emf_N, emf_E, emf_S, emf_W, sgS, sgN, sgW, sgE, emf_SW, emf_NW, emf_NE, emf_SE;
+  if (INTERIOR) {
+    const double *ep = P.emf[pa] + (long long)a * nfaces(g, pa), *eq = P.emf[qa] + (long long)a * nfaces(g, qa);
+    const long long fN = face_lin(g, pa, c[0], c[1], c[2]), fS = face_lin(g, pa, cqm[0], cqm[1], cqm[2]);
+    const long long fE = face_lin(g, qa, c[0], c[1], c[2]), fW = face_lin(g, qa, cpm[0], cpm[1], cpm[2]);
+    emf_N = __ldg(ep + fN); sgN = __ldg(P.sgnf[pa] + fN);
+    emf_S = __ldg(ep + fS); sgS = __ldg(P.sgnf[pa] + fS);
+    emf_E = __ldg(eq + fE); sgE = __ldg(P.sgnf[qa] + fE);
+    emf_W = __ldg(eq + fW); sgW = __ldg(P.sgnf[qa] + fW);
+    // component a of -v x B: v_q B_p - v_p B_q, in the reference's order of the two products
+    auto cell = [&](const int n[3]) {
+      const long long i = lin(g, n[0], n[1], n[2]);
+      const double vp = __ldg(P.Win + (1 + pa) * g.N + i), vq = __ldg(P.Win + (1 + qa) * g.N + i);
+      const double bp = P.bcc_in[pa * g.N + i], bq = P.bcc_in[qa * g.N + i];
+      return a == 2 ? -vp * bq + vq * bp : vq * bp - vp * bq;
+    };
+    emf_SW = cell(cpq);
+    emf_NW = cell(cpm);
+    emf_NE = cell(c);
+    emf_SE = cell(cqm);
+  } else {
+    face_emf_at<C>(P, pa, a, c[0], c[1], c[2], emf_N, sgN);
+    face_emf_at<C>(P, qa, a, c[0], c[1], c[2], emf_E, sgE);
+    face_emf_at<C>(P, pa, a, cqm[0], cqm[1], cqm[2], emf_S, sgS);
+    face_emf_at<C>(P, qa, a, cpm[0], cpm[1], cpm[2], emf_W, sgW);
+    emf_SW = emf_cell<C>(P, a, cpq[0], cpq[1], cpq[2]);
+    emf_NW = emf_cell<C>(P, a, cpm[0], cpm[1], cpm[2]);
+    emf_NE = emf_cell<C>(P, a, c[0], c[1], c[2]);
+    emf_SE = emf_cell<C>(P, a, cqm[0], cqm[1], cqm[2]);
+  }
   double sgn = sgS;
   double demf_S = 0.5 * (1.0 + sgn) * (emf_W - emf_SW) + 0.5 * (1.0 - sgn) * (emf_E - emf_SE);
   sgn = sgN;
@@ -828,44 +845,99 @@ __global__ void __launch_bounds__(256) k_corner(Prm P) {
   double demf_W = 0.5 * (1.0 + sgn) * (emf_S - emf_SW) + 0.5 * (1.0 - sgn) * (emf_N - emf_NW);
   sgn = sgE;
   double demf_E = 0.5 * (1.0 + sgn) * (emf_SE - emf_S) + 0.5 * (1.0 - sgn) * (emf_NE - emf_N);
-  P.cor[a][t] = 0.25 * (emf_S + emf_W + emf_N + emf_E + demf_S - demf_N + demf_W - demf_E);
+  return 0.25 * (emf_S + emf_W + emf_N + emf_E + demf_S - demf_N + demf_W - demf_E);
 }
 
-__device__ __forceinline__ long long cor_lin(const Geo &g, int a, int i, int j, int k) {
-  return lin3(g.nx[0] + (a != 0), g.nx[1] + (a != 1), i, j, k);
+// Nodes on the domain's faces, in the order of a linear index t: the k = 0 and k = nx[2] planes (3D), then
+// per inner plane the border of the (nx[0] + 1) x (nx[1] + 1) rectangle; false past the last one
+template <class C>
+__device__ __forceinline__ bool rim_node(const Geo &g, long long t, int c[3]) {
+  const int n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2], rim = 2 * (n0 + n1);
+  const long long ncap = C::DIM == 3 ? 2ll * (n0 + 1) * (n1 + 1) : 0;
+  if (t < ncap) {
+    unflatten3(t, g.div0[1], g.div1[1], c[0], c[1], c[2]);
+    c[2] = c[2] ? n2 : 0;
+    return true;
+  }
+  t -= ncap;
+  if (t >= (long long)rim * (C::DIM == 3 ? n2 - 1 : 1)) return false;
+  const int m = (int)(t % rim);
+  c[2] = C::DIM == 3 ? (int)(t / rim) + 1 : 0;
+  if (m < n0 + 1) { c[0] = m; c[1] = 0; }                                           // x2 = 0 row
+  else if (m < 2 * (n0 + 1)) { c[0] = m - (n0 + 1); c[1] = n1; }                    // x2 = nx[1] row
+  else if (m < 2 * (n0 + 1) + (n1 - 1)) { c[0] = 0; c[1] = m - 2 * (n0 + 1) + 1; }  // x1 = 0 column
+  else { c[0] = n0; c[1] = m - 2 * (n0 + 1) - (n1 - 1) + 1; }                       // x1 = nx[0] column
+  return true;
 }
 
-// face-B update (source.F90:12208-12437); one thread per face of direction d
-template <class C, int D>
-__global__ void __launch_bounds__(256) k_bface(Prm P) {
-  constexpr int d = D;
+// The corners of every axis whose lower end is a node, one thread per node: interior nodes (1 <= index <
+// nx everywhere; e0 and e1 are nx - 1 of x1 and x2) in the first nin_blocks blocks, by linear index; the
+// nodes on the domain's faces in the others, mapping their ghosts.  Bound by its loads and, with three
+// launches of mapped indices (26 us each for 96^3), by integer work; with the one face-B launch a
+// magnetised 128^3 step went from 3.82 to 3.65 ms.
+template <class C>
+__global__ void __launch_bounds__(256) k_corner(Prm P, unsigned nin_blocks, FastDiv e0, FastDiv e1) {
   if (!*P.active) return;
   const Geo &g = P.g;
-  long long nf = nfaces(g, d);
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf) return;
+  int c[3];
+  if (blockIdx.x < nin_blocks) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)e0.d * e1.d * (C::DIM == 3 ? g.nx[2] - 1 : 1)) return;
+    unflatten3(t, e0, e1, c[0], c[1], c[2]);
+    c[0] += 1;
+    c[1] += 1;
+    if (C::DIM == 3) {
+      c[2] += 1;
+      P.cor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf<C, 0, true>(P, c);
+      P.cor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf<C, 1, true>(P, c);
+    }
+    P.cor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf<C, 2, true>(P, c);
+    return;
+  }
+  if (!rim_node<C>(g, (long long)(blockIdx.x - nin_blocks) * blockDim.x + threadIdx.x, c)) return;
+  if (C::DIM == 3) {
+    if (c[0] < g.nx[0]) P.cor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf<C, 0, false>(P, c);
+    if (c[1] < g.nx[1]) P.cor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf<C, 1, false>(P, c);
+    if (c[2] >= g.nx[2]) return;
+  }
+  P.cor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf<C, 2, false>(P, c);
+}
+
+// face-B update (source.F90:12208-12437); one thread per node updates the low faces of cell (i, j, k)
+template <class C>
+__global__ void __launch_bounds__(256) k_bface(Prm P) {
+  if (!*P.active) return;
+  const Geo &g = P.g;
+  const int n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)(n0 + 1) * (n1 + 1) * (C::DIM == 3 ? n2 + 1 : 1)) return;
   int i, j, k;
-  unflatten3(t, g.div0[d == 0], g.div1[d == 1], i, j, k);
+  unflatten3(t, g.div0[1], g.div1[1], i, j, k);
+  const bool in0 = i < n0, in1 = j < n1, in2 = C::DIM == 2 || k < n2;
   const double dt = P.scal[1];
   const double a1 = P.a1, a2 = P.a2, a3 = P.c3 * dt;
-  const double *E1 = P.cor[0], *E2 = P.cor[1], *E3 = P.cor[2];
-  double tmp;
-  if (d == 0) {
-    if (C::DIM == 2) tmp = (E3[cor_lin(g, 2, i, j + 1, k)] - E3[cor_lin(g, 2, i, j, k)]) * g.inv_dx[1];
-    else tmp = -(E2[cor_lin(g, 1, i, j, k + 1)] - E2[cor_lin(g, 1, i, j, k)]) * g.inv_dx[2] +
-               (E3[cor_lin(g, 2, i, j + 1, k)] - E3[cor_lin(g, 2, i, j, k)]) * g.inv_dx[1];
-  } else if (d == 1) {
-    if (C::DIM == 2) tmp = (E3[cor_lin(g, 2, i, j, k)] - E3[cor_lin(g, 2, i + 1, j, k)]) * g.inv_dx[0];
-    else tmp = (E1[cor_lin(g, 0, i, j, k + 1)] - E1[cor_lin(g, 0, i, j, k)]) * g.inv_dx[2] +
-               (E3[cor_lin(g, 2, i, j, k)] - E3[cor_lin(g, 2, i + 1, j, k)]) * g.inv_dx[0];
-  } else {
-    tmp = (E2[cor_lin(g, 1, i + 1, j, k)] - E2[cor_lin(g, 1, i, j, k)]) * g.inv_dx[0] -
-          (E1[cor_lin(g, 0, i, j + 1, k)] - E1[cor_lin(g, 0, i, j, k)]) * g.inv_dx[1];
+  auto e = [&](int a, long long q) { return __ldg(P.cor[a] + q); };
+  const long long q2 = cor_lin(g, 2, i, j, k), q2y = n0 + 1;
+  auto update = [&](int d, double tmp) {
+    const long long f = face_lin(g, d, i, j, k);
+    double b = P.bf[d][f];
+    double b0;
+    if (P.first_stage) { b0 = b; P.b0f[d][f] = b; } else { b0 = P.b0f[d][f]; }
+    P.bf[d][f] = a1 * b0 + a2 * b + a3 * tmp;
+  };
+  if (C::DIM == 2) {
+    const double E3 = e(2, q2);
+    if (in1) update(0, (e(2, q2 + q2y) - E3) * g.inv_dx[1]);
+    if (in0) update(1, (E3 - e(2, q2 + 1)) * g.inv_dx[0]);
+    return;
   }
-  double b = P.bf[d][t];
-  double b0;
-  if (P.first_stage) { b0 = b; P.b0f[d][t] = b; } else { b0 = P.b0f[d][t]; }
-  P.bf[d][t] = a1 * b0 + a2 * b + a3 * tmp;
+  const long long q0 = cor_lin(g, 0, i, j, k), q0y = n0, q0z = (long long)n0 * (n1 + 1);
+  const long long q1 = cor_lin(g, 1, i, j, k), q1z = (long long)(n0 + 1) * n1;
+  // E1 exists for i < nx1, E2 for j < nx2, E3 for k < nx3
+  const double E1 = in0 ? e(0, q0) : 0.0, E2 = in1 ? e(1, q1) : 0.0, E3 = in2 ? e(2, q2) : 0.0;
+  if (in1 && in2) update(0, -(e(1, q1 + q1z) - E2) * g.inv_dx[2] + (e(2, q2 + q2y) - E3) * g.inv_dx[1]);
+  if (in0 && in2) update(1, (e(0, q0 + q0z) - E1) * g.inv_dx[2] + (E3 - e(2, q2 + 1)) * g.inv_dx[0]);
+  if (in0 && in1) update(2, (e(1, q1 + 1) - E2) * g.inv_dx[0] - (e(0, q0 + q0y) - E1) * g.inv_dx[1]);
 }
 
 // Stage end: flux divergence of the face fluxes, gravity and the RK combine of U

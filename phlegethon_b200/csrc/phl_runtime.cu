@@ -72,17 +72,13 @@ struct RunnerT : Runner {
       if constexpr (C::DIM == 3) k_face<C, 2><<<nblk(nfaces_host(g, 2), 128), 128, 0, s>>>(P);
     }
     if constexpr (C::MHD) {
-      auto ncor = [&](int a) {
-        return (long long)(g.nx[0] + (a != 0)) * (g.nx[1] + (a != 1)) * (C::DIM == 3 ? g.nx[2] + (a != 2) : 1);
-      };
-      if constexpr (C::DIM == 3) {
-        k_corner<C, 0><<<nblk(ncor(0), 256), 256, 0, s>>>(P);
-        k_corner<C, 1><<<nblk(ncor(1), 256), 256, 0, s>>>(P);
-      }
-      k_corner<C, 2><<<nblk(ncor(2), 256), 256, 0, s>>>(P);
-      k_bface<C, 0><<<nblk(nfaces_host(g, 0), 256), 256, 0, s>>>(P);
-      k_bface<C, 1><<<nblk(nfaces_host(g, 1), 256), 256, 0, s>>>(P);
-      if constexpr (C::DIM == 3) k_bface<C, 2><<<nblk(nfaces_host(g, 2), 256), 256, 0, s>>>(P);
+      const long long n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2];
+      const long long nin = (n0 - 1) * (n1 - 1) * (C::DIM == 3 ? n2 - 1 : 1);
+      const long long nrim = 2 * (n0 + n1) * (C::DIM == 3 ? n2 - 1 : 1) + (C::DIM == 3 ? 2 * (n0 + 1) * (n1 + 1) : 0);
+      const unsigned bin = nblk(nin, 256);
+      k_corner<C><<<bin + nblk(nrim, 256), 256, 0, s>>>(P, bin, FastDiv::by((unsigned)n0 - 1),
+                                                        FastDiv::by((unsigned)n1 - 1));
+      k_bface<C><<<nblk((n0 + 1) * (n1 + 1) * (C::DIM == 3 ? n2 + 1 : 1), 256), 256, 0, s>>>(P);
     }
     k_c2p<C><<<nblk(g.N, 128), 128, 0, s>>>(P);
   }

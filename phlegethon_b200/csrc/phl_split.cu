@@ -1210,28 +1210,11 @@ __global__ void __launch_bounds__(256) k_corner_split(Prm P, unsigned nin_blocks
     P.fcor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf_split<C, 2, true>(P, c);
     return;
   }
-  // the nodes on the domain's faces: the k = 0 and k = nx[2] planes (3D), then per inner plane the
-  // border of the (nx[0] + 1) x (nx[1] + 1) rectangle, 2 (nx[0] + nx[1]) of them
-  const int n0 = g.nx[0], n1 = g.nx[1], n2 = g.nx[2], rim = 2 * (n0 + n1);
-  const long long ncap = C::DIM == 3 ? 2ll * (n0 + 1) * (n1 + 1) : 0;
-  long long t = (long long)(blockIdx.x - nin_blocks) * blockDim.x + threadIdx.x;
-  if (t < ncap) {
-    unflatten3(t, g.div0[1], g.div1[1], c[0], c[1], c[2]);
-    c[2] = c[2] ? n2 : 0;
-  } else {
-    t -= ncap;
-    if (t >= (long long)rim * (C::DIM == 3 ? n2 - 1 : 1)) return;
-    const int m = (int)(t % rim);
-    c[2] = C::DIM == 3 ? (int)(t / rim) + 1 : 0;
-    if (m < n0 + 1) { c[0] = m; c[1] = 0; }                                      // x2 = 0 row
-    else if (m < 2 * (n0 + 1)) { c[0] = m - (n0 + 1); c[1] = n1; }               // x2 = nx[1] row
-    else if (m < 2 * (n0 + 1) + (n1 - 1)) { c[0] = 0; c[1] = m - 2 * (n0 + 1) + 1; }  // x1 = 0 column
-    else { c[0] = n0; c[1] = m - 2 * (n0 + 1) - (n1 - 1) + 1; }                  // x1 = nx[0] column
-  }
+  if (!rim_node<C>(g, (long long)(blockIdx.x - nin_blocks) * blockDim.x + threadIdx.x, c)) return;
   if (C::DIM == 3) {
-    if (c[0] < n0) P.fcor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf_split<C, 0, false>(P, c);
-    if (c[1] < n1) P.fcor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf_split<C, 1, false>(P, c);
-    if (c[2] >= n2) return;
+    if (c[0] < g.nx[0]) P.fcor[0][cor_lin(g, 0, c[0], c[1], c[2])] = corner_emf_split<C, 0, false>(P, c);
+    if (c[1] < g.nx[1]) P.fcor[1][cor_lin(g, 1, c[0], c[1], c[2])] = corner_emf_split<C, 1, false>(P, c);
+    if (c[2] >= g.nx[2]) return;
   }
   P.fcor[2][cor_lin(g, 2, c[0], c[1], c[2])] = corner_emf_split<C, 2, false>(P, c);
 }
