@@ -1110,12 +1110,14 @@ __device__ __forceinline__ void cell_emf3(const float v[3], const float b[3], fl
   e[0] = v[2] * b[1] - v[1] * b[2];
   e[1] = v[0] * b[2] - v[2] * b[0];
 }
-// the stage input's cell EMFs, written by the kernel that produced its FP32 state
+// the stage input's cell EMFs, written by the kernel that produced its FP32 state (2D has corners
+// along x3 only)
+template <class C>
 __device__ __forceinline__ void store_cell_emf(const Prm &P, long long c, const float v[3], const float b[3]) {
   float e[3];
   cell_emf3(v, b, e);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) P.fecell[(long long)a * P.g.N + c] = e[a];
+  for (int a = C::DIM == 3 ? 0 : 2; a < 3; ++a) P.fecell[(long long)a * P.g.N + c] = e[a];
 }
 
 // cell-centred -v x B component a of a (possibly ghost) cell from the stored cell EMFs: a mirror
@@ -1373,7 +1375,7 @@ __device__ __forceinline__ void c2p_split_combine(const Prm &P, long long c, C2p
     if (C::MHD) {
       const float bf3[3] = {(float)(bcc[0] * P.inv_b_ref), (float)(bcc[1] * P.inv_b_ref),
                             DIM == 3 ? (float)(bcc[2] * P.inv_b_ref) : 0.0f};
-      store_cell_emf(P, c, vf, bf3);
+      store_cell_emf<C>(P, c, vf, bf3);
     }
 #pragma unroll
     for (int iv = IAS; iv < NV; ++iv) P.Wf_out[(long long)iv * g.N + c] = (float)(u[iv] * inv_rho);
@@ -1484,10 +1486,11 @@ __device__ __forceinline__ bool c2p_split_eos(const Prm &P, long long c, const C
     }
     P.Wf_out[c] = (float)(rdev * P.inv_rho_ref);
     P.Wf_out[(long long)IP * g.N + c] = (float)(pdev * P.inv_p_ref);
-    P.temp[c] = T;
-    P.eint[c] = eint;
     if (!(rho > 0.0) || !(p > 0.0) || !(T > 0.0) || !isfinite(eint)) st.bad += 1;
+    // the next stage starts its Newton from T; nothing in a step reads eint back, nor T without one
+    if (C::HELM || P.last_stage) P.temp[c] = T;
     if (P.last_stage) {
+      P.eint[c] = eint;
       // |v| and b_cc^2 of the new state, read back (U and the face B are this cell's own)
       int i, j, k;
       unflatten3(c, g.div0[0], g.div1[0], i, j, k);
@@ -1743,7 +1746,7 @@ __global__ void k_split_from_prim(Prm P) {
   if (C::MHD) {
     const float vf[3] = {(float)(w[1] / P.v_ref), (float)(w[2] / P.v_ref), DIM == 3 ? (float)(w[3] / P.v_ref) : 0.0f};
     const float bf3[3] = {P.bccf[c], P.bccf[g.N + c], DIM == 3 ? P.bccf[2 * g.N + c] : 0.0f};
-    store_cell_emf(P, c, vf, bf3);
+    store_cell_emf<C>(P, c, vf, bf3);
   }
   P.Wf_out[(long long)IP * g.N + c] = (float)(pdev / P.p_ref);
 #pragma unroll
