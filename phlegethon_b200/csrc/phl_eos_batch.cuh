@@ -86,7 +86,7 @@ __device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, cons
   if (iters) iters[t] = used;
 }
 
-// Learned guess, phase 0: the network's temperature of every sample, left in T for phase 1.  A block
+// Learned guess, phase 0: the network's log10 T of every sample, left in `guess` for phase 1.  A block
 // takes 128 samples: features (the cold energy from 12 table coefficients), one tensor-core product,
 // the FP32 layers as constant-bank operands.  A kernel of its own, so that the waits of the product and
 // the block's barriers are hidden by 8 blocks an SM instead of the 3 that the Newton's registers leave
@@ -94,7 +94,7 @@ __device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, cons
 static __global__ void __launch_bounds__(128, 8) k_eos_guess(HelmTable h, const __grid_constant__ MlpSmall w,
                                                              const __nv_bfloat16 *w2bf, long long n, const double *rho,
                                                              const double *e, const double *abar, const double *zbar,
-                                                             double *T, unsigned long long *stat) {
+                                                             float *guess, unsigned long long *stat) {
   extern __shared__ __align__(128) unsigned char sm[];
   MlpUmmaSmem &S = *reinterpret_cast<MlpUmmaSmem *>(sm);
   mlp_cta_setup(w2bf, S);
@@ -104,18 +104,18 @@ static __global__ void __launch_bounds__(128, 8) k_eos_guess(HelmTable h, const 
   bool ok = true, have = false;
   const float lT = mlp_forward_tile(w, feat, S, 0u, ok, have, stat + STAT_TC_STALLED);
   mlp_cta_teardown(S);
-  if (t < n) T[t] = fmin(fmax(exp10((double)lT), h.Tl * 1.000001), h.Th * 0.999999);
+  if (t < n) guess[t] = lT;
 }
 
 // Phase 1.  guess 0 / 2: warm or bracket guess and the full Newton.  LEARNED: the guess that phase 0
-// left in T, judged by at most 3 reference Newton iterations; a sample whose guess did not
+// left in `lT`, judged by at most 3 reference Newton iterations; a sample whose guess did not
 // converge within them without a reset is appended to `queue` (queue[0] = count, then
 // index | judged iterations << 56) for phase 2, so that the fallback runs in converged warps
 // instead of stalling the accepted lanes.
 template <bool LEARNED>
 __global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long long n, const double *rho, const double *e,
                                                     const double *abar, const double *zbar, double *T,
-                                                    double *p, double *cs, int *iters, int guess,
+                                                    double *p, double *cs, int *iters, int guess, const float *lT,
                                                     unsigned long long *stat, unsigned long long *queue) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   EosStat st;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long 
     int used = 0, clamped = 0;
     bool conv = false;
     if constexpr (LEARNED) {
-      Tg = T[t];
+      Tg = fmin(fmax(exp10((double)lT[t]), h.Tl * 1.000001), h.Th * 0.999999);
       st.v[6] = 1;  // the cold energy of phase 0
       used = helm_rhoe_newton(h, r, ht, ee, Tg, 3, clamped, &conv);
       st.v[3] = clamped;
@@ -206,21 +206,21 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_fallback(HelmTable h, con
   st.flush(stat);
 }
 
-// Launch the inversion on stream s (no synchronisation).  `queue` (n + 1 entries) is needed for
-// the learned guess only.  Returns 0 or a cudaError_t.
+// Launch the inversion on stream s (no synchronisation).  `queue` (n + 1 entries) and `lT` (n) are
+// needed for the learned guess only.  Returns 0 or a cudaError_t.
 inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *e,
                       const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters,
-                      int guess, const Mlp &mlp, unsigned long long *stat, unsigned long long *queue, int nsm) {
+                      int guess, const Mlp &mlp, unsigned long long *stat, unsigned long long *queue, float *lT, int nsm) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
   if (guess != PHL_GUESS_MLP) {
-    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, stat, nullptr);
+    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, nullptr, stat, nullptr);
     return (int)cudaGetLastError();
   }
   const size_t sm = sizeof(MlpUmmaSmem);
   const cudaError_t err = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (err != cudaSuccess) return (int)err;
-  k_eos_guess<<<blocks, 128, sm, s>>>(h, mlp.small, mlp.w2bf, n, rho, e, abar, zbar, T, stat);
-  k_eos_invert<true><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, stat, queue);
+  k_eos_guess<<<blocks, 128, sm, s>>>(h, mlp.small, mlp.w2bf, n, rho, e, abar, zbar, lT, stat);
+  k_eos_invert<true><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, lT, stat, queue);
   // enough resident blocks to cover every SM several times; the loop covers any queue length
   const unsigned fb = (unsigned)std::min<long long>((long long)nsm * 8, (long long)blocks);
   k_eos_fallback<<<fb, 128, 0, s>>>(h, queue, rho, e, abar, zbar, T, p, cs, iters, stat);
@@ -234,6 +234,7 @@ struct EosBatch {
   int *ibuf = nullptr;
   size_t ibytes = 0;
   unsigned long long *queue = nullptr;  // rejected learned guesses (count + entries)
+  float *lT = nullptr;                  // the network's guesses
   long long qcap = 0;
   int nsm = 0;
 
@@ -241,9 +242,11 @@ struct EosBatch {
     if (hbuf) cudaFree(hbuf);
     if (ibuf) cudaFree(ibuf);
     if (queue) cudaFree(queue);
+    if (lT) cudaFree(lT);
     hbuf = nullptr;
     ibuf = nullptr;
     queue = nullptr;
+    lT = nullptr;
     qcap = 0;
     mlp.release();
   }
@@ -272,12 +275,15 @@ struct EosBatch {
     if (n == 0) return 0;
     if (guess == PHL_GUESS_MLP && qcap < n + 1) {
       if (queue) cudaFree(queue);
+      if (lT) cudaFree(lT);
       queue = nullptr;
+      lT = nullptr;
       qcap = 0;
       if (cudaMalloc(&queue, sizeof(unsigned long long) * (size_t)(n + 1)) != cudaSuccess) return -2;
+      if (cudaMalloc(&lT, sizeof(float) * (size_t)n) != cudaSuccess) return -2;
       qcap = n + 1;
     }
-    if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp, stat, queue, sm_count()))
+    if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp, stat, queue, lT, sm_count()))
       return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
     return 0;

@@ -1369,10 +1369,13 @@ static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_FIELDS * PHL_N
 static __device__ __align__(256) int g_noalloc_iters[PHL_NOALLOC_MAX_SAMPLES];
 // queue of rejected learned guesses: count, then one entry per sample
 static __device__ __align__(256) unsigned long long g_noalloc_queue[PHL_NOALLOC_MAX_SAMPLES + 1];
+// the network's guesses
+static __device__ __align__(256) float g_noalloc_guess[PHL_NOALLOC_MAX_SAMPLES];
 constexpr int NOALLOC_MAX_DEVICES = 64;
 double *g_noalloc_dev[NOALLOC_MAX_DEVICES] = {};
 int *g_noalloc_idev[NOALLOC_MAX_DEVICES] = {};
 unsigned long long *g_noalloc_qdev[NOALLOC_MAX_DEVICES] = {};
+float *g_noalloc_gdev[NOALLOC_MAX_DEVICES] = {};
 
 int noalloc_symbol(void **dst, const void *symbol, const char *name) {
   cudaError_t e = cudaGetSymbolAddress(dst, symbol);
@@ -1385,22 +1388,25 @@ std::mutex g_noalloc_mutex;
 
 // once per device, with that device current; the mutex makes the first calls of several host
 // threads on one device look the addresses up once
-int noalloc_setup(int device, double **buf, int **ibuf, unsigned long long **queue) {
+int noalloc_setup(int device, double **buf, int **ibuf, unsigned long long **queue, float **guess) {
   if (device < 0 || device >= NOALLOC_MAX_DEVICES) return PHL_E_INVALID;
   std::lock_guard<std::mutex> lock(g_noalloc_mutex);
   if (!g_noalloc_dev[device]) {
-    void *p = nullptr, *q = nullptr, *r = nullptr;
+    void *p = nullptr, *q = nullptr, *r = nullptr, *u = nullptr;
     int rc;
+    if ((rc = noalloc_symbol(&u, g_noalloc_guess, "g_noalloc_guess"))) return rc;
     if ((rc = noalloc_symbol(&p, g_noalloc_scratch, "g_noalloc_scratch"))) return rc;
     if ((rc = noalloc_symbol(&q, g_noalloc_iters, "g_noalloc_iters"))) return rc;
     if ((rc = noalloc_symbol(&r, g_noalloc_queue, "g_noalloc_queue"))) return rc;
     g_noalloc_idev[device] = static_cast<int *>(q);
     g_noalloc_qdev[device] = static_cast<unsigned long long *>(r);
+    g_noalloc_gdev[device] = static_cast<float *>(u);
     g_noalloc_dev[device] = static_cast<double *>(p);
   }
   *buf = g_noalloc_dev[device];
   *ibuf = g_noalloc_idev[device];
   *queue = g_noalloc_qdev[device];
+  *guess = g_noalloc_gdev[device];
   return PHL_OK;
 }
 }  // namespace
@@ -1421,7 +1427,8 @@ extern "C" int phl_eos_invert_batch_noalloc(phl_ctx *ctx, long long n, const dou
   double *buf = nullptr;
   int *ibuf = nullptr;
   unsigned long long *queue = nullptr;
-  int rc = noalloc_setup(ctx->cfg.device, &buf, &ibuf, &queue);
+  float *lT = nullptr;
+  int rc = noalloc_setup(ctx->cfg.device, &buf, &ibuf, &queue, &lT);
   if (rc) return rc;
   cudaStream_t s = ctx->stream;
   const size_t M = PHL_NOALLOC_MAX_SAMPLES, b = sizeof(double) * (size_t)n;
@@ -1435,7 +1442,7 @@ extern "C" int phl_eos_invert_batch_noalloc(phl_ctx *ctx, long long n, const dou
   CK(cudaMemcpyAsync(d_z, zbar, b, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_T, T_inout, b, cudaMemcpyHostToDevice, s));
   CK((cudaError_t)eos_launch(ctx->helm, s, n, d_rho, d_e, d_a, d_z, d_T, p ? d_p : nullptr, cs ? d_c : nullptr,
-                             iters ? ibuf : nullptr, guess, ctx->eos.mlp, ctx->stat, queue,
+                             iters ? ibuf : nullptr, guess, ctx->eos.mlp, ctx->stat, queue, lT,
                              ctx->eos.sm_count()));
   CK(cudaMemcpyAsync(T_inout, d_T, b, cudaMemcpyDeviceToHost, s));
   if (p) CK(cudaMemcpyAsync(p, d_p, b, cudaMemcpyDeviceToHost, s));
