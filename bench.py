@@ -117,13 +117,15 @@ def step_launches(cfg, form, guess="warm"):
 # DRAM bytes per cell of one stage-kernel launch, from ncu captures of the 128^3 stratified box
 # (dram__bytes_read.sum + dram__bytes_write.sum over 2,097,152 cells); the kernel streams the
 # domain once per launch, so the per-launch traffic scales with the cell count
-TRAFFIC_PER_CELL = {("stratified", "fp32_split"): 499.604224e6 / 2097152,
-                    ("stratified", "fp64"): 557.258496e6 / 2097152,
-                    # one split MHD stage at 128^3 (a middle stage: U0 read): x1 tile faces
-                    # 216.9 MB, walking x2/x3 faces 186.1 + 190.0 MB, corners 3 x 42.2 MB,
-                    # face-B 3 x 50.9 MB, cons->prim 755.2 MB
-                    ("stratified_mhd", "fp32_split"): (216.9e6 + 186.1e6 + 190.0e6 + 3 * 42.2e6 + 3 * 50.9e6
-                                                       + 755.2e6) / 2097152}
+TRAFFIC_PER_CELL = {("stratified", "fp64"): 557.258496e6 / 2097152,
+                    # one split hydro stage at 128^3: row and walk faces 98.5 + 97.1 + 99.1 MB,
+                    # cons->prim 632.0 MB
+                    ("stratified", "fp32_split"): (98.5e6 + 97.1e6 + 99.1e6 + 632.0e6) / 2097152,
+                    # one split MHD stage at 128^3 (a middle stage: U0 read): row faces 154.1 MB,
+                    # walking x2/x3 faces 155.9 + 165.0 MB, corners 132.1 MB, face B 117.6 MB,
+                    # cons->prim 727.9 MB
+                    ("stratified_mhd", "fp32_split"): (154.1e6 + 155.9e6 + 165.0e6 + 132.1e6 + 117.6e6
+                                                       + 727.9e6) / 2097152}
 
 
 # Algorithmic HBM bytes per zone-update of the workloads (minimum traffic of one step of a fused

@@ -714,11 +714,22 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
       }
     }
   }
-  // face fluxes, FP64 or FP32
-  for (int d = 0; d < cfg->sdims; ++d)
-    if ((rc = c->split ? c->alloc(&c->fflux[d], (size_t)nv * c->nfaces(d))
-                       : c->alloc(&c->dflux[d], (size_t)nv * c->nfaces(d))))
-      return rc;
+  // face fluxes, FP64 or FP32.  The split hydro form can do without (its one-kernel stage solves the
+  // faces in place): a domain that leaves no room for them still runs
+  if (!c->split) {
+    for (int d = 0; d < cfg->sdims; ++d)
+      if ((rc = c->alloc(&c->dflux[d], (size_t)nv * c->nfaces(d)))) return rc;
+  } else {
+    size_t off[4] = {0, 0, 0, 0};  // in floats, each direction on 256 bytes
+    for (int d = 0; d < 3; ++d)
+      off[d + 1] = off[d] + (d < cfg->sdims ? ((size_t)nv * c->nfaces(d) + 63) / 64 * 64 : 0);
+    float *all = nullptr;
+    if ((rc = c->alloc(&all, off[3]))) {
+      if (mhd) return rc;
+      cudaGetLastError();  // the failed allocation is no error of the calls that follow
+    }
+    for (int d = 0; d < cfg->sdims && all; ++d) c->fflux[d] = all + off[d];
+  }
   if ((rc = c->alloc(&c->scal, 8))) return rc;
   if ((rc = c->alloc(&c->smax_bits, 1))) return rc;
   if ((rc = c->alloc(&c->active, 1))) return rc;

@@ -1038,7 +1038,7 @@ __global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : 
 // differences and edge values of its neighbours come by shuffle, each slope is formed once, and
 // nothing is carried between faces, so the kernel needs no shared memory, no barrier and any row
 // length fits.  Lanes 0, 1 and 31 hold the stencil's rim: lane l (2 <= l < 31) solves the face
-// below its cell.  Bound by issue slots (70% of the cycles issue, 690 instructions a face); 67 us
+// below its cell.  Bound by issue slots (70% of the cycles issue, 750 instructions a face); 67 us
 // for the x1 faces of a 128^3 MHD stage, where tiles staged in shared memory by bulk copies (766
 // instructions, two block barriers a tile) took 83 and a walk of 4 faces 1% more per stage.
 template <class C>
@@ -1832,7 +1832,9 @@ struct SplitRunnerT : Runner {
     const char *e = getenv("PHL_STAGE_KERNEL");
     return e && strcmp(e, "cell") == 0 ? 1 : (e && strcmp(e, "faces") == 0 ? 2 : 0);
   }();
-  bool one_kernel(const Geo &g) const {
+  bool one_kernel(const Prm &P) const {
+    const Geo &g = P.g;
+    if (!P.fflux[0]) return true;  // no room for the face fluxes
     if (stage_kind) return stage_kind == 1;
     return g.N < (C::DIM == 3 ? 220000 : 430000);
   }
@@ -1841,7 +1843,7 @@ struct SplitRunnerT : Runner {
       k_sf_mark_split<C><<<nblk(sf_mark_cells<C>(P.g), 256), 256, 0, s>>>(P);
       k_sf_flag<C><<<nblk(sf_flag_cells<C>(P.g), 256), 256, 0, s>>>(P);
     }
-    if (!C::MHD && one_kernel(P.g)) {
+    if (!C::MHD && one_kernel(P)) {
       if constexpr (!C::MHD) k_stage_split<C><<<nblk(P.g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
     } else {
       const Geo &g = P.g;
