@@ -19,6 +19,7 @@
 #define PHL_KERNEL_UNIT fp64_unit
 #include "phl_kernels.cuh"
 #include "phl_runner.h"
+#include "phl_memory.h"
 #include "phl_eos_batch.cuh"
 
 using namespace phl;
@@ -294,7 +295,7 @@ struct phl_ctx {
   cudaEvent_t ev_in[HOST_SLOTS] = {}, ev_pack[HOST_SLOTS] = {};
   // EoS batch scratch and MLP
   EosBatch eos;
-  std::vector<void *> allocs;
+  DeviceMemory mem;
 
   ~phl_ctx() {
     drop_graphs();
@@ -307,7 +308,7 @@ struct phl_ctx {
     }
     if (cin) cudaStreamDestroy(cin);
     if (cout) cudaStreamDestroy(cout);
-    for (void *a : allocs) cudaFree(a);
+    mem.release();
     if (stream) cudaStreamDestroy(stream);
   }
   // wait for the downloads of earlier asynchronous host-state calls (every entry point that
@@ -319,18 +320,15 @@ struct phl_ctx {
     hpipe_pending = false;
     return PHL_OK;
   }
+  // room for `count` elements at *p (zeroed and moved when it has to grow)
   template <class T>
   int alloc(T **p, size_t count) {
-    void *q = nullptr;
-    if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T));
-    if (e != cudaSuccess) {
-      g_last_error = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    if (*p && mem.size(*p) >= count * sizeof(T)) return PHL_OK;
+    if (!mem.grow(p, count)) {
+      g_last_error = mem.error;
       return PHL_E_CUDA;
     }
-    cudaMemsetAsync(q, 0, count * sizeof(T), stream);
-    allocs.push_back(q);
-    *p = (T *)q;
+    cudaMemsetAsync(*p, 0, mem.size(*p), stream);
     return PHL_OK;
   }
   long long nfaces(int d) const {
@@ -423,7 +421,7 @@ struct phl_ctx {
     for (int d = 0; d < dim; ++d) {
       long long nf = geo.bg_profile ? (long long)(geo.nx[1] + (d == 1)) : nfaces(d);
       int rc;
-      if (!sf_bg[d] && (rc = alloc(&sf_bg[d], 4 * nf))) return rc;
+      if ((rc = alloc(&sf_bg[d], 4 * nf))) return rc;
       k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_rho_f[d], sf_bg[d], nf, rho_ref);
       k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_p_f[d], sf_bg[d] + 1, nf, p_ref);
       if (helm) k_scale_f32<<<nblk(nf, 256), 256, 0, stream>>>(eq_ge_f[d], sf_bg[d] + 2, nf, 1.0);
@@ -883,12 +881,13 @@ int phl_upload_state(phl_ctx *ctx, const phl_fields *f) {
       faceprof(f->phi_x[d], 1, 0, d);
       if (helm) faceprof(f->eq_gammae_x[d], 1, 0, d);
     }
+    // From here to the end of the call layout and buffers do not belong together, and a buffer that has
+    // to grow moves: nothing steps with them if the call fails, and the graphs hold the old ones.
+    ctx->uploaded = ctx->bg_uploaded = false;
+    ctx->drop_graphs();
     ctx->bg_profile = ok ? 1 : 0;
     ctx->geo.bg_profile = ctx->bg_profile;
-    auto need = [&](double **p, size_t n) -> int {
-      if (!*p) return ctx->alloc(p, n);
-      return PHL_OK;
-    };
+    auto need = [&](double **p, size_t n) { return ctx->alloc(p, n); };
     size_t ncc = ok ? (size_t)ny : (size_t)N;
     if ((rc = need(&ctx->eq_rho_cc, ncc)) || (rc = need(&ctx->eq_p_cc, ncc)) || (rc = need(&ctx->phi_cc, ncc)) ||
         (rc = need(&ctx->grav, (size_t)sd * ncc)))
@@ -942,7 +941,7 @@ int phl_upload_state(phl_ctx *ctx, const phl_fields *f) {
     std::vector<double> prof;
     bool pr = extract_profile(f->eq_prim_cc, 3, 1, n1, n2, n3, 0, 0, 0, n1, n2, n2, prof);
     size_t ne = pr ? (size_t)n2 : (size_t)Ng;
-    if (!ctx->sf_eq_p && (rc = ctx->alloc(&ctx->sf_eq_p, (size_t)Ng))) return rc;
+    if ((rc = ctx->alloc(&ctx->sf_eq_p, (size_t)Ng))) return rc;
     std::vector<double> full;
     if (!pr) {
       full.resize(ne);
@@ -958,10 +957,7 @@ int phl_upload_state(phl_ctx *ctx, const phl_fields *f) {
     CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(s));
-  if (strat && f->eq_prim_cc) {
-    ctx->bg_uploaded = true;
-    ctx->drop_graphs();  // they bake the background layout into their kernel arguments
-  }
+  if (strat && f->eq_prim_cc) ctx->bg_uploaded = true;
   ctx->uploaded = true;
   return PHL_OK;
 }

@@ -74,6 +74,57 @@ def test_new_state_and_background_after_graphs(gpu_lib):
     assert max_abs_diff(ha, hb) == 0.0
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32_split"])
+def test_full_background_after_a_profile(gpu_lib, precision):
+    """The first background is a profile along x2, the second varies along x1: its arrays are larger, and
+    the step graphs hold the layout and the addresses of the first.  Same states as a fresh context."""
+    cfg, h = problems.hot_bubble_2d(20)
+    cfg = cfg.replace(precision=precision)
+    h2 = h.copy()
+    x = h.coords()[0]
+    wave = lambda x: 1.0 + 1e-3 * np.sin(2.0 * np.pi * x)
+    h2.eq_prim_cc[:2] *= wave(x)
+    for d in range(2):
+        h2.eq_prim_x[d][:2] *= wave(h.face_coords(d)[0])
+    ha, hb, hc = h2.copy(), h2.copy(), h.copy()
+
+    def steps(sim):
+        for _ in range(3):
+            sim.hydro_step()
+            sim.compute_hyperbolic_dt()
+        sim.time_loop(3)
+
+    def again(sim, h):
+        sim.upload(h)
+        sim.init_thermo()
+        sim.compute_hyperbolic_dt()
+
+    with start(cfg, h, None) as sim:
+        for _ in range(13):
+            sim.hydro_step()
+            sim.compute_hyperbolic_dt()
+        sim.time_loop(2)
+        again(sim, h2)
+        steps(sim)
+        sim.download(ha)
+        again(sim, h)  # and the profile again
+        steps(sim)
+        sim.download(hc)
+    with start(cfg, h2, None) as sim:
+        steps(sim)
+        sim.download(hb)
+    assert np.isfinite(hb.interior(hb.prim)).all()
+    assert max_abs_diff(ha, hb) == 0.0
+    hd = h.copy()
+    with start(cfg, h, None) as sim:
+        if cfg.precision == "fp32_split":
+            # the scales of the split form are those of the first state a context was given
+            assert h.prim[0].max() == h2.prim[0].max() and h.prim[3].max() == h2.prim[3].max()
+        steps(sim)
+        sim.download(hd)
+    assert max_abs_diff(hc, hd) == 0.0
+
+
 def test_tmax_and_steps_between_calls(gpu_lib):
     """steps_done and the time of consecutive calls, with the clamp to tmax and calls that do nothing."""
     cfg, h = problems.hot_bubble_2d(16)
