@@ -230,26 +230,13 @@ inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const dou
 struct EosBatch {
   Mlp mlp;
   double *hbuf = nullptr;  // staging for the host-pointer variant
-  size_t hbytes = 0;
   int *ibuf = nullptr;
-  size_t ibytes = 0;
   unsigned long long *queue = nullptr;  // rejected learned guesses (count + entries)
   float *lT = nullptr;                  // the network's guesses
-  long long qcap = 0;
   int nsm = 0;
+  DeviceMemory *mem = nullptr;
 
-  void release() {
-    if (hbuf) cudaFree(hbuf);
-    if (ibuf) cudaFree(ibuf);
-    if (queue) cudaFree(queue);
-    if (lT) cudaFree(lT);
-    hbuf = nullptr;
-    ibuf = nullptr;
-    queue = nullptr;
-    lT = nullptr;
-    qcap = 0;
-    mlp.release();
-  }
+  void use(DeviceMemory *m) { mem = mlp.mem = m; }
   int sm_count() {
     if (!nsm) {
       int dev = 0;
@@ -273,16 +260,7 @@ struct EosBatch {
     if (guess < 0 || guess > 2) return -1;
     if (guess == PHL_GUESS_MLP && !mlp.ready) return -4;
     if (n == 0) return 0;
-    if (guess == PHL_GUESS_MLP && qcap < n + 1) {
-      if (queue) cudaFree(queue);
-      if (lT) cudaFree(lT);
-      queue = nullptr;
-      lT = nullptr;
-      qcap = 0;
-      if (cudaMalloc(&queue, sizeof(unsigned long long) * (size_t)(n + 1)) != cudaSuccess) return -2;
-      if (cudaMalloc(&lT, sizeof(float) * (size_t)n) != cudaSuccess) return -2;
-      qcap = n + 1;
-    }
+    if (guess == PHL_GUESS_MLP && !(mem->grow(&queue, (size_t)n + 1) && mem->grow(&lT, (size_t)n))) return -2;
     if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp, stat, queue, lT, sm_count()))
       return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
@@ -292,19 +270,7 @@ struct EosBatch {
                   const double *abar, const double *zbar, double *T, double *p, double *cs, int *iters, int guess,
                   unsigned long long *stat) {
     if (n == 0) return 0;
-    size_t need = sizeof(double) * (size_t)n * 7;
-    if (need > hbytes) {
-      if (hbuf) cudaFree(hbuf);
-      hbuf = nullptr;
-      if (cudaMalloc(&hbuf, need) != cudaSuccess) { hbytes = 0; return -2; }
-      hbytes = need;
-    }
-    if (iters && sizeof(int) * (size_t)n > ibytes) {
-      if (ibuf) cudaFree(ibuf);
-      ibuf = nullptr;
-      if (cudaMalloc(&ibuf, sizeof(int) * (size_t)n) != cudaSuccess) { ibytes = 0; return -2; }
-      ibytes = sizeof(int) * (size_t)n;
-    }
+    if (!mem->grow(&hbuf, (size_t)n * 7) || (iters && !mem->grow(&ibuf, (size_t)n))) return -2;
     double *d_rho = hbuf, *d_e = hbuf + n, *d_a = hbuf + 2 * n, *d_z = hbuf + 3 * n, *d_T = hbuf + 4 * n;
     double *d_p = hbuf + 5 * n, *d_c = hbuf + 6 * n;
     size_t b = sizeof(double) * (size_t)n;

@@ -16,6 +16,7 @@
 #include <mma.h>
 #include <cmath>
 #include "phl_device.cuh"
+#include "phl_memory.h"
 #include "phl_umma.cuh"
 
 namespace phl {
@@ -484,25 +485,23 @@ struct Mlp {
   float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *partial = nullptr, *lossp = nullptr;
   float *feat = nullptr, *target = nullptr;
   __nv_bfloat16 *w2bf = nullptr;
-  long long nsamp = 0;
-  int npart = 0;
+  long long nsamp = 0;  // samples in feat and target
+  DeviceMemory *mem = nullptr;
 
-  void release() {
-    for (void *p : {(void *)params, (void *)grad, (void *)m, (void *)v, (void *)partial, (void *)lossp,
-                    (void *)feat, (void *)target, (void *)w2bf})
-      if (p) cudaFree(p);
-    params = grad = m = v = partial = lossp = feat = target = nullptr;
-    w2bf = nullptr;
-    ready = false;
-  }
   MlpWeights weights() const { return MlpWeights{params, w2bf}; }
   int alloc() {
-    if (params) return 0;
-    if (cudaMalloc(&params, sizeof(float) * MLP_NPARAM) || cudaMalloc(&grad, sizeof(float) * MLP_NPARAM) ||
-        cudaMalloc(&m, sizeof(float) * MLP_NPARAM) || cudaMalloc(&v, sizeof(float) * MLP_NPARAM) ||
-        cudaMalloc(&w2bf, sizeof(__nv_bfloat16) * MLP_H * MLP_H))
-      return -2;
-    return 0;
+    return mem->grow(&params, MLP_NPARAM) && mem->grow(&grad, MLP_NPARAM) && mem->grow(&m, MLP_NPARAM) &&
+                   mem->grow(&v, MLP_NPARAM) && mem->grow(&w2bf, MLP_H * MLP_H)
+               ? 0
+               : -2;
+  }
+  // room for n samples and the partial gradients and losses of a batch
+  int alloc_samples(long long n, long long batch) {
+    nsamp = n;
+    return mem->grow(&feat, (size_t)4 * n) && mem->grow(&target, (size_t)n) &&
+                   mem->grow(&partial, (size_t)(batch / MLP_TILE) * MLP_PSTRIDE) && mem->grow(&lossp, (size_t)batch)
+               ? 0
+               : -2;
   }
   int set(cudaStream_t s, const float *h) {
     if (alloc()) return -2;
@@ -541,23 +540,8 @@ struct Mlp {
   int train(const HelmTable &h, cudaStream_t s, long long n, unsigned long long seed, int epochs, int batch,
             double lr, double *final_loss) {
     if (batch % MLP_TILE || batch <= 0 || n < batch) return -1;
-    if (alloc()) return -2;
-    if (n != nsamp) {
-      if (feat) cudaFree(feat);
-      if (target) cudaFree(target);
-      feat = target = nullptr;
-      if (cudaMalloc(&feat, sizeof(float) * 4 * n) || cudaMalloc(&target, sizeof(float) * n)) return -2;
-      nsamp = n;
-    }
+    if (alloc() || alloc_samples(n, batch)) return -2;
     int nb = batch / MLP_TILE;
-    if (nb > npart) {
-      if (partial) cudaFree(partial);
-      if (lossp) cudaFree(lossp);
-      partial = lossp = nullptr;
-      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_PSTRIDE) || cudaMalloc(&lossp, sizeof(float) * batch))
-        return -2;
-      npart = nb;
-    }
     if (cudaFuncSetAttribute(k_mlp_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(MlpTrainSmem)) != cudaSuccess)
       return -2;
@@ -596,22 +580,7 @@ struct Mlp {
   // gradient on caller-provided pairs (host arrays), for checking against a CPU reference
   int gradient_host(cudaStream_t s, long long n, const float *hf, const float *ht, float *hg, double *loss) {
     if (!ready || n <= 0 || n % MLP_TILE) return -1;
-    if (n != nsamp) {
-      if (feat) cudaFree(feat);
-      if (target) cudaFree(target);
-      feat = target = nullptr;
-      if (cudaMalloc(&feat, sizeof(float) * 4 * n) || cudaMalloc(&target, sizeof(float) * n)) return -2;
-      nsamp = n;
-    }
-    int nb = (int)(n / MLP_TILE);
-    if (nb > npart) {
-      if (partial) cudaFree(partial);
-      if (lossp) cudaFree(lossp);
-      partial = lossp = nullptr;
-      if (cudaMalloc(&partial, sizeof(float) * (size_t)nb * MLP_PSTRIDE) || cudaMalloc(&lossp, sizeof(float) * n))
-        return -2;
-      npart = nb;
-    }
+    if (alloc_samples(n, n)) return -2;
     if (cudaFuncSetAttribute(k_mlp_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(MlpTrainSmem)) != cudaSuccess)
       return -2;

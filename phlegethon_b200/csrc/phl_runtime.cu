@@ -259,7 +259,6 @@ struct phl_ctx {
   bool table_loaded = false, uploaded = false, bg_uploaded = false;
   // staging
   double *stage_buf = nullptr;
-  size_t stage_bytes = 0;
   // graphs: one per parity of the W ping-pong
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   // the same of hydro_step alone, captured once a caller has made HYDRO_GRAPH_AFTER calls (a graph
@@ -300,7 +299,6 @@ struct phl_ctx {
   ~phl_ctx() {
     drop_graphs();
     if (mail) cudaFreeHost(mail);
-    eos.release();
     for (cudaEvent_t e : ev_chunk_out) cudaEventDestroy(e);
     for (int q = 0; q < HOST_SLOTS; ++q) {
       if (ev_in[q]) cudaEventDestroy(ev_in[q]);
@@ -338,12 +336,9 @@ struct phl_ctx {
     return (long long)(geo.nx[0] + (a != 0)) * (geo.nx[1] + (a != 1)) * (dim == 3 ? geo.nx[2] + (a != 2) : 1);
   }
   int ensure_stage(size_t bytes) {
-    if (bytes <= stage_bytes) return PHL_OK;
-    if (stage_buf) cudaFree(stage_buf);
-    stage_buf = nullptr;
-    CK(cudaMalloc(&stage_buf, bytes));
-    stage_bytes = bytes;
-    return PHL_OK;
+    if (mem.grow(&stage_buf, (bytes + sizeof(double) - 1) / sizeof(double))) return PHL_OK;
+    g_last_error = mem.error;
+    return PHL_E_CUDA;
   }
   Prm prm(int stage_idx) const {
     Prm P;
@@ -616,6 +611,7 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
   c->cfg = *cfg;
   c->dim = cfg->sdims;
   c->nv = cfg->nvars;
+  c->eos.use(&c->mem);
   bool mhd = cfg->flags & PHL_MHD, helm = cfg->flags & PHL_HELMHOLTZ;
   bool wb = cfg->flags & PHL_WB, etot = cfg->flags & PHL_EVOLVE_ETOT, grav = cfg->flags & PHL_GRAVITY;
   if (!(wb == etot && etot == grav)) return PHL_E_UNSUPPORTED;
@@ -755,14 +751,12 @@ int phl_load_helm_table(phl_ctx *ctx, const double *tab, const double *dpdr) {
   if (nr < 2 || nT < 2) return PHL_E_INVALID;
   CK(cudaSetDevice(c.device));
   int rc;
-  if (!ctx->htab) {
-    if ((rc = ctx->alloc(&ctx->htab, (size_t)9 * nr * nT))) return rc;
-    if ((rc = ctx->alloc(&ctx->hdpd, (size_t)4 * nr * nT))) return rc;
-    if ((rc = ctx->alloc(&ctx->hrho, (size_t)nr))) return rc;
-    if ((rc = ctx->alloc(&ctx->hT, (size_t)nT))) return rc;
-    if ((rc = ctx->alloc(&ctx->hirho, (size_t)nr))) return rc;
-    if ((rc = ctx->alloc(&ctx->hiT, (size_t)nT))) return rc;
-  }
+  if ((rc = ctx->alloc(&ctx->htab, (size_t)9 * nr * nT))) return rc;
+  if ((rc = ctx->alloc(&ctx->hdpd, (size_t)4 * nr * nT))) return rc;
+  if ((rc = ctx->alloc(&ctx->hrho, (size_t)nr))) return rc;
+  if ((rc = ctx->alloc(&ctx->hT, (size_t)nT))) return rc;
+  if ((rc = ctx->alloc(&ctx->hirho, (size_t)nr))) return rc;
+  if ((rc = ctx->alloc(&ctx->hiT, (size_t)nT))) return rc;
   // nodes as load_helm_table builds them (source.F90:23091-23104)
   double dT = (c.helm_lthi - c.helm_ltlo) / (double)(nT - 1);
   double drho = (c.helm_ldhi - c.helm_ldlo) / (double)(nr - 1);
@@ -1166,13 +1160,15 @@ int host_pipe_setup(phl_ctx *ctx) {
     if ((rc = ctx->alloc(&h.in, h.plane() * h.h3)) ||
         (rc = ctx->alloc(&h.out, (size_t)h.ncomp * h.fx * h.fy * h.fz)))
       return rc;
-    CK(cudaEventCreateWithFlags(&ctx->ev_in[q], cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ctx->ev_pack[q], cudaEventDisableTiming));
+    // (what a call that failed on its way has made already stays)
+    if (!ctx->ev_in[q]) CK(cudaEventCreateWithFlags(&ctx->ev_in[q], cudaEventDisableTiming));
+    if (!ctx->ev_pack[q]) CK(cudaEventCreateWithFlags(&ctx->ev_pack[q], cudaEventDisableTiming));
   }
-  ctx->ev_chunk_out.assign(nchunks, nullptr);
-  for (int k = 0; k < nchunks; ++k) CK(cudaEventCreateWithFlags(&ctx->ev_chunk_out[k], cudaEventDisableTiming));
-  CK(cudaStreamCreateWithFlags(&ctx->cin, cudaStreamNonBlocking));
-  CK(cudaStreamCreateWithFlags(&ctx->cout, cudaStreamNonBlocking));
+  ctx->ev_chunk_out.resize(nchunks, nullptr);
+  for (cudaEvent_t &e : ctx->ev_chunk_out)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!ctx->cin) CK(cudaStreamCreateWithFlags(&ctx->cin, cudaStreamNonBlocking));
+  if (!ctx->cout) CK(cudaStreamCreateWithFlags(&ctx->cout, cudaStreamNonBlocking));
   CK(cudaStreamSynchronize(ctx->stream));  // the staging allocations are zeroed on it
   ctx->hpipe_ready = true;
   return PHL_OK;

@@ -36,6 +36,8 @@ void fake_reset(void) {
   refuse_graphs = 0;
   last = cudaSuccess;
   room = (size_t)1 << 40;
+  used = 0;
+  for (int b = 0; b < nblk; ++b) blk[b].live = 0;  /* what an earlier test left */
 }
 void fake_room(size_t bytes) { room = bytes; }           /* capacity of the device */
 size_t fake_used(void) { return used; }

@@ -1,5 +1,8 @@
 """What the host does with device memory, on the CPU: the library linked with a runtime that has no device
 (hostrt.py)."""
+import ctypes as C
+import gc
+
 import numpy as np
 import pytest
 
@@ -87,7 +90,7 @@ def test_background_buffers_grow_with_the_layout(rt, case, precision):
         sim.upload(h)
         k_unpack_fits(rt)
         k_scale_fits(rt)
-    assert rt.violations() == 0
+    assert rt.violations() == 0 and rt.used() == 0
 
 
 def test_refused_background_leaves_a_context_that_does_not_run(rt):
@@ -121,4 +124,128 @@ def test_refused_background_leaves_a_context_that_does_not_run(rt):
         k_scale_fits(rt)
         assert refused > 0
         sim.time_loop(1)
-    assert rt.violations() == 0
+    assert rt.violations() == 0 and rt.used() == 0
+
+
+# ------------------------------------------------------------------ buffers that could not be replaced
+PSTRIDE, TILE = 4608, 64  # floats per partial gradient, samples per block of k_mlp_train_step
+
+
+def train_launches_fit(rt):
+    """Every training launch finds its samples, partial gradients and losses in live blocks."""
+    rows = rt.launches_of("k_mlp_train_step")
+    for grid, (_, _, _, _, n, _, batch, _, _), room in rows:
+        assert room[0] > 0 and room[1] > 0
+        assert room[2] >= 16 * n and room[3] >= 4 * n
+        assert room[7] >= 4 * PSTRIDE * grid and room[8] >= 4 * batch and grid * TILE == batch
+    for _, _, room in rt.launches_of("k_mlp_adam") + rt.launches_of("k_mlp_reduce"):
+        assert all(room[i] > 0 for i in (0, 2))
+    return len(rows)
+
+
+def each_refusal(rt, call, retry):
+    """call() with its first, second, ... allocation refused, retry() after each; the number refused."""
+    refused = 0
+    while True:
+        rt.refuse(refused)
+        rc = call()
+        rt.refuse(-1)
+        if rc == 0:
+            return refused
+        assert rc == -2 and refused < 30
+        refused += 1
+        retry()
+
+
+def test_training_after_a_refused_allocation(rt):
+    """Training and gradient calls whose buffers could not grow, then calls of the old sizes."""
+    cfg, h = problem("hydro")
+    rt.watch("k_mlp_train_step", "PPPPPPiPP")
+    rt.watch("k_mlp_adam", "PiPPP")
+    rt.watch("k_mlp_reduce", "PiP")
+    feat, target, grad = np.zeros((4096, 4), np.float32), np.zeros(4096, np.float32), np.zeros(4545, np.float32)
+    with started(cfg, h) as sim:
+        loss = C.c_double()
+        train = lambda n, batch: sim.lib.phl_mlp_train(sim.ctx, n, 1, 1, batch, 1e-3, C.byref(loss))
+        gradient = lambda n: sim.lib.phl_mlp_gradient(sim.ctx, n, feat.ctypes.data, target.ctypes.data,
+                                                      grad.ctypes.data, C.byref(loss))
+
+        def again(n, batch):
+            assert train(n, batch) == 0 and gradient(batch) == 0
+
+        # the first call of a context, parameters included
+        assert each_refusal(rt, lambda: train(256, 64), lambda: None) > 1
+        # more samples, a larger batch, gradients of more samples than a batch
+        assert each_refusal(rt, lambda: train(2048, 64), lambda: again(256, 64)) > 0
+        assert each_refusal(rt, lambda: train(2048, 512), lambda: again(2048, 64)) > 0
+        assert each_refusal(rt, lambda: gradient(4096), lambda: again(2048, 512)) > 0
+        again(256, 64)
+        assert train_launches_fit(rt) > 40
+    assert rt.violations() == 0 and rt.used() == 0
+
+
+@pytest.mark.parametrize("guess", [1, 2])
+def test_batch_after_a_refused_allocation(rt, guess):
+    """Batch inversions of host arrays whose buffers could not grow, then smaller ones."""
+    cfg, h = problem("hydro")
+    rt.watch("k_eos_guess", "ssPPPPPPPP")
+    rt.watch("k_eos_invertILb1E", "sPPPPPPPPPiPPP")
+    rt.watch("k_eos_invertILb0E", "sPPPPPPPPPiPPP")
+    with started(cfg, h) as sim:
+        assert sim.lib.phl_mlp_set_params(sim.ctx, (C.c_float * 4545)()) == 0
+
+        def invert(n):
+            a = [np.ones(n) for _ in range(7)]
+            it = np.zeros(n, np.int32)
+            return sim.lib.phl_eos_invert_batch(sim.ctx, n, *[x.ctypes.data for x in a], it.ctypes.data, guess)
+        assert each_refusal(rt, lambda: invert(100), lambda: None) > 0
+        assert each_refusal(rt, lambda: invert(1000), lambda: invert(50)) > 0
+        for _, (_, n, *_), room in rt.launches_of("k_eos_invertILb%dE" % (guess == 1)):
+            assert all(room[i] >= 8 * n for i in range(2, 9)) and room[9] >= 4 * n
+            if guess == 1:
+                assert room[11] >= 4 * n and room[13] >= 8 * (n + 1)
+        if guess == 1:
+            for _, (_, _, _, n, *_), room in rt.launches_of("k_eos_guess"):
+                assert room[8] >= 4 * n
+    assert rt.violations() == 0 and rt.used() == 0
+
+
+@pytest.mark.parametrize("case", ["bubble", "hydro", "mhd"])
+def test_calls_after_a_refused_allocation(rt, case):
+    """The table, the upload and the host pipeline with each of their allocations refused in turn: the call
+    fails and succeeds when it is made again, and nothing is left when the context goes."""
+    from phlegethon_b200.abi import Simulation, PhlError
+    cfg, h = problem(case)
+    cfg = cfg.replace(precision="fp32_split")
+    rt.watch("k_unpack", "PPiiiiiiiiiiP")
+
+    def code(call):
+        try:
+            call()
+            return 0
+        except PhlError as e:
+            return e.code
+    k = 0
+    while True:  # contexts whose initialisation is refused leave nothing behind
+        rt.refuse(k)
+        try:
+            sim = Simulation(cfg, tiny_table(cfg) if cfg.helmholtz else None)
+            break
+        except PhlError as e:
+            assert e.code == -2 and k < 100
+        rt.refuse(-1)
+        gc.collect()
+        k += 1
+    rt.refuse(-1)
+    with sim:
+        if cfg.helmholtz:
+            assert each_refusal(rt, lambda: code(lambda: sim.load_helm_table(*tiny_table(cfg))), lambda: None) == 0
+        assert each_refusal(rt, lambda: code(lambda: sim.upload(h)), lambda: None) > 0
+        sim.init_thermo()
+        sim.compute_hyperbolic_dt()
+        assert each_refusal(rt, lambda: code(lambda: sim.time_loop_host_async(h, 1)), sim.wait_host) > 0
+        sim.wait_host()
+        sim.time_loop(1)
+        sim.download(h.copy())
+        k_unpack_fits(rt)
+    assert rt.violations() == 0 and rt.used() == 0
