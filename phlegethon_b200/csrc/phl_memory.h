@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
+#include <functional>
 #include <string>
 #include <unordered_map>
 
@@ -13,11 +14,17 @@ namespace phl {
 struct DeviceMemory {
   std::unordered_map<void *, size_t> blocks;
   std::string error;  // of the last allocation that failed
+  // gives up a block that the context can do without; false: there is none (any more)
+  std::function<bool()> give_up;
 
   // a block of its own, or nullptr; the failed allocation is no error of the calls that follow
   void *get(size_t bytes) {
     void *p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && give_up && give_up()) {
+      cudaGetLastError();
+      e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       error = std::string("cudaMalloc: ") + cudaGetErrorString(e);

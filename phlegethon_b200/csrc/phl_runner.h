@@ -11,6 +11,9 @@ struct Runner {
   virtual ~Runner() {}
   // one RK stage (all kernels of the stage)
   virtual void stage(const Prm &P, cudaStream_t s) = 0;
+  // split path only: whether its stages on this grid use the face fluxes (Prm::fflux); a hydro stage
+  // runs without them too
+  virtual bool face_fluxes(const Geo &) const { return true; }
   // FP64 runners (phl_runtime.cu) only: the standalone CFL maximum over the FP64 primitive
   // state and the step-0 thermodynamics.  A split-precision context runs these two through the
   // FP64 runner of its option set, so each of these kernels is compiled once, with the FP64

@@ -238,7 +238,7 @@ struct phl_ctx {
   double *eq_rho_f[3] = {}, *eq_p_f[3] = {}, *eq_ge_f[3] = {}, *phi_f[3] = {};
   float *sf_bg[3] = {};  // split path
   float *bccf = nullptr, *femf[3] = {}, *fsgn[3] = {}, *fcor[3] = {};                // split MHD
-  float *fflux[3] = {};
+  float *fflux[3] = {}, *spare_flux = nullptr;  // spare_flux: their block, where a stage can do without
   float *fecell = nullptr;                                                             // split MHD
   float *mlp_feat = nullptr, *mlp_out = nullptr;  // learned guess in the split MHD step
   unsigned *rescue_q = nullptr;                    // PHL_GUESS_MLP_RESCUE queue (count + cells)
@@ -446,6 +446,16 @@ struct phl_ctx {
       if (hydro_graph[p]) { cudaGraphExecDestroy(hydro_graph[p]); hydro_graph[p] = nullptr; }
     }
   }
+  // the split hydro form's face fluxes, given back for an allocation that found no room: the stages run
+  // in the one kernel that needs none from here on
+  bool give_up_fluxes() {
+    if (!spare_flux) return false;
+    cudaStreamSynchronize(stream);
+    drop_graphs();
+    for (float *&f : fflux) f = nullptr;
+    mem.put(&spare_flux);
+    return true;
+  }
   // hydro_step: all RK stages starting from W[cur]
   void launch_stages() {
     for (int s = 0; s < cfg.rk_stages; ++s) runner->stage(prm(s), stream);
@@ -453,19 +463,27 @@ struct phl_ctx {
   // one time_loop iteration as a CUDA graph (captured on first use per W parity): tmax clamp,
   // the RK stages, time += dt, the next dt
   template <class Body>
+  int make_graph(cudaGraphExec_t &g, Body body) {
+    cudaGraph_t gph;
+    CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    body();
+    CK(cudaStreamEndCapture(stream, &gph));
+    cudaError_t e = cudaGraphInstantiate(&g, gph, 0);
+    cudaGraphDestroy(gph);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      g = nullptr;
+      g_last_error = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
+      return PHL_E_CUDA;
+    }
+    return PHL_OK;
+  }
+  template <class Body>
   int run_graph(cudaGraphExec_t &g, Body body) {
     if (!g) {
-      cudaGraph_t gph;
-      CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      body();
-      CK(cudaStreamEndCapture(stream, &gph));
-      cudaError_t e = cudaGraphInstantiate(&g, gph, 0);
-      cudaGraphDestroy(gph);
-      if (e != cudaSuccess) {
-        g = nullptr;
-        g_last_error = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
-        return PHL_E_CUDA;
-      }
+      int rc = make_graph(g, body);
+      if (rc && give_up_fluxes()) rc = make_graph(g, body);
+      if (rc) return rc;
     }
     CK(cudaGraphLaunch(g, stream));
     return PHL_OK;
@@ -708,21 +726,23 @@ int phl_init(const phl_config *cfg, phl_ctx **out) {
       }
     }
   }
-  // face fluxes, FP64 or FP32.  The split hydro form can do without (its one-kernel stage solves the
-  // faces in place): a domain that leaves no room for them still runs
+  // Face fluxes, FP64 or FP32.  The split hydro form can do without (its one-kernel stage solves the
+  // faces in place): it has none on grids that run that kernel anyway, and a domain that leaves no room for
+  // them, now or when a later call of the context allocates, still runs.
   if (!c->split) {
     for (int d = 0; d < cfg->sdims; ++d)
       if ((rc = c->alloc(&c->dflux[d], (size_t)nv * c->nfaces(d)))) return rc;
-  } else {
+  } else if (c->runner->face_fluxes(g)) {
     size_t off[4] = {0, 0, 0, 0};  // in floats, each direction on 256 bytes
     for (int d = 0; d < 3; ++d)
       off[d + 1] = off[d] + (d < cfg->sdims ? ((size_t)nv * c->nfaces(d) + 63) / 64 * 64 : 0);
     float *all = nullptr;
-    if ((rc = c->alloc(&all, off[3]))) {
-      if (mhd) return rc;
-      cudaGetLastError();  // the failed allocation is no error of the calls that follow
-    }
+    if ((rc = c->alloc(&all, off[3])) && mhd) return rc;
     for (int d = 0; d < cfg->sdims && all; ++d) c->fflux[d] = all + off[d];
+    if (!mhd) {
+      c->spare_flux = all;
+      c->mem.give_up = [ctx = c.get()] { return ctx->give_up_fluxes(); };
+    }
   }
   if ((rc = c->alloc(&c->scal, 8))) return rc;
   if ((rc = c->alloc(&c->smax_bits, 1))) return rc;

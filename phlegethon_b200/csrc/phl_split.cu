@@ -1532,7 +1532,7 @@ __global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_split(Prm P) {
 
 // A whole hydro stage in one kernel, one thread per cell: every face is solved by both of its cells,
 // nothing goes through memory but the state.  On small grids, whose kernels are all latency, one
-// launch beats the face kernels and cons->prim (SplitRunnerT::one_kernel has the line).
+// launch beats the face kernels and cons->prim (SplitRunnerT::face_fluxes has the line).
 template <class C>
 __global__ void __launch_bounds__(C2P_BLOCK) k_stage_split(Prm P) {
   if (!*P.active) return;
@@ -1832,18 +1832,17 @@ struct SplitRunnerT : Runner {
     const char *e = getenv("PHL_STAGE_KERNEL");
     return e && strcmp(e, "cell") == 0 ? 1 : (e && strcmp(e, "faces") == 0 ? 2 : 0);
   }();
-  bool one_kernel(const Prm &P) const {
-    const Geo &g = P.g;
-    if (!P.fflux[0]) return true;  // no room for the face fluxes
-    if (stage_kind) return stage_kind == 1;
-    return g.N < (C::DIM == 3 ? 220000 : 430000);
+  bool face_fluxes(const Geo &g) const override {
+    if (C::MHD) return true;
+    if (stage_kind) return stage_kind == 2;
+    return g.N >= (C::DIM == 3 ? 220000 : 430000);
   }
   void stage(const Prm &P, cudaStream_t s) override {
     if constexpr (C::SF) {
       k_sf_mark_split<C><<<nblk(sf_mark_cells<C>(P.g), 256), 256, 0, s>>>(P);
       k_sf_flag<C><<<nblk(sf_flag_cells<C>(P.g), 256), 256, 0, s>>>(P);
     }
-    if (!C::MHD && one_kernel(P)) {
+    if (!C::MHD && !P.fflux[0]) {  // small grid, or no room for the face fluxes
       if constexpr (!C::MHD) k_stage_split<C><<<nblk(P.g.N, C2P_BLOCK), C2P_BLOCK, 0, s>>>(P);
     } else {
       const Geo &g = P.g;

@@ -14,8 +14,8 @@ enum { MAXB = 4096, MAXK = 8192, MAXW = 32, MAXLOG = 65536, MAXARG = 24 };
 
 static struct { char *p; size_t n; int live; } blk[MAXB];
 static int nblk;
-static size_t used, room = (size_t)1 << 40;
-static long refuse_at = -1, mallocs, violations, instantiations, graph_refused;
+static size_t used, most, room = (size_t)1 << 40;
+static long refuse_at = -1, mallocs, violations, instantiations;
 static int refuse_graphs;
 static cudaError_t last;
 long long fake_extent(const void *p);
@@ -31,18 +31,19 @@ static int capturing;
 
 /* ---- control, called by the tests */
 void fake_reset(void) {
-  nlog = nlaunch = ncaptured = violations = mallocs = instantiations = graph_refused = 0;
+  nlog = nlaunch = ncaptured = violations = mallocs = instantiations = 0;
   refuse_at = -1;
   refuse_graphs = 0;
   last = cudaSuccess;
   room = (size_t)1 << 40;
-  used = 0;
+  used = most = 0;
   for (int b = 0; b < nblk; ++b) blk[b].live = 0;  /* what an earlier test left */
 }
 void fake_room(size_t bytes) { room = bytes; }           /* capacity of the device */
 size_t fake_used(void) { return used; }
+size_t fake_peak(void) { return most; }
 void fake_refuse(long k) { refuse_at = k < 0 ? -1 : mallocs + k; }  /* refuse the k-th allocation from now */
-void fake_refuse_graphs(int on) { refuse_graphs = on; }
+void fake_refuse_graphs(int n) { refuse_graphs = n; }  /* the next n instantiations */
 long fake_violations(void) { return violations; }
 long fake_instantiations(void) { return instantiations; }
 long fake_launches(void) { return nlaunch; }
@@ -133,6 +134,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   if (!q) return set(cudaErrorMemoryAllocation);
   blk[nblk].p = q; blk[nblk].n = n; blk[nblk++].live = 1;
   used += n;
+  if (used > most) most = used;
   *p = q;
   return cudaSuccess;
 }
@@ -213,7 +215,7 @@ cudaError_t cudaGraphDestroy(cudaGraph_t g) { free(g); return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t g, unsigned long long f) {
   (void)g; (void)f;
   *e = NULL;
-  if (refuse_graphs) { ++graph_refused; return set(cudaErrorMemoryAllocation); }
+  if (refuse_graphs > 0) { --refuse_graphs; return set(cudaErrorMemoryAllocation); }
   ++instantiations;
   *e = malloc(8);
   return cudaSuccess;

@@ -249,3 +249,115 @@ def test_calls_after_a_refused_allocation(rt, case):
         sim.download(h.copy())
         k_unpack_fits(rt)
     assert rt.violations() == 0 and rt.used() == 0
+
+
+# ------------------------------------------------------------------ face fluxes of the split hydro form
+def hydro_calls(cfg, h):
+    """Every call of a context that allocates, and steps before and after."""
+    with started(cfg, h) as sim:
+        sim.time_loop(2)
+        sim.time_loop_host_async(h.copy(), 1)
+        sim.wait_host()
+        for _ in range(12):
+            sim.hydro_step()
+            sim.compute_hyperbolic_dt()
+        n = 64
+        a = [np.ones(n) for _ in range(7)]
+        if cfg.helmholtz:
+            assert sim.lib.phl_mlp_train(sim.ctx, 256, 1, 1, 64, 1e-3, None) == 0
+            assert sim.lib.phl_eos_invert_batch(sim.ctx, n, *[x.ctypes.data for x in a], None, 1) == 0
+        sim.time_loop(2)
+        sim.download(h.copy())
+
+
+def faces(cfg):
+    return [cfg.n_cells // n * (n + 1) for n in (cfg.nx1, cfg.nx2, cfg.nx3)[:cfg.sdims]]
+
+
+def stage_kernels(rt):
+    return {k: len(rt.launches_of(k)) for k in ("k_stage_split", "k_face_split")}
+
+
+def watch_stages(rt):
+    rt.watch("k_stage_split", "s")
+    rt.watch("k_face_split", "s")  # walks and rows as well
+
+
+@pytest.mark.parametrize("case", ["bubble", "hydro"])
+def test_no_call_fails_for_the_face_fluxes(rt, monkeypatch, case):
+    """A domain runs on a device that has room for it without the face fluxes, whether they fit at first or
+    not: they are given back when another allocation finds no room."""
+    cfg, h = problem(case)
+    cfg = cfg.replace(precision="fp32_split")
+    monkeypatch.setenv("PHL_STAGE_KERNEL", "faces")
+    hydro_calls(cfg, h)
+    with_fluxes = rt.peak()
+    without = with_fluxes - sum(4 * ((cfg.nvars * n + 63) // 64 * 64) for n in faces(cfg))
+    watch_stages(rt)
+    kinds = set()
+    for room in np.linspace(without, with_fluxes, 9).astype(int):
+        rt.reset()
+        rt.room(int(room))
+        hydro_calls(cfg, h)
+        assert rt.violations() == 0 and rt.used() == 0
+        n = stage_kernels(rt)
+        kinds.add((n["k_stage_split"] > 0, n["k_face_split"] > 0))
+    # room until a later call, room to the end
+    assert kinds == {(True, True), (False, True)}
+
+
+def test_refused_face_fluxes(rt, monkeypatch):
+    """phl_init with each allocation refused: fails, or (the face fluxes, or one after them) goes on without."""
+    from phlegethon_b200.abi import PhlError, Simulation
+    cfg, h = problem("bubble")
+    cfg = cfg.replace(precision="fp32_split")
+    monkeypatch.setenv("PHL_STAGE_KERNEL", "faces")
+    watch_stages(rt)
+    went_on = 0
+    for k in range(40):
+        rt.reset()
+        rt.refuse(k)
+        try:
+            sim = Simulation(cfg)
+        except PhlError as e:
+            assert e.code == -2
+            continue
+        refused = rt.mallocs() > k
+        rt.refuse(-1)
+        with sim:
+            sim.upload(h)
+            sim.init_thermo()
+            sim.compute_hyperbolic_dt()
+            sim.time_loop(1)
+        n = stage_kernels(rt)
+        assert (n["k_stage_split"] > 0) == refused and (n["k_face_split"] > 0) == (not refused)
+        went_on += refused
+        if not refused:
+            break
+    assert went_on > 1
+
+
+def test_small_grids_hold_no_face_fluxes(rt, monkeypatch):
+    """A grid whose hydro stages run in one kernel has no use for the face fluxes."""
+    cfg, h = problem("hydro")
+    cfg = cfg.replace(precision="fp32_split")
+    used = {}
+    for kind in ("auto", "cell", "faces"):
+        monkeypatch.setenv("PHL_STAGE_KERNEL", kind)
+        with started(cfg, h):
+            used[kind] = rt.used()
+    assert used["auto"] == used["cell"]
+    assert used["faces"] >= used["cell"] + 4 * cfg.nvars * sum(faces(cfg))
+
+
+def test_refused_graph_gives_the_face_fluxes_back(rt, monkeypatch):
+    """No room for a step graph: the face fluxes make some."""
+    cfg, h = problem("hydro")
+    monkeypatch.setenv("PHL_STAGE_KERNEL", "faces")
+    watch_stages(rt)
+    with started(cfg.replace(precision="fp32_split"), h) as sim:
+        before = rt.used()
+        rt.refuse_graphs(1)  # the next one only
+        sim.time_loop(1)
+        assert rt.used() < before
+        assert stage_kernels(rt)["k_stage_split"] == 3
