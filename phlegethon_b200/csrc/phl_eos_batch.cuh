@@ -260,6 +260,7 @@ struct EosBatch {
     if (guess < 0 || guess > 2) return -1;
     if (guess == PHL_GUESS_MLP && !mlp.ready) return -4;
     if (n == 0) return 0;
+    if (guess == PHL_GUESS_MLP && mlp.refresh(s)) return -2;
     if (guess == PHL_GUESS_MLP && !(mem->grow(&queue, (size_t)n + 1) && mem->grow(&lT, (size_t)n))) return -2;
     if (eos_launch(h, s, n, rho, e, abar, zbar, T, p, cs, iters, guess, mlp, stat, queue, lT, sm_count()))
       return -2;

@@ -481,6 +481,7 @@ static __global__ void __launch_bounds__(128) k_mlp_infer(const __grid_constant_
 struct Mlp {
   bool ready = false;
   MlpSmall small;  // host copy of the FP32 layers of params, an argument of the inference kernels
+  bool small_ok = false;  // it is the copy of what params holds now
   MlpRange range;
   float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *partial = nullptr, *lossp = nullptr;
   float *feat = nullptr, *target = nullptr;
@@ -505,11 +506,25 @@ struct Mlp {
   }
   int set(cudaStream_t s, const float *h) {
     if (alloc()) return -2;
+    small_ok = false;
     if (cudaMemcpyAsync(params, h, sizeof(float) * MLP_NPARAM, cudaMemcpyHostToDevice, s) != cudaSuccess) return -2;
     k_mlp_to_bf16<<<(MLP_H * MLP_H + 255) / 256, 256, 0, s>>>(params, w2bf);
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
     mlp_small_from_params(h, small);
-    ready = true;
+    ready = small_ok = true;
+    return 0;
+  }
+  // the host copy of the FP32 layers, read back where a call that changed the parameters failed before it
+  // could; every launch that takes `small` comes after this
+  int refresh(cudaStream_t s) {
+    if (small_ok) return 0;
+    float host[MLP_NPARAM];
+    if (get(s, host)) {  // waits for the stream
+      cudaGetLastError();  // reported here, no error of the calls that follow
+      return -2;
+    }
+    mlp_small_from_params(host, small);
+    small_ok = true;
     return 0;
   }
   int get(cudaStream_t s, float *h) {
@@ -545,6 +560,7 @@ struct Mlp {
     if (cudaFuncSetAttribute(k_mlp_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(MlpTrainSmem)) != cudaSuccess)
       return -2;
+    small_ok = false;  // until the parameters that the updates leave have been read back
     k_mlp_make_samples<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(h, n, seed, range, feat, target);
     if (!ready) {
       k_mlp_init<<<(MLP_NPARAM + 255) / 256, 256, 0, s>>>(params, seed ^ 0xABCDEFull);
@@ -571,9 +587,7 @@ struct Mlp {
     if (final_loss) {
       if (gradient(s, 0, batch, final_loss)) return -2;
     }
-    float host[MLP_NPARAM];
-    if (get(s, host)) return -2;  // waits for the stream
-    mlp_small_from_params(host, small);
+    if (refresh(s)) return -2;
     ready = true;
     return 0;
   }
@@ -595,6 +609,7 @@ struct Mlp {
   int infer(cudaStream_t s, long long n, const float *f, float *o, unsigned long long *stalled) {
     if (!ready) return -4;
     if (n == 0) return 0;
+    if (refresh(s)) return -2;
     k_mlp_infer<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(small, w2bf, n, f, o, stalled);
     if (cudaGetLastError() != cudaSuccess) return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;

@@ -1036,6 +1036,10 @@ static int ready(phl_ctx *ctx, bool step = false) {
     g_last_error = "eos_guess = PHL_GUESS_MLP: train the network (phl_mlp_train) or set its parameters first";
     return PHL_E_STATE;
   }
+  if (step && ctx->eos.mlp.ready) {
+    CK(cudaSetDevice(ctx->cfg.device));
+    if (ctx->eos.mlp.refresh(ctx->stream)) return PHL_E_CUDA;
+  }
   return PHL_OK;
 }
 
@@ -1211,6 +1215,7 @@ int phl_run_steps_host_async(phl_ctx *ctx, phl_fields *f, int nsteps) {
     if (!f->b_x[d]) return PHL_E_INVALID;
   CK(cudaSetDevice(c.device));
   int rc;
+  if (ctx->eos.mlp.ready && ctx->eos.mlp.refresh(ctx->stream)) return PHL_E_CUDA;
   if ((rc = host_pipe_setup(ctx))) return rc;
   cudaStream_t S = ctx->stream;
   double *host[phl_ctx::HOST_SLOTS] = {f->prim, f->temp, f->eint, (helm && fast) ? f->gammaf : nullptr,
@@ -1453,6 +1458,7 @@ extern "C" int phl_eos_invert_batch_noalloc(phl_ctx *ctx, long long n, const dou
   float *lT = nullptr;
   int rc = noalloc_setup(ctx->cfg.device, &buf, &ibuf, &queue, &lT);
   if (rc) return rc;
+  if (guess == PHL_GUESS_MLP && ctx->eos.mlp.refresh(ctx->stream)) return PHL_E_CUDA;
   cudaStream_t s = ctx->stream;
   const size_t M = PHL_NOALLOC_MAX_SAMPLES, b = sizeof(double) * (size_t)n;
   double *d_rho = buf, *d_e = buf + M, *d_a = buf + 2 * M, *d_z = buf + 3 * M, *d_T = buf + 4 * M;

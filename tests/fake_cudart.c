@@ -16,7 +16,7 @@ static struct { char *p; size_t n; int live; } blk[MAXB];
 static int nblk;
 static size_t used, most, room = (size_t)1 << 40;
 static long refuse_at = -1, mallocs, violations, instantiations;
-static int refuse_graphs;
+static int refuse_graphs, refuse_downloads;
 static cudaError_t last;
 long long fake_extent(const void *p);
 
@@ -33,7 +33,7 @@ static int capturing;
 void fake_reset(void) {
   nlog = nlaunch = ncaptured = violations = mallocs = instantiations = 0;
   refuse_at = -1;
-  refuse_graphs = 0;
+  refuse_graphs = refuse_downloads = 0;
   last = cudaSuccess;
   room = (size_t)1 << 40;
   used = most = 0;
@@ -44,6 +44,7 @@ size_t fake_used(void) { return used; }
 size_t fake_peak(void) { return most; }
 void fake_refuse(long k) { refuse_at = k < 0 ? -1 : mallocs + k; }  /* refuse the k-th allocation from now */
 void fake_refuse_graphs(int n) { refuse_graphs = n; }  /* the next n instantiations */
+void fake_refuse_downloads(int n) { refuse_downloads = n; }  /* the next n copies to the host */
 long fake_violations(void) { return violations; }
 long fake_instantiations(void) { return instantiations; }
 long fake_launches(void) { return nlaunch; }
@@ -155,6 +156,7 @@ cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, enum cudaMemcpyKind k, cudaStream_t st) {
   (void)st;
   int ok = 1;
+  if (k == cudaMemcpyDeviceToHost && refuse_downloads > 0) { --refuse_downloads; return set(cudaErrorUnknown); }
   if (k != cudaMemcpyDeviceToHost) ok &= inside(d, n);
   if (k != cudaMemcpyHostToDevice) ok &= inside(s, n);
   if (ok && !capturing) memmove(d, s, n);

@@ -361,3 +361,44 @@ def test_refused_graph_gives_the_face_fluxes_back(rt, monkeypatch):
         sim.time_loop(1)
         assert rt.used() < before
         assert stage_kernels(rt)["k_stage_split"] == 3
+
+
+# ------------------------------------------------------------------ the network's two copies
+def test_inference_uses_the_parameters_on_the_device(rt):
+    """A training call that changes the parameters and then fails: the FP32 layers that later launches
+    take by value are those of the device, in the batch, the inference and the step."""
+    cfg, h = problem("mhd")
+    cfg = cfg.replace(precision="fp32_split", eos_guess="mlp_rescue")
+    rt.watch("k_mlp_train_step", "PPPPPPiPP")
+    # first word of the by-value layers: W1[0]
+    rt.watch("k_eos_guess", "si")
+    rt.watch("k_mlp_infer", "i")
+    rt.watch("k_c2p_rescue", "si")
+    bits = lambda x: int(np.float32(x).view(np.int32))
+    last = lambda k: rt.launches_of(k)[-1][1][1 if k != "k_mlp_infer" else 0]
+    from phlegethon_b200.abi import Simulation
+    with Simulation(cfg, tiny_table(cfg)) as sim:
+        sim.upload(h)
+        sim.init_thermo()
+        sim.compute_hyperbolic_dt()
+        w = np.zeros(4545, np.float32)
+        w[0] = 1.0
+        assert sim.lib.phl_mlp_set_params(sim.ctx, w.ctypes.data_as(C.POINTER(C.c_float))) == 0
+        sim.time_loop(1)
+        assert last("k_c2p_rescue") == bits(1.0)
+        n = 16
+        a = [np.ones(n) for _ in range(7)]
+        feat, out = np.zeros((n, 4), np.float32), np.zeros(n, np.float32)
+        calls = (("k_eos_guess", lambda: sim.lib.phl_eos_invert_batch(sim.ctx, n, *[x.ctypes.data for x in a], None, 1)),
+                 ("k_mlp_infer", lambda: sim.lib.phl_mlp_infer_device(sim.ctx, n, feat.ctypes.data, out.ctypes.data)),
+                 ("k_c2p_rescue", lambda: sim.lib.phl_run_steps(sim.ctx, 1, np.inf, None, None)),
+                 ("k_c2p_rescue", lambda: sim.lib.phl_hydro_step(sim.ctx)))
+        for q, (kernel, call) in enumerate(calls):
+            rt.refuse_downloads(1000)
+            assert sim.lib.phl_mlp_train(sim.ctx, 256, 1, 1, 64, 1e-3, None) == -2
+            params = rt.launches_of("k_mlp_train_step")[-1][1][0]
+            C.c_float.from_address(params).value = 2.0 + q  # what the updates would have done
+            assert call() == -2  # not with layers of two networks
+            rt.refuse_downloads(0)
+            assert call() == 0
+            assert last(kernel) == bits(2.0 + q), kernel
