@@ -261,8 +261,8 @@ struct phl_ctx {
   double *stage_buf = nullptr;
   // graphs: one per parity of the W ping-pong
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  // the same of hydro_step alone, captured once a caller has made HYDRO_GRAPH_AFTER calls (a graph
-  // costs about as much to make as it saves in that many)
+  // the same of hydro_step alone, captured once a caller has made HYDRO_GRAPH_AFTER calls since the graphs
+  // were last dropped (a graph costs about as much to make as it saves in that many)
   static constexpr int HYDRO_GRAPH_AFTER = 8;
   cudaGraphExec_t hydro_graph[2] = {nullptr, nullptr};
   int hydro_calls = 0;
@@ -440,7 +440,10 @@ struct phl_ctx {
     P.gout = gam[cur];
     runner->split_to_prim(P, stream);
   }
+  // (a caller whose calls keep dropping them, like an upload with its background before every step, stays
+  // with launches instead of making a graph a step: 61 us a hydro_step of a 64^2 bubble, 132 making one)
   void drop_graphs() {
+    hydro_calls = 0;
     for (int p = 0; p < 2; ++p) {
       if (graph[p]) { cudaGraphExecDestroy(graph[p]); graph[p] = nullptr; }
       if (hydro_graph[p]) { cudaGraphExecDestroy(hydro_graph[p]); hydro_graph[p] = nullptr; }

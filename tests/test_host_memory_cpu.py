@@ -402,3 +402,18 @@ def test_inference_uses_the_parameters_on_the_device(rt):
             rt.refuse_downloads(0)
             assert call() == 0
             assert last(kernel) == bits(2.0 + q), kernel
+
+
+# ------------------------------------------------------------------ graphs of the driver's steps
+def test_hydro_step_graphs_are_made_once(rt):
+    """A graph a buffer parity after eight calls; none for a driver that uploads its whole state, background
+    included, before every step."""
+    cfg, h = problem("bubble")
+    with started(cfg, h) as sim:
+        for _ in range(30):
+            sim.hydro_step()
+        assert rt.instantiations() == 2  # three stages: the parity alternates
+        for _ in range(30):
+            sim.upload(h)
+            sim.hydro_step()
+        assert rt.instantiations() == 2
