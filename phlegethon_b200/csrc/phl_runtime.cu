@@ -502,7 +502,8 @@ struct phl_ctx {
     return PHL_OK;
   }
   // hydro_step with the current dt: launched kernel by kernel at first, as a graph for callers that
-  // keep stepping this way
+  // keep stepping this way (kernel by kernel again where there is no room for a graph: it only saves
+  // launch time)
   int launch_hydro_step() {
     auto body = [&] {
       k_set_active<<<1, 1, 0, stream>>>(active, smax_bits);
@@ -513,7 +514,10 @@ struct phl_ctx {
       body();
       CK(cudaGetLastError());
     } else if (int rc = run_graph(hydro_graph[cur], body)) {
-      return rc;
+      if (hydro_graph[cur]) return rc;
+      hydro_calls = 0;  // the next try is a few calls away
+      body();
+      CK(cudaGetLastError());
     }
     cur = (cur + cfg.rk_stages) & 1;
     return PHL_OK;

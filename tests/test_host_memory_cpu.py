@@ -417,3 +417,19 @@ def test_hydro_step_graphs_are_made_once(rt):
             sim.upload(h)
             sim.hydro_step()
         assert rt.instantiations() == 2
+
+
+def test_hydro_step_without_room_for_a_graph(rt):
+    """A driver that has given all device memory to a pool of its own: hydro_step goes on launching."""
+    cfg, h = problem("bubble")
+    rt.watch("k_c2p", "s")
+    with started(cfg, h) as sim:
+        rt.refuse_graphs(1000)
+        for _ in range(30):
+            sim.hydro_step()
+        # three stages a call; a try that failed has captured its launches as well
+        assert rt.instantiations() == 0 and len(rt.launches_of("k_c2p")) >= 3 * 30
+        rt.refuse_graphs(0)
+        for _ in range(12):
+            sim.hydro_step()
+        assert rt.instantiations() > 0
