@@ -32,11 +32,13 @@
 namespace phl {
 
 // LIM2ND slope df db / (df + db) in FP32 for differences of the same sign, else 0, without forming
-// df db (which can overflow or underflow) and without a branch: |db| / (|df| + |db|) lies in (0, 1),
-// and the 1e-37 in the sum only keeps 0 / 0 out (no difference above 1e-30 sees it).
+// df db (which can overflow or underflow) and without a branch: |db| / (|df| + |db|) lies in (0, 1).
+// The test of the sum keeps 0 / 0 out, and a NaN difference: it gives slope 0, as the reference's
+// df db > 0 does, so that a cell beside a NaN keeps finite edges.
 __device__ __forceinline__ float plm_slope_f32(float sf, float sb) {
-  const float s = sf * (fabsf(sb) * (1.0f / (fabsf(sf) + fabsf(sb) + 1e-37f)));
-  return (__float_as_int(sf) ^ __float_as_int(sb)) >= 0 ? s : 0.0f;
+  const float sum = fabsf(sf) + fabsf(sb);
+  const float s = sf * (fabsf(sb) * (1.0f / sum));
+  return (__float_as_int(sf) ^ __float_as_int(sb)) >= 0 && sum > 0.0f ? s : 0.0f;
 }
 __device__ __forceinline__ void plm_f32(float qm, float qc, float qp, float &lo, float &hi) {
   const float slope = plm_slope_f32(qp - qc, qc - qm);

@@ -80,3 +80,39 @@ def test_mhd_rows_equal_walks(gpu_lib, table, monkeypatch, case):
         h = permute_axes(h, (1, 0, 2) if case == "walls_x1" else (0, 2, 1))
     ha, hb = both(h.cfg, h, tab, monkeypatch, "PHL_FACE_KERNEL", "row", "walk")
     assert div_b_max(ha) <= 1e-13 and div_b_max(hb) <= 1e-13
+
+
+@pytest.mark.parametrize("kind", ["cell", "faces"])
+@pytest.mark.parametrize("riemann,sdims", [("hllc", 2), ("lhllc", 2), ("hllc", 3), ("hlld", 2)])
+def test_a_nan_spreads_as_in_fp64(gpu_lib, monkeypatch, riemann, sdims, kind):
+    """One cell with a NaN density: after a step the same cells hold a NaN as in the FP64 form (a NaN
+    difference limits the slope to 0, so each stage reaches the neighbouring faces' other cells only).
+    The gradients are positive along every axis: both differences at the cells beside the NaN have the
+    same sign bit."""
+    from phlegethon_b200.abi import Simulation
+    from phlegethon_b200.grid import Config, HostGrid
+    monkeypatch.setenv("PHL_STAGE_KERNEL", kind)
+    n, masks = (17, 16, 18 if sdims == 3 else 1), []
+    for form in ("fp64", "fp32_split"):
+        cfg = Config(sdims=sdims, nx1=n[0], nx2=n[1], nx3=n[2], ngc=2, nas=0, riemann=riemann, rk_stages=2,
+                     mhd=riemann == "hlld", mach_cutoff=1e-4, bc=[["periodic", "periodic"]] * 3, precision=form)
+        h = HostGrid(cfg)
+        x, y, z = h.coords()
+        h.prim[0] = 1.0 + 0.3 * x + 0.4 * y + 0.1 * z
+        h.prim[1:1 + sdims] = 0.1
+        h.prim[1 + sdims] = 1.0 + 0.2 * x + 0.1 * y + 0.1 * z
+        if cfg.mhd:
+            for d in range(sdims):
+                h.b_x[d][...] = 0.1
+        with Simulation(cfg) as sim:
+            sim.upload(h)
+            sim.init_thermo()
+            dt, smax = sim.compute_hyperbolic_dt()
+            sim.download(h)
+            h.interior(h.prim)[0, 8, 7, n[2] // 2] = np.nan
+            sim.upload(h)
+            sim.set_time(0.0, dt, smax)
+            sim.hydro_step()
+            sim.download(h)
+        masks.append(np.isnan(h.interior(h.prim)).any(axis=0))
+    assert masks[0].any() and np.array_equal(*masks), (masks[0].sum(), masks[1].sum())
