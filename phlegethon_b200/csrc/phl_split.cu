@@ -1534,9 +1534,11 @@ __global__ void __launch_bounds__(C2P_BLOCK, C::MINB_C2P32) k_c2p_split(Prm P) {
 
 // A whole hydro stage in one kernel, one thread per cell: every face is solved by both of its cells,
 // nothing goes through memory but the state.  On small grids, whose kernels are all latency, one
-// launch beats the face kernels and cons->prim (SplitRunnerT::face_fluxes has the line).
+// launch beats the face kernels and cons->prim (SplitRunnerT::face_fluxes has the line).  PPH at four
+// blocks per SM (128 registers): a 40^3 box, one wave instead of one and an eighth of three blocks,
+// 16.7 us a stage against 24.5.
 template <class C>
-__global__ void __launch_bounds__(C2P_BLOCK) k_stage_split(Prm P) {
+__global__ void __launch_bounds__(C2P_BLOCK, C::REC == REC_PPH && !C::SF ? 4 : 0) k_stage_split(Prm P) {
   if (!*P.active) return;
   constexpr int NV = C::NV, DIM = C::DIM, SW = C::SW, NS = 2 * SW + 1;
   const Geo &g = P.g;
@@ -1825,11 +1827,33 @@ struct SplitRunnerT : Runner {
     const char *e = getenv("PHL_FACE_KERNEL");
     return e && strcmp(e, "walk") == 0;
   }();
-  // A hydro stage in one per-cell kernel on grids of up to about one and a half (3D) or three (2D)
-  // waves of its blocks; with more cells the face kernels, which solve each face once, pay for their
-  // launches.  us per stage, one kernel / face kernels: Helmholtz box 20^3 21 / 32, 32^3 22 / 33, 48^3
-  // 34 / 40, 150x101x70 201 / 162; hot bubble 64^2 9 / 15, 400^2 16 / 19, 700^2 32 / 31, 1024^2 68 / 61.
-  // PHL_STAGE_KERNEL=cell / =faces select one of them on any grid (comparisons).
+  // A hydro stage in one per-cell kernel on grids of up to ONE_KERNEL_WAVES waves of its blocks; with
+  // more cells the face kernels, which solve each face once, pay for their launches.  A wave is 38,000
+  // cells (without USE_FASTEOS, 254 registers) to 152,000 (2D ideal gas, 64).  Three waves, but one where a
+  // cell's edges cost more than its solver (LIM5TH, and PPH with its flattened edges), since a cell's are
+  // formed four times here and twice there.  us per stage, one kernel / face kernels, the last size
+  // below and the first above the line (a few percent between the two forms on either side of it):
+  //   3D Helmholtz FASTEOS LHLLC 60^3 42.5 / 43.1, 62^3 49.6 / 46.1; HLLC 60^3 43.1 / 43.4, 62^3 51.5 / 46.3
+  //   without FASTEOS LHLLC      48^3 155 / 170,   50^3 193 / 179
+  //   PPH                        60^3 40.9 / 41.9, 62^3 48.6 / 45.2
+  //   LIM5TH                     38^3 22.1 / 25.8, 40^3 39.8 / 28.2
+  //   PLM flattened              52^3 46.0 / 46.0, 56^3 55.6 / 49.5; PPH flattened 38^3 28.4 / 31.6, 40^3 41.0 / 32.4
+  //   3D ideal gas LHLLC         70^3 33.0 / 33.9, 74^3 38.7 / 35.3
+  //   2D ideal gas LHLLC         640^2 23.2 / 22.6; bubble 624^2 24.8 / 24.1, 640^2 26.0 / 24.9
+  //   2D Helmholtz               528^2 36.6 / 36.7, 544^2 41.3 / 38.9; 2D flattened 576^2 32.1 / 32.2, 600^2 34.5 / 33.4
+  // PHL_STAGE_KERNEL=cell / =faces select one of the forms on any grid (comparisons).
+  static constexpr int ONE_KERNEL_WAVES = C::REC == REC_LIM2ND || (C::REC == REC_PPH && !C::SF) ? 3 : 1;
+  static long long one_kernel_cells() {
+    int dev = 0, sms = 0, blocks = 0;
+    if constexpr (!C::MHD) {
+      if (cudaGetDevice(&dev) != cudaSuccess ||
+          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, (const void *)k_stage_split<C>, C2P_BLOCK, 0) !=
+              cudaSuccess)
+        return 0;
+    }
+    return (long long)ONE_KERNEL_WAVES * blocks * sms * C2P_BLOCK;
+  }
   const int stage_kind = [] {
     const char *e = getenv("PHL_STAGE_KERNEL");
     return e && strcmp(e, "cell") == 0 ? 1 : (e && strcmp(e, "faces") == 0 ? 2 : 0);
@@ -1837,7 +1861,7 @@ struct SplitRunnerT : Runner {
   bool face_fluxes(const Geo &g) const override {
     if (C::MHD) return true;
     if (stage_kind) return stage_kind == 2;
-    return g.N >= (C::DIM == 3 ? 220000 : 430000);
+    return g.N > one_kernel_cells();
   }
   void stage(const Prm &P, cudaStream_t s) override {
     if constexpr (C::SF) {

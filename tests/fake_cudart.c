@@ -2,8 +2,8 @@
  * objects in place of libcudart.  Device memory is host memory that starts as zeros; copies and
  * memsets really happen, and any that leaves a live block is counted and skipped.  Kernels do not run:
  * a launch is logged, with the argument values of the kernels the test watches.  Allocations and graph
- * instantiations can be refused.  Freed blocks are never handed out again, so an address tells which
- * allocation it came from. */
+ * instantiations can be refused.  Freed blocks are not handed out again before a reset, so an address
+ * tells which allocation it came from. */
 #include <cuda_runtime_api.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -16,12 +16,14 @@ static struct { char *p; size_t n; int live; } blk[MAXB];
 static int nblk;
 static size_t used, most, room = (size_t)1 << 40;
 static long refuse_at = -1, mallocs, violations, instantiations;
-static int refuse_graphs, refuse_downloads;
+static int refuse_graphs, refuse_downloads, blocks_per_sm = 4;
 static cudaError_t last;
 long long fake_extent(const void *p);
 
 static struct { const void *f; char name[256]; } kern[MAXK];
 static int nkern;
+static struct { const void *host; size_t n; char *dev; } var[64];
+static int nvar;
 static struct { char part[64]; char sig[MAXARG + 1]; } watch[MAXW];
 static int nwatch;
 struct launch { int watch, captured; unsigned grid; long long a[MAXARG], room[MAXARG]; };
@@ -34,10 +36,12 @@ void fake_reset(void) {
   nlog = nlaunch = ncaptured = violations = mallocs = instantiations = 0;
   refuse_at = -1;
   refuse_graphs = refuse_downloads = 0;
+  blocks_per_sm = 4;
   last = cudaSuccess;
   room = (size_t)1 << 40;
   used = most = 0;
-  for (int b = 0; b < nblk; ++b) blk[b].live = 0;  /* what an earlier test left */
+  for (int b = 0; b < nblk; ++b) free(blk[b].p);  /* freed ones and what an earlier test left */
+  nblk = 0;
 }
 void fake_room(size_t bytes) { room = bytes; }           /* capacity of the device */
 size_t fake_used(void) { return used; }
@@ -45,6 +49,7 @@ size_t fake_peak(void) { return most; }
 void fake_refuse(long k) { refuse_at = k < 0 ? -1 : mallocs + k; }  /* refuse the k-th allocation from now */
 void fake_refuse_graphs(int n) { refuse_graphs = n; }  /* the next n instantiations */
 void fake_refuse_downloads(int n) { refuse_downloads = n; }  /* the next n copies to the host */
+void fake_blocks_per_sm(int n) { blocks_per_sm = n; }
 long fake_violations(void) { return violations; }
 long fake_instantiations(void) { return instantiations; }
 long fake_launches(void) { return nlaunch; }
@@ -66,6 +71,9 @@ long long fake_extent(const void *p) {
   for (int b = 0; b < nblk; ++b)
     if (blk[b].live && (const char *)p >= blk[b].p && (const char *)p < blk[b].p + blk[b].n)
       return blk[b].p + blk[b].n - (const char *)p;
+  for (int v = 0; v < nvar; ++v)
+    if (var[v].dev && (const char *)p >= var[v].dev && (const char *)p < var[v].dev + var[v].n)
+      return var[v].dev + var[v].n - (const char *)p;
   return -1;
 }
 static int inside(const void *p, size_t n) {
@@ -87,8 +95,6 @@ void __cudaRegisterFunction(void **h, const char *f, char *df, const char *name,
     snprintf(kern[nkern++].name, sizeof kern[0].name, "%s", name);
   }
 }
-static struct { const void *host; size_t n; void *dev; } var[64];
-static int nvar;
 void __cudaRegisterVar(void **h, char *host, char *dev, const char *name, int ext, size_t size, int constant, int global) {
   (void)h; (void)dev; (void)name; (void)ext; (void)constant; (void)global;
   if (nvar < 64) { var[nvar].host = host; var[nvar++].n = size; }
@@ -184,12 +190,7 @@ cudaError_t cudaMemcpy3DAsync(const struct cudaMemcpy3DParms *p, cudaStream_t st
 cudaError_t cudaGetSymbolAddress(void **p, const void *sym) {
   for (int v = 0; v < nvar; ++v)
     if (var[v].host == sym) {
-      size_t u = used;
-      if (!var[v].dev) {
-        blk[nblk].p = var[v].dev = calloc(1, var[v].n);
-        blk[nblk].n = var[v].n; blk[nblk++].live = 1;
-      }
-      used = u;
+      if (!var[v].dev) var[v].dev = calloc(1, var[v].n);
       *p = var[v].dev;
       return cudaSuccess;
     }
@@ -202,6 +203,7 @@ cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { (void)d; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) { (void)a; (void)d; *v = 148; return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v) { (void)f; (void)a; (void)v; return cudaSuccess; }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *f, int b, size_t s) { (void)f; (void)b; (void)s; *n = blocks_per_sm; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { cudaError_t e = last; last = cudaSuccess; return e; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { (void)f; *s = malloc(8); return cudaSuccess; }

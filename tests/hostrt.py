@@ -19,7 +19,7 @@ class FakeRuntime:
         self.lib = C.CDLL(path)
         for name, args, res in (("room", [C.c_size_t], None), ("used", [], C.c_size_t), ("peak", [], C.c_size_t), ("refuse", [C.c_long], None),
                                 ("refuse_graphs", [C.c_int], None), ("refuse_downloads", [C.c_int], None),
-                                ("violations", [], C.c_long),
+                                ("blocks_per_sm", [C.c_int], None), ("violations", [], C.c_long),
                                 ("instantiations", [], C.c_long), ("launches", [], C.c_long), ("mallocs", [], C.c_long),
                                 ("watch", [C.c_char_p, C.c_char_p], C.c_int), ("log", [], C.c_long),
                                 ("log_watch", [C.c_long], C.c_int), ("log_grid", [C.c_long], C.c_uint),

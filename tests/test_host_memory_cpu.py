@@ -350,6 +350,28 @@ def test_small_grids_hold_no_face_fluxes(rt, monkeypatch):
     assert used["faces"] >= used["cell"] + 4 * cfg.nvars * sum(faces(cfg))
 
 
+@pytest.mark.parametrize("case,below,above", [("bubble", 237, 239), ("lim2nd", 38, 39), ("pph", 38, 39),
+                                              ("lim5th", 26, 27), ("sf", 38, 39), ("sf_pph", 26, 27), ("given", 38, 39)])
+def test_one_kernel_line_is_in_waves(rt, case, below, above):
+    """Hydro stages run in one kernel up to three waves of its blocks (one for LIM5TH and flattened PPH): here of
+    one block of 128 cells on each of 148 SMs."""
+    waves = 1 if case in ("lim5th", "sf_pph") else 3
+    watch_stages(rt)
+    for n in (below, above):
+        if case == "bubble":
+            cfg, h = problems.hot_bubble_2d(n)
+        else:
+            cfg, h = problems.stratified_3d(n, rec=case[-3:] if "pph" in case else case if case == "lim5th" else "lim2nd",
+                                            shock_flattening=case.startswith("sf"), fasteos=case != "given")
+        assert (cfg.n_cells <= waves * 148 * 128) == (n == below)
+        rt.reset()
+        rt.blocks_per_sm(1)
+        with started(cfg.replace(precision="fp32_split"), h) as sim:
+            sim.time_loop(1)
+        k = stage_kernels(rt)
+        assert (k["k_stage_split"] > 0, k["k_face_split"] > 0) == (n == below, n == above), n
+
+
 def test_refused_graph_gives_the_face_fluxes_back(rt, monkeypatch):
     """No room for a step graph: the face fluxes make some."""
     cfg, h = problem("hydro")
