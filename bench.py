@@ -76,30 +76,10 @@ def default_size(name):
     return {"stratified": 256, "stratified_mhd": 256, "hot_bubble": 256, "orszag_tang": 1024}[name]
 
 
-def stage_kernels(cfg, form, guess="warm"):
-    """The parts of a stage that the traffic model below counts, and their number in one step with
-    every direction and axis a part of its own (plus k_pre_step and k_post_step).  What one launch
-    covers is step_launches' business."""
-    s = cfg.rk_stages
-    if cfg.mhd:
-        nax = 3 if cfg.sdims == 3 else 1
-        if form == "fp32_split":
-            per = cfg.sdims + nax + cfg.sdims + 1 + (1 if guess == "mlp_rescue" else 0)
-            names = "k_face_split_mhd + k_corner_split + k_bface_split + k_c2p_mhd_split"
-        else:
-            per = cfg.sdims + nax + cfg.sdims + 1
-            names = "k_face + k_corner + k_bface + k_c2p"
-        return names + " (one MHD stage)", s * per + 2
-    if form == "fp32_split":
-        tiled = cfg.sdims == 3 and cfg.nx1 % 32 == 0 and cfg.nx2 % 8 == 0 and cfg.nx3 % 16 == 0
-        return ("k_stage_split_tiled" if tiled else "k_stage_split") + " (FP32 fluxes, FP64 state/EoS)", s + 2
-    return "k_face + k_c2p (FP64)", s * (cfg.sdims + 1) + 2
-
-
-def step_launches(cfg, form, guess="warm"):
+def step_launches(cfg, form, guess="warm", one_kernel=False):
     """Name of what the per-stage timing covers, and the kernel launches of one step (the stage
     kernels plus k_pre_step and k_post_step; the learned rescue adds its queue kernel to every
-    stage)."""
+    stage).  one_kernel: the split hydro stages run in one kernel (a context without face fluxes)."""
     s = cfg.rk_stages
     if form != "fp32_split":
         if cfg.mhd:
@@ -109,15 +89,17 @@ def step_launches(cfg, form, guess="warm"):
         # faces per direction, corners, face B, cons->prim
         per = cfg.sdims + 3 + (1 if guess == "mlp_rescue" else 0)
         return "k_face_split + k_corner_split + k_bface_split + k_c2p_split (one MHD stage)", s * per + 2
-    if cfg.n_cells < (220000 if cfg.sdims == 3 else 430000):
+    if one_kernel:
         return "k_stage_split (FP32 fluxes, FP64 state/EoS)", s + 2
     return "k_face_split + k_c2p_split (one hydro stage)", s * (cfg.sdims + 1) + 2
 
 
-# DRAM bytes per cell of one stage-kernel launch, from ncu captures of the 128^3 stratified box
-# (dram__bytes_read.sum + dram__bytes_write.sum over 2,097,152 cells); the kernel streams the
-# domain once per launch, so the per-launch traffic scales with the cell count
-TRAFFIC_PER_CELL = {("stratified", "fp64"): 557.258496e6 / 2097152,
+# DRAM bytes per cell of one stage, from ncu captures of the 128^3 stratified box
+# (dram__bytes_read.sum + dram__bytes_write.sum over 2,097,152 cells); the kernels stream the
+# domain once per launch, so the traffic scales with the cell count
+TRAFFIC_PER_CELL = {# one FP64 hydro stage (a middle stage: U0 read): row faces 230.7 MB, walking x2/x3 faces
+                    # 245.8 + 245.1 MB, cons->prim 1164.2 MB
+                    ("stratified", "fp64"): (230.7e6 + 245.8e6 + 245.1e6 + 1164.2e6) / 2097152,
                     # one split hydro stage at 128^3: row and walk faces 98.5 + 97.1 + 99.1 MB,
                     # cons->prim 632.0 MB
                     ("stratified", "fp32_split"): (98.5e6 + 97.1e6 + 99.1e6 + 632.0e6) / 2097152,
@@ -126,6 +108,14 @@ TRAFFIC_PER_CELL = {("stratified", "fp64"): 557.258496e6 / 2097152,
                     # cons->prim 727.9 MB
                     ("stratified_mhd", "fp32_split"): (154.1e6 + 155.9e6 + 165.0e6 + 132.1e6 + 117.6e6
                                                        + 727.9e6) / 2097152}
+
+
+def traffic_per_cell(name, form, cells, one_kernel):
+    """DRAM bytes per cell of one stage where the captured kernels run: grids whose FP64 x2 and x3
+    faces walk (a million cells) and whose hydro stages use the face kernels; None elsewhere."""
+    if one_kernel or (form == "fp64" and cells < 1000000):
+        return None
+    return TRAFFIC_PER_CELL.get((name, form))
 
 
 # Algorithmic HBM bytes per zone-update of the workloads (minimum traffic of one step of a fused
@@ -433,6 +423,7 @@ def measure_form(args, name, cfg, h, table, form, local, dist, want_e2e, guess="
         mlp_params = np.zeros(MLP_NPARAMS, dtype=np.float32)
         assert sim.lib.phl_mlp_get_params(sim.ctx, mlp_params.ctypes.data_as(C.POINTER(C.c_float))) == 0
     sim.compute_hyperbolic_dt()
+    one_kernel = form == "fp32_split" and not cfg.mhd and not sim.device_field("flux_x1_32")
     stream = torch.cuda.ExternalStream(sim.stream(), device=torch.device("cuda", local))
     sim.time_loop(args.warmup)
     sim.reset_status()
@@ -453,7 +444,7 @@ def measure_form(args, name, cfg, h, table, form, local, dist, want_e2e, guess="
     out = h.copy()
     sim.download(out)
     res = {"form": form, "guess": guess, "ms": ms, "done": done, "clocks": clocks, "status": status, "state": out,
-           "train": train, "mlp_params": mlp_params}
+           "train": train, "mlp_params": mlp_params, "one_kernel": one_kernel}
     if not kernel_timing:
         sim.close()
         return res
@@ -761,12 +752,11 @@ def run_ours(args):
     model_bytes = step_bytes_per_cell(cfg.replace(precision=head_form))
     launch_ms = head["launch_ms"]
     achieved = bytes_per_cell * cells / cfg.rk_stages / (launch_ms * 1e-3) / 1e9
-    kname, launches_per_step = step_launches(cfg, head_form, head_guess)
-    tpc = TRAFFIC_PER_CELL.get((name, head_form))
+    kname, launches_per_step = step_launches(cfg, head_form, head_guess, head["one_kernel"])
+    tpc = traffic_per_cell(name, head_form, cells, head["one_kernel"])
     roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / peaks["hbm_gbs"], "traffic": tpc * cells if tpc else None,
-            "traffic_source": ("ncu DRAM bytes of one stage at 128^3, scaled by cells" if name == "stratified_mhd"
-                               else "ncu DRAM bytes of one launch at 128^3, scaled by cells") if tpc else None,
+            "traffic_source": "ncu DRAM bytes of one stage at 128^3, scaled by cells" if tpc else None,
             "kernel": kname, "peak_kind": peak_kind,
             "launch_ms": launch_ms, "bytes_per_zone_update": bytes_per_cell,
             "traffic_model": {"bytes_per_zone_update": model_bytes,
@@ -928,12 +918,13 @@ def eos_line(args, with_cpu=True):
             "agreement": agree,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "traffic": None, "peak_kind": peak_kind,
-                         "kernel": "k_eos_invert + k_eos_fallback",
+                         "kernel": "k_eos_guess + k_eos_invert + k_eos_fallback",
                          "note": "FP64-compute bound (EoS evaluations); HBM fraction stated for completeness"},
             "cpu_baseline": cpu,
             "e2e": {"value": n / (e2e_ms * 1e-3), "unit": "inversions/s", "h2d_bytes_per_step": 40 * n,
                     "d2h_bytes_per_step": 12 * n},
-            "gpu_launches": 2 * args.steps, "clocks": m["clocks"]}
+            # per batch: k_eos_guess, k_eos_invert, k_eos_fallback
+            "gpu_launches": 3 * args.steps, "clocks": m["clocks"]}
     return line
 
 

@@ -1351,9 +1351,11 @@ void *phl_device_field(phl_ctx *ctx, const char *name) {
   if (n == "gammaf_dev32") return ctx->gf[ctx->cur];
   if (n == "b_cc32") return ctx->bccf;
   // CT scratch of the last stage: face EMFs [3][faces] and mass-flux signs per face direction,
-  // corner EMFs per axis (FP64 form, and the FP32 arrays of the split form with suffix 32)
+  // corner EMFs per axis (FP64 form, and the FP32 arrays of the split form with suffix 32); the split
+  // form's face fluxes, NULL where its hydro stages run in one kernel
   static const char *dn[3] = {"1", "2", "3"};
   for (int d = 0; d < 3; ++d) {
+    if (n == std::string("flux_x") + dn[d] + "_32") return ctx->fflux[d];
     if (n == std::string("emf_x") + dn[d]) return ctx->emf[d];
     if (n == std::string("sign_x") + dn[d]) return ctx->sgnf[d];
     if (n == std::string("emf_corner") + dn[d]) return ctx->cor[d];

@@ -885,7 +885,7 @@ constexpr int RESCUE_BLOCKS = 4 * 148;
 // nothing between faces and needs 72 registers.  Without USE_FASTEOS, where each face runs two FP64
 // (rho, P) -> T solves, 4 (128 registers): a 256^3 MHD step took 36.9 ms against 43.4 with the
 // registers unbounded (253 registers, 2 blocks per SM), 37.5 at 3
-constexpr int WALK_MINB = 5, WALK_MINB_HYDRO = 5, WALK_MINB_GIVEN = 4, ROW_MINB = 6;
+constexpr int WALK_MINB = 5, WALK_MINB_GIVEN = 4, ROW_MINB = 6;
 
 // Raw values of one cell for the walking face kernel along D: the FP32 state (0 .. NV-1), the
 // cell B components transverse to D (NBT of them from NV on; the component along D is not
@@ -966,7 +966,7 @@ __device__ __forceinline__ void face_from_edges(const Prm &P, long long fidx, in
 // (the per-face kernel does both twice) and its edge values are carried to the next face.  The
 // faces, their arithmetic and the stored results are those of k_face_split.
 template <class C, int D, int K>
-__global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : (C::MHD ? WALK_MINB : WALK_MINB_HYDRO)) k_face_split_walk(Prm P) {
+__global__ void __launch_bounds__(128, C::EOSM == EOS_GIVEN ? WALK_MINB_GIVEN : WALK_MINB) k_face_split_walk(Prm P) {
   static_assert(C::REC == REC_LIM2ND, "the walk carries LIM2ND edge values");
   if (!*P.active) return;
   using L = WalkCell<C, D>;

@@ -82,8 +82,22 @@ def test_bench_algorithmic_bytes():
     assert bench.algorithmic_bytes_per_cell("stratified_mhd", "fp64") == 1120
     assert bench.algorithmic_bytes_per_cell("stratified", "fp32_split") == 712
     assert bench.algorithmic_bytes_per_cell("hot_bubble", "fp64") == 448
-    name, launches = bench.stage_kernels(cfgm.replace(precision="fp32_split"), "fp32_split")
-    assert "k_face_split_mhd" in name and launches == 3 * (3 + 3 + 3 + 1) + 2
+    # kernel launches of a step: three face directions, corners, face B, cons->prim per stage
+    name, launches = bench.step_launches(cfgm.replace(precision="fp32_split"), "fp32_split")
+    assert "k_c2p_split" in name and launches == 3 * (3 + 1 + 1 + 1) + 2
+    assert bench.step_launches(cfgm, "fp32_split", "mlp_rescue")[1] == launches + 3
+    assert bench.step_launches(cfg, "fp32_split")[1] == bench.step_launches(cfg, "fp64")[1] == 3 * (3 + 1) + 2
+    assert bench.step_launches(cfg, "fp32_split", one_kernel=True)[1] == 3 + 2
+    # and they name kernels that exist, as do the traffic figures' conditions
+    src = "".join(open(os.path.join(ROOT, "phlegethon_b200", "csrc", f)).read()
+                  for f in ("phl_kernels.cuh", "phl_split.cu", "phl_eos_batch.cuh"))
+    for c, form, kw in ((cfgm, "fp32_split", {}), (cfgm, "fp64", {}), (cfg, "fp32_split", {}), (cfg, "fp64", {}),
+                        (cfg, "fp32_split", {"one_kernel": True})):
+        for k in re.findall(r"k_\w+", bench.step_launches(c, form, **kw)[0]):
+            assert re.search(r"\b%s(?:_row|_walk)?\(" % k, src), k
+    assert bench.traffic_per_cell("stratified", "fp64", 1000, False) is None
+    assert bench.traffic_per_cell("stratified", "fp32_split", 1 << 21, True) is None
+    assert bench.traffic_per_cell("stratified_mhd", "fp32_split", 1 << 24, False) > 0
 
 
 def test_python_binding_matches_header_arity(lib_path):
