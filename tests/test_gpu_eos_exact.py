@@ -68,12 +68,17 @@ def test_energy_bitwise_at_and_around_the_nodes(gpu_lib):
         assert sim.lib.phl_eos_energy_device(sim.ctx, len(want), d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(),
                                              d[3].data_ptr(), e.data_ptr()) == 0
         got = e.cpu().numpy()
-    # the oracle's log10 and the device's may put a state within an ulp of a node into either cell, whose
-    # interpolants meet there to rounding; everywhere else the bits agree
-    on_node = np.abs(got - want) <= 1e-13 * np.abs(want)
+    # the oracle's log10 and the device's may put a state within a few ulp of a node into either cell,
+    # whose interpolants meet there to rounding; everywhere else the bits agree.  The logarithms, the step
+    # and the nodes' own powers are off by a few ulp of log10 x, which is x to some 1e-14
+    rho_n, T_n, _, _ = helm_table.nodes(**helm_table.X1_TABLE)
+    dist = lambda x, nodes: np.abs(x[:, None] / nodes[None, :] - 1.0).min(axis=1)
+    on_node = np.minimum(dist(s[0] * (s[3] / s[2]), rho_n), dist(s[1], T_n)) < 2e-13
     same = got.view(np.int64) == want.view(np.int64)
-    assert np.all(same | on_node)
-    assert same.mean() > 0.9
+    assert np.all(same[~on_node])
+    assert np.all(np.abs(got - want) <= 1e-13 * np.abs(want))
+    # states of both kinds: five of eight draws of T, and of rho Ye, stay off their node by 1e-12 and more
+    assert on_node.mean() > 0.5 and (~on_node).mean() > 0.3
 
 
 @pytest.mark.gpu

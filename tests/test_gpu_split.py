@@ -67,34 +67,35 @@ def test_split_keeps_hydrostatic_balance(gpu_lib, table):
 
 
 @pytest.mark.parametrize("riemann", ["lhllc", "hllc"])
-def test_tiled_stage_equals_per_cell_stage(gpu_lib, table, riemann, monkeypatch):
-    """The face-reuse tiled stage kernel (grids divisible by its 32 x 8 x 16 tile) against the
-    per-cell kernel, which solves every face twice (once per neighbour, so its two copies of a
-    face flux can differ in the last FP32 bits where the compiler contracts differently).  Both
-    sit at the same FP32 rounding distance from the FP64 form."""
+def test_face_kernels_equal_one_kernel_stage(gpu_lib, table, riemann, monkeypatch):
+    """The hydro stage through the face kernels against the one-kernel stage, which solves every face
+    twice (once per neighbour, so its two copies of a face flux can differ in the last FP32 bits where
+    the compiler contracts differently).  Both sit at the same FP32 rounding distance from the FP64
+    form."""
     cfg, h = problems.stratified_3d(32, ny=16, nz=32, riemann=riemann)
     monkeypatch.setenv("PHL_STAGE_KERNEL", "cell")
     hc, stc = run_form(cfg, h, 6, table, "fp32_split")
-    monkeypatch.setenv("PHL_STAGE_KERNEL", "auto")
-    ht, stt = run_form(cfg, h, 6, table, "fp32_split")
+    monkeypatch.setenv("PHL_STAGE_KERNEL", "faces")
+    hf, stf = run_form(cfg, h, 6, table, "fp32_split")
     h64, _ = run_form(cfg, h, 6, table, "fp64")
-    assert stt["nonfinite"] == 0 and stt["newton_nonconverged"] == 0
-    e_t = field_errors(ht, h64)
+    assert stf["nonfinite"] == 0 and stf["newton_nonconverged"] == 0
+    e_f = field_errors(hf, h64)
     e_c = field_errors(hc, h64)
-    diff = field_errors(ht, hc)
+    diff = field_errors(hf, hc)
     for f in e_c:
-        # no further from FP64 than the per-cell kernel, and apart by FP32 rounding noise only
-        assert e_t[f] <= 1.5 * e_c[f] + 1e-12, (f, e_t, e_c)
+        # no further from FP64 than the one-kernel stage, and apart by FP32 rounding noise only
+        assert e_f[f] <= 1.5 * e_c[f] + 1e-12, (f, e_f, e_c)
         assert diff[f] <= 2.0 * e_c[f] + 1e-12, (f, diff, e_c)
 
 
-def test_tiled_stage_tensor_copies_equal_cell_copies(gpu_lib, table, monkeypatch):
-    """Interior tiles stage planes with bulk tensor copies (TMA), boundary tiles cell by cell; the
-    staged data is the same, so the result equals the cell-by-cell staging bit for bit."""
-    cfg, h = problems.stratified_3d(96, ny=24, nz=32)
-    monkeypatch.setenv("PHL_STAGE_KERNEL", "tiled_cpasync")
+@pytest.mark.parametrize("n,ny,nz,kind", [(96, 24, 32, "cell"), (64, 64, 64, "faces")])
+def test_default_stage_is_the_one_its_size_selects(gpu_lib, table, monkeypatch, n, ny, nz, kind):
+    """A grid below and one above the one-kernel line: the default run is the selected form's, bit for
+    bit."""
+    cfg, h = problems.stratified_3d(n, ny=ny, nz=nz)
+    monkeypatch.setenv("PHL_STAGE_KERNEL", kind)
     ha, sta = run_form(cfg, h, 4, table, "fp32_split")
-    monkeypatch.setenv("PHL_STAGE_KERNEL", "auto")
+    monkeypatch.delenv("PHL_STAGE_KERNEL")
     hb, stb = run_form(cfg, h, 4, table, "fp32_split")
     assert stb["nonfinite"] == 0 and stb["tensor_core_stalls"] == 0
     assert stb["newton_iterations"] == sta["newton_iterations"]
@@ -311,12 +312,11 @@ def test_split_against_oracle(gpu_lib, oracle, table, family):
 
 
 @pytest.mark.parametrize("mhd_case", ["stratified_mhd", "orszag_tang"])
-def test_tiled_faces_equal_walking_faces(gpu_lib, table, mhd_case, monkeypatch):
-    """The face kernels that stage tiles in shared memory with bulk tensor copies (grids whose
-    extents are multiples of the tiles) against the walking face kernels: the same edges and the
-    same solver on the same inputs, so both sit at the same FP32 rounding distance from the FP64
-    form and apart by rounding noise only (the compiler contracts the edge arithmetic differently
-    in the two kernels)."""
+def test_row_faces_equal_walking_faces(gpu_lib, table, mhd_case, monkeypatch):
+    """The x1 faces by warp rows (the default) against the walking face kernel along x1: the same edges
+    and the same solver on the same inputs, so both sit at the same FP32 rounding distance from the FP64
+    form and apart by rounding noise only (the compiler contracts the edge arithmetic differently in the
+    two kernels)."""
     if mhd_case == "stratified_mhd":
         cfg, h = problems.stratified_3d(128, ny=16, nz=8, mhd=True)
         tab = table
@@ -325,7 +325,7 @@ def test_tiled_faces_equal_walking_faces(gpu_lib, table, mhd_case, monkeypatch):
         tab = None
     monkeypatch.setenv("PHL_FACE_KERNEL", "walk")
     ha, sta = run_form(cfg, h, 3, tab, "fp32_split")
-    monkeypatch.setenv("PHL_FACE_KERNEL", "tile")
+    monkeypatch.setenv("PHL_FACE_KERNEL", "row")
     hb, stb = run_form(cfg, h, 3, tab, "fp32_split")
     h64, _ = run_form(cfg, h, 3, tab, "fp64")
     assert stb["nonfinite"] == 0 and stb["tensor_core_stalls"] == 0

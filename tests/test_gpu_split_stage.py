@@ -3,9 +3,13 @@ x1 (29 faces each), the walks of 8 faces along x2 and x3, and the one-kernel hyd
 grids, which solves every face from both of its cells with the ghost mapping of single loads.
 
 Two kernels that do the same FP32 arithmetic sit at the same rounding distance from the FP64 form and
-apart by rounding noise only, so each must be no further from FP64 than 1.5 times the other, and the
-two no further apart than the sum of their distances.  A wrong stencil, ghost or face index moves a
-field by its own size."""
+apart by rounding noise only: each must be no further from FP64 than 1.5 times the other, and in no cell
+may the two differ, or either be off FP64, by more than a bound on that noise.  The bound: an FP32
+flux of a flow of Mach number M carries an error of a few 2^-24 M of the cell's own density, pressure,
+sound speed, temperature and B^2 in units of the pressure; a step of three stages adds some ten such
+errors a face, the few steps here not more than 100 (measured 36 between the forms and FP64, 14 between
+two kernels).  A wrong stencil, ghost or face index moves a cell by a fraction of M or of its field, 1e4
+times as much and more."""
 import numpy as np
 import pytest
 
@@ -16,11 +20,28 @@ from util import div_b_max, field_errors, permute_axes
 pytestmark = pytest.mark.gpu
 
 
+def cell_differences(ha, hb):
+    """Largest difference in any cell, in units of the cell's density, pressure, sound speed and temperature
+    (B of the pressure's root), and the rms Mach number."""
+    sd, ip = ha.cfg.sdims, 1 + ha.cfg.sdims
+    a, b = ha.interior(ha.prim), hb.interior(hb.prim)
+    d, cs = np.abs(a - b), np.sqrt(b[ip] / b[0])
+    out = {"rho": (d[0] / b[0]).max(), "p": (d[ip] / b[ip]).max(), "v": (d[1:ip] / cs).max(),
+           "e": np.abs(ha.interior(ha.eint) / hb.interior(hb.eint) - 1.0).max(),
+           "T": np.abs(ha.interior(ha.temp) / hb.interior(hb.temp) - 1.0).max()}
+    if ha.cfg.mhd:
+        out["b"] = max(np.abs(ha.bface_interior(k) - hb.bface_interior(k)).max() for k in range(sd)) / np.sqrt(b[ip].min())
+    return out, np.sqrt((b[1:ip] ** 2).sum(axis=0).mean()) / cs.mean()
+
+
 def check(ha, hb, h64):
-    ea, eb, diff = field_errors(ha, h64), field_errors(hb, h64), field_errors(ha, hb)
+    ea, eb = field_errors(ha, h64), field_errors(hb, h64)
     for f in ea:
         assert ea[f] <= 1.5 * eb[f] + 1e-12 and eb[f] <= 1.5 * ea[f] + 1e-12, (f, ea, eb)
-        assert diff[f] <= ea[f] + eb[f] + 1e-12, (f, diff, ea, eb)
+    for a, b in ((ha, hb), (ha, h64), (hb, h64)):
+        diff, mach = cell_differences(a, b)
+        for f in diff:
+            assert diff[f] <= 100 * 2.0 ** -24 * mach, (f, diff, mach)
 
 
 def both(cfg, h, table, monkeypatch, var, a, b, steps=3):
@@ -30,7 +51,8 @@ def both(cfg, h, table, monkeypatch, var, a, b, steps=3):
     hb, stb = run_form(cfg, h, steps, table, "fp32_split")
     h64, _ = run_form(cfg, h, steps, table, "fp64")
     for st in (sta, stb):
-        assert st["nonfinite"] == 0 and st["newton_calls"] in (0, steps * 3 * cfg.n_cells)
+        assert st["nonfinite"] == 0
+        assert st["newton_calls"] == (steps * 3 * cfg.n_cells if cfg.helmholtz else 0)
     check(ha, hb, h64)
     return ha, hb
 
