@@ -26,6 +26,12 @@ namespace phl {
 // 2.91 at 2 (unbounded); 10^6 samples, bracket guess 0.49 ms against 0.55 and 0.55.  The 36
 // coefficients kept in shared memory between the evaluations of a solve ran 3 to 5% slower.
 constexpr int EOS_MINB = 3;
+// Without p and cs the warm start's kernel holds no full evaluation and fits 4 blocks (128 registers, no
+// spills): 2^20 samples from a guess 0.1% off 202 us against 220 at 3 and 268 at 5 (with p and cs 320 at
+// 3, 335 at 4).
+constexpr int EOS_MINB_WARM = 4;
+// single energies: 2^20 88 us with blocks of 128, 5 per SM, against 96 with 2 blocks of 256
+constexpr int ENERGY_THREADS = 128, ENERGY_MINB = 5;
 
 // cold guess; returns the number of EoS evaluations the search used
 __device__ __forceinline__ int bracket_guess(const HelmTable &h, const HelmRho &r, HelmTemp &t, double e, double &Tg) {
@@ -49,8 +55,10 @@ __device__ __forceinline__ int bracket_guess(const HelmTable &h, const HelmRho &
   return evals;
 }
 
-__global__ void k_eos_energy(HelmTable h, long long n, const double *rho, const double *T, const double *abar,
-                             const double *zbar, double *e) {
+__global__ void __launch_bounds__(ENERGY_THREADS, ENERGY_MINB) k_eos_energy(HelmTable h, long long n,
+                                                                            const double *rho, const double *T,
+                                                                            const double *abar, const double *zbar,
+                                                                            double *e) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   e[t] = helm_given2_energy(h, rho[t], T[t], abar[t], zbar[t]);
@@ -73,11 +81,12 @@ struct EosStat {
   }
 };
 
-// outputs of one finished inversion
+// outputs of one finished inversion (OUT: p or cs among them)
+template <bool OUT>
 __device__ __forceinline__ void eos_finish(const HelmTable &h, long long t, const HelmRho &r, HelmTemp &ht,
                                            double Tg, int used, double *T, double *p, double *cs, int *iters) {
   T[t] = Tg;
-  if (p || cs) {
+  if (OUT && (p || cs)) {
     double P, E, snd, cv;
     helm_full(h, r, ht, Tg, P, E, snd, cv);
     if (p) p[t] = P;
@@ -107,16 +116,16 @@ static __global__ void __launch_bounds__(128, 8) k_eos_guess(HelmTable h, const 
   if (t < n) guess[t] = lT;
 }
 
-// Phase 1.  guess 0 / 2: warm or bracket guess and the full Newton.  LEARNED: the guess that phase 0
-// left in `lT`, judged by at most 3 reference Newton iterations; a sample whose guess did not
-// converge within them without a reset is appended to `queue` (queue[0] = count, then
-// index | judged iterations << 56) for phase 2, so that the fallback runs in converged warps
-// instead of stalling the accepted lanes.
-template <bool LEARNED>
-__global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long long n, const double *rho, const double *e,
-                                                    const double *abar, const double *zbar, double *T,
-                                                    double *p, double *cs, int *iters, int guess, const float *lT,
-                                                    unsigned long long *stat, unsigned long long *queue) {
+// Phase 1.  Warm or bracket guess: the full Newton.  Learned guess: the one that phase 0 left in `lT`,
+// judged by at most 3 reference Newton iterations; a sample whose guess did not converge within them
+// without a reset is appended to `queue` (queue[0] = count, then index | judged iterations << 56) for
+// phase 2, so that the fallback runs in converged warps instead of stalling the accepted lanes.
+template <int GUESS, bool OUT>
+__global__ void __launch_bounds__(128, GUESS == PHL_GUESS_WARM && !OUT ? EOS_MINB_WARM : EOS_MINB)
+k_eos_invert(HelmTable h, long long n, const double *rho, const double *e, const double *abar, const double *zbar,
+             double *T, double *p, double *cs, int *iters, const float *lT, unsigned long long *stat,
+             unsigned long long *queue) {
+  constexpr bool LEARNED = GUESS == PHL_GUESS_MLP;
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   EosStat st;
   bool reject = false;
@@ -137,21 +146,21 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_invert(HelmTable h, long 
         st.v[0] = 1;
         st.v[1] = used;
         st.v[4] = 1;
-        eos_finish(h, t, r, ht, Tg, used, T, p, cs, iters);
+        eos_finish<OUT>(h, t, r, ht, Tg, used, T, p, cs, iters);
       } else {
         reject = true;
         judged = used;
         st.v[5] = 1;
       }
     } else {
-      if (guess == PHL_GUESS_BRACKET) st.v[6] = bracket_guess(h, r, ht, ee, Tg);
+      if constexpr (GUESS == PHL_GUESS_BRACKET) st.v[6] = bracket_guess(h, r, ht, ee, Tg);
       else Tg = T[t];
       used = helm_rhoe_newton(h, r, ht, ee, Tg, 100, clamped, &conv);
       st.v[0] = 1;
       st.v[1] = used;
       st.v[2] = !conv;
       st.v[3] = clamped;
-      eos_finish(h, t, r, ht, Tg, used, T, p, cs, iters);
+      eos_finish<OUT>(h, t, r, ht, Tg, used, T, p, cs, iters);
     }
   }
   if constexpr (LEARNED) {
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(128, EOS_MINB) k_eos_fallback(HelmTable h, con
       st.v[1] += judged + used;
       st.v[2] += !conv;
       st.v[3] += clamped;
-      eos_finish(h, t, r, ht, Tg, judged + used, T, p, cs, iters);
+      eos_finish<true>(h, t, r, ht, Tg, judged + used, T, p, cs, iters);
     }
   }
   st.flush(stat);
@@ -213,14 +222,16 @@ inline int eos_launch(const HelmTable &h, cudaStream_t s, long long n, const dou
                       int guess, const Mlp &mlp, unsigned long long *stat, unsigned long long *queue, float *lT, int nsm) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
   if (guess != PHL_GUESS_MLP) {
-    k_eos_invert<false><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, nullptr, stat, nullptr);
+    auto k = guess == PHL_GUESS_BRACKET ? k_eos_invert<PHL_GUESS_BRACKET, true>
+                                        : (p || cs ? k_eos_invert<PHL_GUESS_WARM, true> : k_eos_invert<PHL_GUESS_WARM, false>);
+    k<<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, nullptr, stat, nullptr);
     return (int)cudaGetLastError();
   }
   const size_t sm = sizeof(MlpUmmaSmem);
   const cudaError_t err = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (err != cudaSuccess) return (int)err;
   k_eos_guess<<<blocks, 128, sm, s>>>(h, mlp.small, mlp.w2bf, n, rho, e, abar, zbar, lT, stat);
-  k_eos_invert<true><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, guess, lT, stat, queue);
+  k_eos_invert<PHL_GUESS_MLP, true><<<blocks, 128, 0, s>>>(h, n, rho, e, abar, zbar, T, p, cs, iters, lT, stat, queue);
   // enough resident blocks to cover every SM several times; the loop covers any queue length
   const unsigned fb = (unsigned)std::min<long long>((long long)nsm * 8, (long long)blocks);
   k_eos_fallback<<<fb, 128, 0, s>>>(h, queue, rho, e, abar, zbar, T, p, cs, iters, stat);
@@ -249,7 +260,7 @@ struct EosBatch {
   int energy(const HelmTable &h, cudaStream_t s, long long n, const double *rho, const double *T,
              const double *abar, const double *zbar, double *e) {
     if (n == 0) return 0;
-    k_eos_energy<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(h, n, rho, T, abar, zbar, e);
+    k_eos_energy<<<(unsigned)((n + ENERGY_THREADS - 1) / ENERGY_THREADS), ENERGY_THREADS, 0, s>>>(h, n, rho, T, abar, zbar, e);
     if (cudaGetLastError() != cudaSuccess) return -2;
     if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
     return 0;

@@ -99,3 +99,34 @@ def test_bracket_inversion_bitwise(gpu_lib, n):
         assert rc == 0
     T_want, it_want = helm.invert_batch(rho, e, abar, zbar, guess=2)
     assert np.array_equal(out, T_want) and np.array_equal(it, it_want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("out", [False, True])
+@pytest.mark.parametrize("n,off", [(1, 0.0), (129, 1e-3), (1000, 0.3), (1000, 0.0)])
+def test_warm_inversion_bitwise(gpu_lib, n, off, out):
+    """The Newton from a warm start against the oracle bit for bit, with p and cs and without (the two are
+    kernels of their own); p and cs are those of the bracket guess where T is the same."""
+    import pyoracle
+    from phlegethon_b200.abi import Simulation
+    tab = helm_table.generate(**helm_table.X1_TABLE)
+    cfg, _ = problems.stratified_3d(8, table=helm_table.X1_TABLE)
+    helm = pyoracle.Helm.for_config(cfg, *tab)
+    rho, T, abar, zbar = problems.eos_samples(n, seed=n + 1)
+    e = np.array([helm.given2(*q, deriv=False)[0] for q in zip(rho, T, abar, zbar)])
+    T0 = T * (1.0 + off)
+    got, it, p, cs = T0.copy(), np.zeros(n, dtype=np.int32), np.zeros(n), np.zeros(n)
+    with Simulation(cfg, tab) as sim:
+        def invert(t, pp, cc, guess):
+            po = (pp.ctypes.data, cc.ctypes.data) if pp is not None else (None, None)
+            assert sim.lib.phl_eos_invert_batch(sim.ctx, n, *[a.ctypes.data for a in (rho, e, abar, zbar)], t.ctypes.data,
+                                                *po, it.ctypes.data, guess) == 0
+        tb, pb, cb = np.zeros(n), np.zeros(n), np.zeros(n)
+        invert(tb, pb, cb, 2)
+        invert(got, p if out else None, cs if out else None, 0)
+    T_want, it_want = helm.invert_batch(rho, e, abar, zbar, T0=T0, guess=0)
+    assert np.array_equal(got, T_want) and np.array_equal(it, it_want)
+    if out:
+        same = got == tb
+        assert np.all(p > 0.0) and np.all(cs > 0.0)
+        assert np.array_equal(p[same], pb[same]) and np.array_equal(cs[same], cb[same])

@@ -184,13 +184,13 @@ def test_training_after_a_refused_allocation(rt):
     assert rt.violations() == 0 and rt.used() == 0
 
 
-@pytest.mark.parametrize("guess", [1, 2])
+@pytest.mark.parametrize("guess", [0, 1, 2])
 def test_batch_after_a_refused_allocation(rt, guess):
     """Batch inversions of host arrays whose buffers could not grow, then smaller ones."""
     cfg, h = problem("hydro")
     rt.watch("k_eos_guess", "ssPPPPPPPP")
-    rt.watch("k_eos_invertILb1E", "sPPPPPPPPPiPPP")
-    rt.watch("k_eos_invertILb0E", "sPPPPPPPPPiPPP")
+    kernel = "k_eos_invertILi%dE" % guess
+    rt.watch(kernel, "sPPPPPPPPPPPP")
     with started(cfg, h) as sim:
         assert sim.lib.phl_mlp_set_params(sim.ctx, (C.c_float * 4545)()) == 0
 
@@ -200,10 +200,10 @@ def test_batch_after_a_refused_allocation(rt, guess):
             return sim.lib.phl_eos_invert_batch(sim.ctx, n, *[x.ctypes.data for x in a], it.ctypes.data, guess)
         assert each_refusal(rt, lambda: invert(100), lambda: None) > 0
         assert each_refusal(rt, lambda: invert(1000), lambda: invert(50)) > 0
-        for _, (_, n, *_), room in rt.launches_of("k_eos_invertILb%dE" % (guess == 1)):
+        for _, (_, n, *_), room in rt.launches_of(kernel):
             assert all(room[i] >= 8 * n for i in range(2, 9)) and room[9] >= 4 * n
             if guess == 1:
-                assert room[11] >= 4 * n and room[13] >= 8 * (n + 1)
+                assert room[10] >= 4 * n and room[12] >= 8 * (n + 1)
         if guess == 1:
             for _, (_, _, _, n, *_), room in rt.launches_of("k_eos_guess"):
                 assert room[8] >= 4 * n
