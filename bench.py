@@ -97,9 +97,9 @@ def step_launches(cfg, form, guess="warm", one_kernel=False):
 # DRAM bytes per cell of one stage, from ncu captures of the 128^3 stratified box
 # (dram__bytes_read.sum + dram__bytes_write.sum over 2,097,152 cells); the kernels stream the
 # domain once per launch, so the traffic scales with the cell count
-TRAFFIC_PER_CELL = {# one FP64 hydro stage (a middle stage: U0 read): row faces 230.7 MB, walking x2/x3 faces
-                    # 245.8 + 245.1 MB, cons->prim 1164.2 MB
-                    ("stratified", "fp64"): (230.7e6 + 245.8e6 + 245.1e6 + 1164.2e6) / 2097152,
+TRAFFIC_PER_CELL = {# one FP64 hydro stage (a middle stage: U0 read): row faces 231.0 MB, walking x2/x3 faces
+                    # 246.8 + 244.8 MB, cons->prim 1127.6 MB
+                    ("stratified", "fp64"): (231.0e6 + 246.8e6 + 244.8e6 + 1127.6e6) / 2097152,
                     # one split hydro stage at 128^3: row and walk faces 98.5 + 97.1 + 99.1 MB,
                     # cons->prim 632.0 MB
                     ("stratified", "fp32_split"): (98.5e6 + 97.1e6 + 99.1e6 + 632.0e6) / 2097152,
