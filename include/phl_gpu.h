@@ -158,7 +158,9 @@ void phl_finalize(phl_ctx *ctx);
  * helm_* range parameters exactly as the reference does. */
 int phl_load_helm_table(phl_ctx *ctx, const double *helm_table_var, const double *dpdrho_table_var);
 
-/* Copy the reference-layout host arrays to the device (static background and dynamic state). */
+/* Copy the reference-layout host arrays to the device (static background and dynamic state).  A later
+ * call may leave the background out, or bring another one of any layout; if it fails on the way to the
+ * new background, steps answer PHL_E_STATE until an upload with a background succeeds. */
 int phl_upload_state(phl_ctx *ctx, const phl_fields *host);
 /* Copy the dynamic state back (prim interior+ghost layout, temp, eint, gammaf, b_cc, b_x*).
  * Ghost cells of the host arrays are left untouched.  Called before write_output /
